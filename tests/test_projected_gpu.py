@@ -1,0 +1,56 @@
+"""The projected eigensolver (trl_cuda_small_eigen_partial) where its kernels change shape.
+
+Tolerances, relative to ||T||_2: every stage is backward stable, with an error of a modest
+multiple of eps (2.2e-16) that grows at most like N <= 1024: 1e-12 for eigenvalues, 1e-11 for
+residuals and orthogonality, as for the larger matrices of test_kernels_gpu.py.
+"""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(cuda_handle, D, kvec, bs=1, scale=1.0):
+    N = D.shape[0]
+    nblk = N // bs
+    T = (D * scale).reshape(nblk, bs, nblk, bs).transpose(0, 2, 1, 3).copy()
+    beta = torch.eye(bs, dtype=torch.float64, device="cuda") * scale
+    _, evecs, ev, _ = cuda_handle.small_eigen_partial(torch.from_numpy(T).cuda(), beta, min(N, 4), 1e-8, kvec)
+    w = np.linalg.eigvalsh(D)
+    w = w[np.argsort(-np.abs(w), kind="stable")]
+    nrm = max(np.abs(w).max(), 1e-300)
+    X = evecs.cpu().numpy().transpose(0, 2, 1, 3).reshape(N, N)[:, :kvec]
+    ev = ev / scale
+    assert np.abs(np.abs(ev) - np.abs(w)).max() <= 1e-12 * nrm
+    assert np.abs(np.sort(ev) - np.sort(w)).max() <= 1e-12 * nrm
+    assert np.abs(D @ X - X * ev[:kvec]).max() <= 1e-11 * nrm
+    assert np.abs(X.T @ X - np.eye(kvec)).max() <= 1e-11
+
+
+# edges of the tridiagonalisation: rows of one warp (128 apart), the last size with rows in
+# registers (512) and in shared memory (624), rows in global memory beyond
+@pytest.mark.parametrize("N", [3, 4, 17, 127, 128, 129, 255, 256, 257, 384, 385, 511, 512, 513, 624, 625])
+def test_sizes(cuda_handle, N):
+    M = np.random.default_rng(N).standard_normal((N, N))
+    _check(cuda_handle, M + M.T, min(N, 24))
+
+
+def test_columns_that_are_already_reduced(cuda_handle):
+    """No reflector anywhere (tridiagonal and diagonal matrices), and for a part of the columns."""
+    rng = np.random.default_rng(1)
+    N = 200
+    D = np.diag(rng.uniform(1.0, 2.0, N)) + np.diag(rng.standard_normal(N - 1), 1)
+    D = np.triu(D) + np.triu(D, 1).T
+    _check(cuda_handle, D, 20)
+    _check(cuda_handle, np.diag(np.arange(1.0, N + 1.0)), 20)
+    M = rng.standard_normal((N - 70, N - 70))
+    D[70:, 70:] += M + M.T
+    D[69, 70] = D[70, 69] = 0.0
+    _check(cuda_handle, D, 20)
+
+
+@pytest.mark.parametrize("scale", [2.0 ** 450, 2.0 ** -450])
+def test_extreme_scales(cuda_handle, scale):
+    M = np.random.default_rng(2).standard_normal((140, 140))
+    _check(cuda_handle, M + M.T, 16, bs=4, scale=scale)

@@ -73,26 +73,40 @@ __global__ void __launch_bounds__(1024) k_max_abs(const double* __restrict__ T, 
 // then wrong (cuSOLVER's syevd on the GPU fails the same way on such matrices).
 constexpr double kFlushRel = 1e-30;
 
-// dense column-major A (N x N) from the lower triangle of the block matrix T
-__global__ void k_assemble_dense(const double* __restrict__ T, int nblk, int bs, const double* __restrict__ tmax, double* __restrict__ A)
+// 2^-e with 2^(e-1) <= tmax < 2^e: an exact scale that brings max|T| into [0.5, 1), so that
+// squares and products of the scaled entries neither overflow nor underflow
+__device__ __forceinline__ int scale_exponent(double tmax)
+{
+  if (!(tmax > 0.0) || isinf(tmax)) return 0;
+  const int e = ilogb(tmax) + 1;
+  return e < -1000 ? -1000 : (e > 1000 ? 1000 : e);
+}
+
+// dense column-major A (N x N) from the lower triangle of the block matrix T; `scaled`:
+// times 2^-scale_exponent(max|T|)
+__global__ void k_assemble_dense(const double* __restrict__ T, int nblk, int bs, const double* __restrict__ tmax, int scaled, double* __restrict__ A)
 {
   ::trl_detail::pdl_enter();
   const int N = nblk * bs;
   const int64_t total = static_cast<int64_t>(N) * N;
   const double floor = kFlushRel * *tmax;
+  const double scale = scaled ? scalbn(1.0, -scale_exponent(*tmax)) : 1.0;
   for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total; e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int c = static_cast<int>(e / N), r = static_cast<int>(e % N); // A[c*N + r] = M(r, c)
     const int hi = r > c ? r : c, lo = r > c ? c : r;
     const int bi = hi / bs, ri = hi % bs, bj = lo / bs, cj = lo % bs;
     const double v = T[(static_cast<int64_t>(bi) * nblk + bj) * bs * bs + ri * bs + cj];
-    A[e] = fabs(v) < floor ? 0.0 : v;
+    A[e] = fabs(v) < floor ? 0.0 : v * scale;
   }
 }
 
-// rank of each eigenvalue in decreasing |theta| order (ties keep ascending index)
-__global__ void k_rank(const double* __restrict__ w, int N, int* __restrict__ perm, double* __restrict__ evals_sorted, const int* __restrict__ syevd_info, int* status)
+// rank of each eigenvalue in decreasing |theta| order (ties keep ascending index); tmax: w is
+// that of a matrix scaled by 2^-scale_exponent(*tmax) (null: not scaled)
+__global__ void k_rank(const double* __restrict__ w, int N, const double* __restrict__ tmax, int* __restrict__ perm, double* __restrict__ evals_sorted,
+                       const int* __restrict__ syevd_info, int* status)
 {
   ::trl_detail::pdl_enter();
+  const double unscale = tmax ? scalbn(1.0, scale_exponent(*tmax)) : 1.0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && *syevd_info != 0) atomicOr(status, TRL_DEV_EIGEN);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
     const double ai = fabs(w[i]);
@@ -102,7 +116,7 @@ __global__ void k_rank(const double* __restrict__ w, int N, int* __restrict__ pe
       r += (aj > ai) || (aj == ai && j < i);
     }
     perm[r] = i;
-    evals_sorted[r] = w[i];
+    evals_sorted[r] = w[i] * unscale;
   }
 }
 
@@ -267,11 +281,11 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
 
   const unsigned g = grid_for(h, static_cast<int64_t>(N) * N, 256, 4);
   launch(k_max_abs, 1, 1024, 0, h->stream, T, static_cast<int64_t>(N) * N, tmax);
-  launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, A);
+  launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, 0, A);
   if (int st = after_launch(h, "assemble")) return st;
   cs = cusolverDnDsyevd(sh, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A, N, w, static_cast<double*>(h->syevd_work), lwork, info);
   if (cs != CUSOLVER_STATUS_SUCCESS) return set_error(h, TRL_ECUDA, "syevd failed (%d)", static_cast<int>(cs));
-  launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, perm, evals, info, h->d_status);
+  launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, static_cast<const double*>(nullptr), perm, evals, info, h->d_status);
   if (int st = after_launch(h, "rank")) return st;
   launch(k_scatter_evecs, g, 256, 0, h->stream, A, perm, nblk, bs, evecs);
   if (int st = after_launch(h, "scatter")) return st;
@@ -299,10 +313,8 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
 // trl_cuda_small_eigen_partial returns every eigenvalue but only the first kvec eigenvectors
 // (|theta| descending), which is all the driver reads (the kept blocks, lanczos.hh:105-131).
 // For 3 <= N <= kTriMaxN and kvec <= kTriMaxVec it runs without cuSOLVER:
-//  1. k_tridiag: Householder tridiagonalisation Q^T A Q = T in ONE thread-block cluster of
-//     8 or 16 CTAs. A (full symmetric storage) is distributed over the CTAs by rows (row g
-//     on CTA g % C, in its shared memory up to N = 640); each step exchanges the Householder column and the
-//     vector p = tau A v through distributed shared memory, two cluster barriers per step.
+//  1. k_tridiag: Householder tridiagonalisation Q^T A Q = T in ONE thread-block cluster of 16
+//     CTAs that exchange one column per step through distributed shared memory.
 //     (cuSOLVER's tridiagonalisation of the same matrix is a sequence of small kernels, about
 //     3.7 ms at N = 384 on B200.)
 //  2. k_bisect: all eigenvalues of T by bisection on Sturm counts, one warp per eigenvalue,
@@ -322,26 +334,26 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
 
 namespace {
 
-// The tridiagonalisation runs in one thread-block cluster; its rows live in the CTAs' shared
-// memory while they fit, in global memory (the dense copy it works on, L2-resident) beyond:
-//   N <= kTriMaxN8      8 CTAs (portable cluster size), rows in shared memory;
-//   N <= kTriMaxN16    16 CTAs (non-portable cluster size), rows in shared memory;
-//   N <= kTriMaxN      16 CTAs, rows in global memory.
-// Rows per CTA * N * 8 B must fit one CTA's shared memory (227 KB) for the first two.
+// The tridiagonalisation runs in one thread-block cluster of 16 CTAs (a non-portable cluster
+// size): N <= kTriMaxReg with the rows in registers (k_tridiag); beyond that, or where the
+// device cannot hold such a cluster, in shared memory (N <= kTriMaxShared) or in global memory
+// (k_tridiag_mem).
 constexpr int kTriThreads = 512;
-constexpr double kTinyNorm2 = 1e-290; // squared column norms below this are treated as zero
-constexpr int kTriMaxN8 = 448;
-constexpr int kTriMaxN16 = 640;
+constexpr double kTinyNorm2 = 1e-290; // squared column norms below this are treated as zero (entries are at most 1)
+constexpr int kTriMaxReg = 512;
+constexpr int kTriMaxShared = 624; // 39 rows and 7 vectors of N doubles in one CTA
 constexpr int kTriMaxN = 1024;
 constexpr int kTriMaxVec = 256;    // vectors by inverse iteration
 constexpr int kTriIters = 3;       // inverse-iteration sweeps
 constexpr int kBisectMaxN = kTriMaxN;
 constexpr size_t kTriGsMaxBytes = 200 * 1024; // the K vectors of N entries in one CTA's shared memory (else in global memory)
 
-size_t tridiag_smem(int N, int C, bool global_rows)
+enum TriRows { kTriRegs, kTriShared, kTriGlobal };
+
+size_t tridiag_smem(int N, int C, TriRows rows)
 {
-  const int RB = (N + C - 1) / C;
-  return sizeof(double) * ((global_rows ? 0 : static_cast<size_t>(RB) * N) + 4 * N + 2 * C * (kTriThreads / 32) + 8);
+  // {t, a} x 2, then v x 2 and w where the CTA shares them, then its rows
+  return sizeof(double) * static_cast<size_t>(N) * ((rows == kTriRegs ? 4 : 7) + (rows == kTriShared ? (N + C - 1) / C : 0));
 }
 
 __device__ __forceinline__ double warp_sum(double v)
@@ -390,136 +402,449 @@ __device__ __forceinline__ void stage(double* dst, const double* __restrict__ sr
   }
 }
 
-// A: N x N symmetric (full storage). Outputs: d[N], e[N-1] of T = Q^T A Q with
-// Q = H_0 ... H_{N-3}, H_k = I - tau_k v_k v_k^T, v_k stored in refl[k*N + k+1 .. N-1]
-// (refl[k*N + k+1] = 1). Row g belongs to CTA g % C of the cluster (C CTAs); with
-// kGlobalRows it is updated in place in A (only its owner reads or writes it, so the CTA's
-// own barriers order the accesses), otherwise it is copied into the owner's shared memory.
-// Exchange by pushing: before each cluster barrier every CTA stores its entries of the
-// Householder column (then of p = tau A v) and its per-warp partial sums into the shared
-// memory of every CTA of the cluster (st.shared::cluster through map_shared_rank); after
-// the barrier each CTA reads only its own shared memory. Every CTA reduces the same
-// partials in the same order, so all hold bit-identical scalars. A buffer filled at one
-// barrier is read before the next one, which its next writers wait for.
-template <int C, bool kGlobalRows>
+// 16-byte store {a, b} into shared memory of another CTA of the cluster (dst, bar: shared::cluster
+// addresses of that CTA), counted as 16 bytes on its mbarrier: the data is visible to whoever
+// sees the barrier's phase complete, without a cluster barrier or a fence on either side.
+__device__ __forceinline__ void st_async_pair(uint32_t dst, double a, double b, uint32_t bar)
+{
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst), "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)),
+               "r"(bar)
+               : "memory");
+}
+
+// address in CTA `rank` of the cluster of the shared variable at `addr` of this CTA
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank)
+{
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+// mbar_wait (common.cuh) for a phase that other CTAs of the cluster complete
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* status, uint32_t limit = (1u << 24))
+{
+  const uint32_t a = smem_addr(bar);
+  for (uint32_t it = 0; it < limit; ++it) {
+    uint32_t done;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(done)
+                 : "r"(a), "r"(parity)
+                 : "memory");
+    if (done) return true;
+  }
+  atomicOr(status, TRL_DEV_TIMEOUT);
+  return false;
+}
+
+// Householder tridiagonalisation. A: N x N symmetric (full storage, max|A| in [0.5, 1)).
+// Outputs: d[N], e[N-1] of Q^T A Q with Q = H_0 ... H_{N-3}, H_k = I - tau_k u_k u_k^T, u_k
+// stored in refl[k*N + k+1 .. N-1] (not normalised).
+//
+// One cluster of kTriC CTAs of kTriW warps; row g belongs to CTA g % 16 and there to warp
+// (g / 16) % 8, which holds it in registers (lane l: columns l, l + 32, ...): row i of a warp
+// lies in [128 i, 128 i + 127]. The chain of N steps is bound by latency, so a step is one
+// exchange between the CTAs and two sums over a warp, and every warp runs it for itself, with no
+// barrier over the CTA or the cluster:
+//  - step s starts with each warp sending {t_g, a_gs} of its rows g >= s to every CTA, t = A u_{s-1}
+//    and a_gs the row's entry in column s before the update of step s - 1, as one 16-byte
+//    asynchronous store that counts on the receiver's mbarrier;
+//  - with all pairs there, every warp of every CTA forms w = tau t - K u, column s after the
+//    rank-2 update (x = a - u w_s - w u_s), and u_s from x. They compute from the same operands in
+//    the same order, so all hold the same bits, and the column's norm needs no second exchange;
+//  - it updates its own rows, and multiplies them by u_s. The only entry of u_s that depends on the
+//    norm is the first, so that product and its sum run beside the norm's:
+//    t = sum_{j > s+1} a_j x_j + a_{s+1} u_{s+1}. tau is not needed before the next exchange.
+// Buffers and barriers alternate by step: a warp sends step s + 1 only after it has read step
+// s, and step s + 2 needs every row's data of step s + 1, so nothing is overwritten unread. A
+// warp leaves when its last row has been sent; the warp with the CTA's last row arms the
+// barrier of each step. Steps [128 F, 128 F + 127] run a body of their own without the rows
+// and columns before 128 F, so that the body has no branches and its chains overlap.
+// Measured on B200 (ncu, us a launch): N = 384 525, N = 512 920, N = 160 120. The kernel before
+// this one (rows in shared memory, two cluster barriers and three CTA barriers a step, the
+// sums over all CTAs' partials): 1,719, 2,604, 480. At N = 384 a step is about 2,300 cycles:
+// sending and waiting 660, reading the pairs and the first sum 440, rows and columns 750, the
+// second sum and the norm 410.
+constexpr int kTriC = 16;
+constexpr int kTriW = 8;
+constexpr int kTriStride = kTriC * kTriW; // rows of one warp are this far apart
+
+template <int RPW>
+struct TriState {
+  static constexpr int Q = 4 * RPW; // column groups of 32
+  double a[RPW][Q], u[Q], ug[RPW], t[RPW], col[RPW];
+  double us, half, dprev, eprev; // u_{s-1}[s]; (u . u) / 2 of u_{s-1} (0: no reflector); d, e of step s - 1
+  int s;
+};
+
+struct TriArgs {
+  int N, g0, glast; // matrix size; this warp's first and last row
+  bool keeper;
+  uint32_t to_pairs, to_bar; // lane q: addresses in CTA q
+  const double2* pairs;
+  uint64_t* bars;
+  double *dout, *eout, *tau_out, *refl;
+  int* status;
+};
+
+// Steps 128 F ... 128 F + 127 (fewer at the end). false: this warp is done.
+template <int RPW, int F>
+__device__ __forceinline__ bool tri_steps(TriState<RPW>& st, const TriArgs& k)
+{
+  constexpr int Q = TriState<RPW>::Q, Q0 = 4 * F;
+  const int lane = threadIdx.x & 31, N = k.N;
+  for (; st.s < kTriStride * (F + 1); ++st.s) {
+    const int s = st.s, cur = s & 1;
+    if (s < N - 1) {
+#pragma unroll
+      for (int i = F; i < RPW; ++i) {
+        const int g = k.g0 + i * kTriStride;
+        if (g >= s && g < N && lane < kTriC)
+          st_async_pair(k.to_pairs + static_cast<uint32_t>((cur * N + g) * 16), st.t[i], st.col[i], k.to_bar + static_cast<uint32_t>(cur * 8));
+      }
+    }
+    const double tau = st.half > 0.0 ? 1.0 / st.half : 0.0;
+    if (s > 0 && (s & (kTriStride - 1)) == k.g0) { // the owner of row s writes reflector s - 1
+      if (s < N - 1) {
+#pragma unroll
+        for (int q = Q0; q < Q; ++q) {
+          const int j = q * 32 + lane;
+          if (j >= s && j < N) k.refl[static_cast<size_t>(s - 1) * N + j] = st.u[q];
+        }
+      }
+      if (lane == 0) {
+        k.dout[s - 1] = st.dprev;
+        k.eout[s - 1] = st.eprev;
+        k.tau_out[s - 1] = tau;
+      }
+    }
+    if (s == k.glast) {
+      if (s == N - 1 && lane == 0) { // the last diagonal entry is not sent: nobody needs it
+#pragma unroll
+        for (int i = F; i < RPW; ++i)
+          if (k.g0 + i * kTriStride == s) k.dout[s] = st.col[i];
+      }
+      return false;
+    }
+    if (k.keeper && lane == 0) mbar_arrive_expect_tx(&k.bars[cur], static_cast<uint32_t>(N - s) * 16u);
+    const bool late = !mbar_wait_cluster(&k.bars[cur], static_cast<uint32_t>(s >> 1) & 1u, k.status);
+    if (__any_sync(0xffffffffu, late)) return false; // whole warp: gives up, the status word says why
+    // ---- w = tau t - K u with K = tau^2 (t . u) / 2; x: column s after the update
+    const double2* pc = k.pairs + cur * N;
+    const double us = st.us;
+    // four rows of 16 column groups leave no registers for the t_j as well: they are read again
+    constexpr bool kReload = RPW - F >= 4;
+    double w[Q], x[Q];
+    double k4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int q = Q0; q < Q; ++q) {
+      const int j = q * 32 + lane;
+      double2 p = make_double2(0.0, 0.0);
+      if (j >= s && j < N) p = pc[j];
+      w[q] = p.x;
+      x[q] = p.y;
+      k4[q & 3] = fma(p.x, st.u[q], k4[q & 3]);
+    }
+    const double2 ps = pc[s];
+    const double K = 0.5 * tau * tau * warp_sum((k4[0] + k4[1]) + (k4[2] + k4[3]));
+    const double ws = fma(-K, us, tau * ps.x);
+    st.dprev = fma(-2.0 * ws, us, ps.y);
+    if constexpr (kReload) asm volatile("" ::: "memory");
+    // ... column by column, with this warp's rows: update, product with x, entry of column s + 1
+    double wg[RPW], t2[RPW][2];
+#pragma unroll
+    for (int i = F; i < RPW; ++i) {
+      wg[i] = fma(-K, st.ug[i], tau * st.t[i]);
+      t2[i][0] = t2[i][1] = 0.0;
+    }
+    double xg[RPW];
+#pragma unroll
+    for (int i = F; i < RPW; ++i) xg[i] = st.col[i] - fma(st.ug[i], ws, wg[i] * us);
+    double n4[4] = {0.0, 0.0, 0.0, 0.0};
+    double x0 = 0.0;
+#pragma unroll
+    for (int q = Q0; q < Q; ++q) {
+      const int j = q * 32 + lane;
+      if constexpr (kReload) w[q] = j >= s && j < N ? pc[j].x : 0.0;
+      const double wq = fma(-K, st.u[q], tau * w[q]);
+      const double uq = st.u[q];
+      double xq = x[q] - fma(uq, ws, wq * us);
+      if (j == s + 1) x0 = xq;
+      if (j <= s + 1) xq = 0.0;
+      n4[q & 3] = fma(xq, xq, n4[q & 3]);
+#pragma unroll
+      for (int i = F; i < RPW; ++i) {
+        const double aq = fma(-st.ug[i], wq, fma(-wg[i], uq, st.a[i][q]));
+        st.a[i][q] = aq;
+        t2[i][q & 1] = fma(aq, xq, t2[i][q & 1]);
+        if (q == Q0) st.col[i] = aq;
+        else st.col[i] = j == s + 1 ? aq : st.col[i];
+      }
+      st.u[q] = xq;
+    }
+    double tn[RPW];
+#pragma unroll
+    for (int i = F; i < RPW; ++i) {
+      tn[i] = t2[i][0] + t2[i][1];
+      st.ug[i] = xg[i];
+    }
+    double xnorm2 = (n4[0] + n4[1]) + (n4[2] + n4[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      xnorm2 += __shfl_xor_sync(0xffffffffu, xnorm2, o);
+#pragma unroll
+      for (int i = F; i < RPW; ++i) tn[i] += __shfl_xor_sync(0xffffffffu, tn[i], o);
+    }
+    x0 = __shfl_sync(0xffffffffu, x0, (s + 1) & 31);
+    // ---- reflector s: u = x + copysign(||x||, x_{s+1}) e_{s+1}, tau = 2 / (u . u)
+    // a column whose squares underflow is left as it is (H = I): a reflector built from a
+    // norm computed in the subnormal range would not be orthogonal
+    const double norm2 = fma(x0, x0, xnorm2);
+    const double norm = (xnorm2 > 0.0 && norm2 > kTinyNorm2) ? sqrt(norm2) : 0.0;
+    const double beta = norm > 0.0 ? -copysign(norm, x0) : x0;
+    st.us = x0 - beta;
+#pragma unroll
+    for (int q = Q0; q < Q; ++q)
+      if (q * 32 + lane == s + 1) st.u[q] = st.us;
+#pragma unroll
+    for (int i = F; i < RPW; ++i) {
+      st.col[i] = __shfl_sync(0xffffffffu, st.col[i], (s + 1) & 31);
+      st.t[i] = fma(st.col[i], st.us, tn[i]);
+      if (k.g0 + i * kTriStride == s + 1) st.ug[i] = st.us;
+    }
+    st.half = norm * (norm + fabs(x0));
+    st.eprev = beta;
+  }
+  return true;
+}
+
+template <int RPW, int F>
+__device__ __forceinline__ void tri_phases(TriState<RPW>& st, const TriArgs& k)
+{
+  if constexpr (F < RPW) {
+    if (tri_steps<RPW, F>(st, k)) tri_phases<RPW, F + 1>(st, k);
+  }
+}
+
+template <int RPW>
+__global__ void __launch_bounds__(kTriW * 32, 1)
+    k_tridiag(double* __restrict__ A, int N, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out,
+              double* __restrict__ refl, int* status)
+{
+  ::trl_detail::pdl_enter();
+  namespace cg = cooperative_groups;
+  constexpr int Q = TriState<RPW>::Q;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int r = static_cast<int>(cluster.block_rank());
+  extern __shared__ __align__(16) double sm[]; // [2][N] pairs {t, a}
+  __shared__ __align__(8) uint64_t bars[2];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    mbar_init_fence();
+  }
+  TriArgs k;
+  k.N = N;
+  k.g0 = r + kTriC * warp;
+  k.glast = k.g0 < N ? k.g0 + (N - 1 - k.g0) / kTriStride * kTriStride : -1;
+  const int cta_rows = r < N ? (N - 1 - r) / kTriC + 1 : 0;
+  k.keeper = cta_rows > 0 && warp == (cta_rows - 1) % kTriW;
+  // lane q < 16 sends to CTA q
+  k.to_pairs = cluster_addr(smem_addr(sm), lane < kTriC ? lane : 0);
+  k.to_bar = cluster_addr(smem_addr(&bars[0]), lane < kTriC ? lane : 0);
+  k.pairs = reinterpret_cast<const double2*>(sm);
+  k.bars = bars;
+  k.dout = dout;
+  k.eout = eout;
+  k.tau_out = tau_out;
+  k.refl = refl;
+  k.status = status;
+  TriState<RPW> st;
+#pragma unroll
+  for (int i = 0; i < RPW; ++i) {
+    const int g = k.g0 + i * kTriStride;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) st.a[i][q] = (g < N && q * 32 + lane < N) ? A[static_cast<size_t>(g) * N + q * 32 + lane] : 0.0;
+    st.col[i] = __shfl_sync(0xffffffffu, st.a[i][0], 0);
+    st.ug[i] = st.t[i] = 0.0;
+  }
+#pragma unroll
+  for (int q = 0; q < Q; ++q) st.u[q] = 0.0;
+  st.us = st.half = st.dprev = st.eprev = 0.0;
+  st.s = 0;
+  cluster.sync(); // every CTA's barriers exist before any store counts on them
+  if (k.glast >= 0) tri_phases<RPW, 0>(st, k);
+  cluster.sync(); // no CTA leaves while another may still store into its shared memory
+}
+
+// The same reduction for matrices whose rows do not fit the cluster's registers, or where a
+// cluster of 16 CTAs cannot be resident: rows in the owner's shared memory, or in global memory
+// (A itself, L2-resident), updated in place by the lanes of the owning warp; v normalised to v_k[k+1] = 1; the CTA's threads
+// share the vectors, thread t holding entries t + 512 e, and the sums are over the CTA.
+// RPW: rows a warp owns at most, ceil(ceil(N / C) / 16).
+// N = 576 (shared memory) and N = 640, 768, 1024 (global): see kTriVariants.
+constexpr int kTriEntries = kTriMaxN / kTriThreads;
+
+// Sum over the CTA of kTriThreads threads, all threads get it: one shuffle tree, one barrier,
+// the warps' partials re-read by everyone in one order. `slot` (16 doubles) may be reused
+// after one more barrier.
+__device__ __forceinline__ double tri_block_sum(double v, double* slot)
+{
+  constexpr int NW = kTriThreads / 32;
+  v = warp_sum(v);
+  if ((threadIdx.x & 31) == 0) slot[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < NW; ++q) s[q & 3] += slot[q];
+  return (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+template <int C, int RPW, bool kGlobalRows>
 __global__ void __launch_bounds__(kTriThreads, 1)
-    k_tridiag(double* __restrict__ A, int N, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out, double* __restrict__ refl)
+    k_tridiag_mem(double* __restrict__ A, int N, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out,
+                  double* __restrict__ refl, int* status)
 {
   ::trl_detail::pdl_enter();
   namespace cg = cooperative_groups;
   constexpr int NW = kTriThreads / 32;
-  constexpr int NP = C * NW; // partials per exchange
-  static_assert(NP % 32 == 0, "partials are reduced as NP / 32 per lane");
+  constexpr int E = kTriEntries;
   cg::cluster_group cluster = cg::this_cluster();
   const int r = static_cast<int>(cluster.block_rank());
   const int RB = (N + C - 1) / C;
   extern __shared__ __align__(16) double sm[];
-  double* const rows = kGlobalRows ? nullptr : sm; // RB x N, local row l = global row r + C * l
-  double* xfull = sm + (kGlobalRows ? 0 : RB * N); // N: column k below the diagonal (pushed by the owners)
-  double* pfull = xfull + N;      // N: p (pushed by the owners)
-  double* vfull = pfull + N;      // N
-  double* wfull = vfull + N;      // N
-  double* part = wfull + N;       // NP sums of squares (slot rank * NW + warp), then x0
-  double* part2 = part + NP + 8;  // NP partial p.v
+  __shared__ __align__(16) double red[2][NW];
+  __shared__ double x0s;
+  __shared__ __align__(8) uint64_t bars[2];
+  double* const pa = sm;                 // [2][N] pairs {p, a}, written by the rows' owners
+  double* const vbuf = pa + 4 * N;       // [2][N] v_k by parity of k
+  double* const wbuf = vbuf + 2 * N;     // [N] w_{k-1}
+  double* const rows = wbuf + N;         // RB x N, local row l = global row r + C * l
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  auto row = [&](int l) -> double* { return kGlobalRows ? A + static_cast<size_t>(r + C * l) * N : rows + static_cast<size_t>(l) * N; };
 
-  auto local_sum = [&](const double* slot) {
-    double s = 0.0;
-#pragma unroll
-    for (int q = 0; q < NP / 32; ++q) s += slot[lane + 32 * q];
-    return warp_sum(s);
-  };
-  // store v at offset `at` of `buf` in every CTA of the cluster
-  auto push = [&](double* buf, int at, double v) {
-#pragma unroll
-    for (int q = 0; q < C; ++q) cluster.map_shared_rank(buf, q)[at] = v;
-  };
-
-  if (!kGlobalRows) {
-    for (int l = 0; l < RB; ++l) {
-      const int g = r + C * l;
-      if (g < N) stage(rows + l * N, A + static_cast<size_t>(g) * N, N);
-      else
-        for (int j = tid; j < N; j += kTriThreads) rows[l * N + j] = 0.0;
-    }
+  if (!kGlobalRows)
+    for (int l = 0; l < RB; ++l)
+      if (r + C * l < N) stage(rows + l * N, A + static_cast<size_t>(r + C * l) * N, N);
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    mbar_init_fence();
   }
-  cluster.sync(); // every CTA is running before any pushes into it
+  for (int j = tid; j < 3 * N; j += kTriThreads) vbuf[j] = 0.0; // v, w
+  // lane q < C sends to CTA q
+  const uint32_t to_pa = cluster_addr(smem_addr(pa), lane < C ? lane : 0);
+  const uint32_t to_bar = cluster_addr(smem_addr(&bars[0]), lane < C ? lane : 0);
+  cluster.sync(); // every CTA's barriers exist before any store counts on them
 
-  for (int k = 0; k < N - 2; ++k) {
-    const int l0 = (k + 1 - r + C - 1) / C > 0 ? (k + 1 - r + C - 1) / C : 0; // first local row > k
-    if (r == k % C && tid == 0) dout[k] = row(k / C)[k];
-    // ---- phase A: push this CTA's entries of x = A[k+1:, k] and its partial sum of squares
+  double tau = 0.0;
+  double vj[E]; // v_k[tid + 512 e]
+#pragma unroll
+  for (int e = 0; e < E; ++e) vj[e] = 0.0;
+  for (int k = -1; k <= N - 2; ++k) { // step k: d[k+1], e[k+1], reflector k+1
+    const int s = k + 1;
+    const int cur = s & 1; // buffers of v_k, of this step's exchange; the other one holds v_{k-1}
+    const double* v = vbuf + cur * N;
+    const double* vp = vbuf + (cur ^ 1) * N;
+    if (tid == 0) mbar_arrive_expect_tx(&bars[cur], static_cast<uint32_t>(N - s) * 16u);
+    // ---- rows g > k: rank-2 update of step k - 1, p = tau A v, entry of column k + 1
+    const int l0 = s - r > 0 ? (s - r + C - 1) / C : 0; // first local row >= s
+    const int lw = l0 + (warp + NW - l0 % NW) % NW;     // this warp's first one
     {
-      double ssq = 0.0;
-      if (tid < RB - l0) {
-        const int l = l0 + tid, g = r + C * l;
-        if (g < N) {
-          const double x = row(l)[k];
-          push(xfull, g, x);
-          if (g > k + 1) ssq = x * x;
+      double acc[RPW], col[RPW], vg[RPW], wg[RPW];
+      double* rl[RPW];
+      bool on[RPW];
+#pragma unroll
+      for (int i = 0; i < RPW; ++i) {
+        const int l = lw + i * NW, g = r + C * l;
+        on[i] = l < RB && g < N;
+        rl[i] = kGlobalRows ? A + static_cast<size_t>(on[i] ? g : 0) * N : rows + static_cast<size_t>(on[i] ? l : 0) * N;
+        vg[i] = on[i] ? vp[g] : 0.0;
+        wg[i] = on[i] ? wbuf[g] : 0.0;
+        acc[i] = col[i] = 0.0;
+      }
+      const int q0 = s & ~31; // columns from the multiple of 32 at or below k + 1 (v, vp, w are zero or unused before it)
+      for (int j = q0 + lane; j < N; j += 32) {
+        const double vjj = v[j], vpj = vp[j], wpj = wbuf[j];
+        double a[RPW];
+#pragma unroll
+        for (int i = 0; i < RPW; ++i) a[i] = on[i] ? rl[i][j] : 0.0;
+#pragma unroll
+        for (int i = 0; i < RPW; ++i)
+          if (on[i]) {
+            a[i] = fma(-vg[i], wpj, fma(-wg[i], vpj, a[i]));
+            rl[i][j] = a[i];
+            acc[i] = fma(a[i], vjj, acc[i]);
+            if (j == s) col[i] = a[i];
+          }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < RPW; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+#pragma unroll
+      for (int i = 0; i < RPW; ++i) {
+        col[i] = __shfl_sync(0xffffffffu, col[i], s & 31);
+        if (on[i] && lane < C) {
+          const int g = r + C * (lw + i * NW);
+          st_async_pair(to_pa + static_cast<uint32_t>((cur * N + g) * 16), tau * acc[i], col[i], to_bar + static_cast<uint32_t>(cur * 8));
         }
       }
-      ssq = warp_sum(ssq);
-      if (lane < C) cluster.map_shared_rank(part, lane)[r * NW + warp] = ssq;
-      if (tid == 0 && r == (k + 1) % C) push(part, NP, row((k + 1) / C)[k]);
     }
-    cluster.sync(); // #1
-    const double xnorm2 = local_sum(part);
-    const double x0 = part[NP];
-    double tau = 0.0, beta = x0, scale = 0.0;
-    // a column whose squares underflow is left as it is (H = I): a reflector built from a
-    // norm computed in the subnormal range would not be orthogonal
-    if (xnorm2 > 0.0 && x0 * x0 + xnorm2 > kTinyNorm2) {
+    const bool late = !mbar_wait_cluster(&bars[cur], static_cast<uint32_t>(s >> 1) & 1u, status);
+    // ---- w_k = p - K v, K = tau (p . v) / 2
+    const double2* pc = reinterpret_cast<const double2*>(pa) + cur * N;
+    double p[E], a[E];
+    double pv = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int j = tid + e * kTriThreads;
+      const double2 q = j >= s && j < N ? pc[j] : make_double2(0.0, 0.0);
+      p[e] = q.x;
+      a[e] = q.y;
+      pv = fma(q.x, vj[e], pv);
+    }
+    const double p1 = pc[s].x;
+    if (__syncthreads_or(late)) break; // whole CTA: give up, the status word says why
+    const double K = 0.5 * tau * tri_block_sum(pv, red[0]);
+    const double w1 = p1 - K; // v_k[k+1] = 1
+    // ---- column k + 1 after step k: its diagonal entry and x below it
+    double x[E], w[E];
+    double ssq = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int j = tid + e * kTriThreads;
+      w[e] = k >= 0 ? p[e] - K * vj[e] : 0.0;
+      x[e] = k >= 0 ? a[e] - (vj[e] * w1 + w[e]) : a[e];
+      if (j == s && r == 0) dout[s] = x[e];
+      if (j == s + 1) x0s = x[e];
+      if (j > s + 1 && j < N) ssq = fma(x[e], x[e], ssq);
+    }
+    const double xnorm2 = tri_block_sum(ssq, red[1]);
+    if (s == N - 1) break; // d[N-1] was the last
+    const double x0 = x0s;
+    double beta = x0, scale = 0.0;
+    tau = 0.0;
+    if (xnorm2 > 0.0 && x0 * x0 + xnorm2 > kTinyNorm2) { // as in k_tridiag
       beta = -copysign(sqrt(x0 * x0 + xnorm2), x0);
       tau = (beta - x0) / beta;
       scale = 1.0 / (x0 - beta);
     }
-    for (int j = k + 1 + tid; j < N; j += kTriThreads) vfull[j] = (j == k + 1) ? 1.0 : xfull[j] * scale;
-    __syncthreads();
-    if (r == k % C) {
-      for (int j = k + 1 + tid; j < N; j += kTriThreads) refl[static_cast<size_t>(k) * N + j] = vfull[j];
-      if (tid == 0) {
-        tau_out[k] = tau;
-        eout[k] = beta;
+    double* vn = vbuf + (cur ^ 1) * N; // v_{k+1}; all of this step's reads of v_{k-1} and w_{k-1} are behind the barriers above
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int j = tid + e * kTriThreads;
+      vj[e] = j > s + 1 ? x[e] * scale : (j == s + 1 ? 1.0 : 0.0);
+      if (j < N) {
+        vn[j] = vj[e];
+        wbuf[j] = w[e];
+        if (r == s % C && j > s && s < N - 2) refl[static_cast<size_t>(s) * N + j] = vj[e];
       }
     }
-    // ---- phase C: p = tau * A_trail v for this CTA's rows (warp per row), pushed with the
-    // partial p.v
-    double pv = 0.0;
-    for (int l = l0 + warp; l < RB; l += NW) {
-      const int g = r + C * l;
-      if (g >= N) break;
-      const double* rl = row(l);
-      double s = 0.0;
-      for (int j = k + 1 + lane; j < N; j += 32) s = fma(rl[j], vfull[j], s);
-      s = warp_sum(s) * tau;
-      if (lane < C) cluster.map_shared_rank(pfull, lane)[g] = s;
-      pv = fma(s, vfull[g], pv);
-    }
-    if (lane < C) cluster.map_shared_rank(part2, lane)[r * NW + warp] = pv;
-    cluster.sync(); // #2
-    const double K = 0.5 * tau * local_sum(part2);
-    for (int j = k + 1 + tid; j < N; j += kTriThreads) wfull[j] = pfull[j] - K * vfull[j];
-    __syncthreads();
-    // ---- phase D: rank-2 update of this CTA's trailing rows (warp per row)
-    if (tau != 0.0) {
-      for (int l = l0 + warp; l < RB; l += NW) {
-        const int g = r + C * l;
-        if (g >= N) break;
-        double* rl = row(l);
-        const double vg = vfull[g], wg = wfull[g];
-        for (int j = k + 1 + lane; j < N; j += 32) rl[j] -= vg * wfull[j] + wg * vfull[j];
-      }
+    if (r == 0 && tid == 0) {
+      eout[s] = beta;
+      tau_out[s] = tau;
     }
     __syncthreads();
-  }
-  if (tid == 0) {
-    if (N >= 2 && r == (N - 2) % C) dout[N - 2] = row((N - 2) / C)[N - 2];
-    if (r == (N - 1) % C) {
-      dout[N - 1] = row((N - 1) / C)[N - 1];
-      if (N >= 2) eout[N - 2] = row((N - 1) / C)[N - 2];
-    }
   }
   cluster.sync(); // no CTA leaves while another may still store into its shared memory
 }
@@ -928,20 +1253,24 @@ __global__ void k_zero_cols(double* __restrict__ Y, int nblk, int bs, int K)
   }
 }
 
-using TriKernel = void (*)(double*, int, double*, double*, double*, double*);
+using TriKernel = void (*)(double*, int, double*, double*, double*, double*, int*);
 
 struct TriVariant {
   TriKernel fn;
   int C;       // CTAs in the cluster
-  bool global; // rows in global memory
+  int threads;
+  TriRows rows;
   int max_n;
 };
 
 constexpr TriVariant kTriVariants[] = {
-    {k_tridiag<8, false>, 8, false, kTriMaxN8},
-    {k_tridiag<16, false>, 16, false, kTriMaxN16},
-    {k_tridiag<16, true>, 16, true, kTriMaxN},
-    {k_tridiag<8, true>, 8, true, kTriMaxN},
+    {k_tridiag<1>, kTriC, kTriW * 32, kTriRegs, 128},
+    {k_tridiag<2>, kTriC, kTriW * 32, kTriRegs, 256},
+    {k_tridiag<3>, kTriC, kTriW * 32, kTriRegs, 384},
+    {k_tridiag<4>, kTriC, kTriW * 32, kTriRegs, kTriMaxReg},
+    {k_tridiag_mem<16, 3, false>, 16, kTriThreads, kTriShared, kTriMaxShared},
+    {k_tridiag_mem<16, 4, true>, 16, kTriThreads, kTriGlobal, kTriMaxN},
+    {k_tridiag_mem<8, 8, true>, 8, kTriThreads, kTriGlobal, kTriMaxN},
 };
 constexpr int kNumTriVariants = sizeof(kTriVariants) / sizeof(kTriVariants[0]);
 
@@ -949,8 +1278,8 @@ void tri_config(const TriVariant& v, int N, cudaStream_t stream, cudaLaunchConfi
 {
   cfg = cudaLaunchConfig_t{};
   cfg.gridDim = dim3(v.C);
-  cfg.blockDim = dim3(kTriThreads);
-  cfg.dynamicSmemBytes = tridiag_smem(N, v.C, v.global);
+  cfg.blockDim = dim3(v.threads);
+  cfg.dynamicSmemBytes = tridiag_smem(N, v.C, v.rows);
   cfg.stream = stream;
   attr = cudaLaunchAttribute{};
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -978,7 +1307,7 @@ const TriVariant* tri_variant(int device, int N)
                         cudaFuncSetAttribute(k_wy_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * kWyRows * kTriMaxN)) == cudaSuccess;
     for (int i = 0; i < kNumTriVariants && common; ++i) {
       const TriVariant& v = kTriVariants[i];
-      if (cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tridiag_smem(v.max_n, v.C, v.global))) != cudaSuccess) continue;
+      if (cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tridiag_smem(v.max_n, v.C, v.rows))) != cudaSuccess) continue;
       if (v.C > 8 && cudaFuncSetAttribute(v.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) continue;
       cudaLaunchConfig_t cfg{};
       cudaLaunchAttribute attr{};
@@ -1037,19 +1366,19 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
 
   const unsigned g = grid_for(h, static_cast<int64_t>(N) * N, 256, 4);
   launch(k_max_abs, 1, 1024, 0, h->stream, T, static_cast<int64_t>(N) * N, tmax);
-  launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, A);
+  launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, 1, A);
   if (int st = after_launch(h, "assemble")) return st;
   cudaMemsetAsync(flags, 0, 2 * sizeof(int), h->stream);
   {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
     tri_config(*tv, N, h->stream, cfg, attr);
-    cudaLaunchKernelEx(&cfg, tv->fn, A, N, d, e, tau, refl);
+    cudaLaunchKernelEx(&cfg, tv->fn, A, N, d, e, tau, refl, h->d_status);
     if (int st = after_launch(h, "tridiagonalise")) return st;
   }
   launch(k_bisect, (N + 7) / 8, 256, 0, h->stream, d, e, N, w);
   if (int st = after_launch(h, "bisect")) return st;
-  launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, perm, evals, flags, h->d_status);
+  launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, tmax, perm, evals, flags, h->d_status);
   if (int st = after_launch(h, "rank")) return st;
   launch(k_select, 1, kTriMaxVec, 0, h->stream, perm, K, sel, slot);
   if (int st = after_launch(h, "select")) return st;
