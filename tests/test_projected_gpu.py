@@ -54,3 +54,23 @@ def test_columns_that_are_already_reduced(cuda_handle):
 def test_extreme_scales(cuda_handle, scale):
     M = np.random.default_rng(2).standard_normal((140, 140))
     _check(cuda_handle, M + M.T, 16, bs=4, scale=scale)
+
+
+# kept vectors at the edges of the 8-vector tiles and 32-entry strips, and groups of equal
+# or nearly equal eigenvalues: none, some, one of 40, all
+@pytest.mark.parametrize("N,kvec", [(130, 1), (130, 7), (130, 8), (130, 9), (161, 112), (300, 256)])
+def test_kept_vectors(cuda_handle, N, kvec):
+    M = np.random.default_rng(kvec).standard_normal((N, N))
+    _check(cuda_handle, M + M.T, kvec)
+
+
+@pytest.mark.parametrize("gap", [0.0, 1e-14, 3e-11, 1e-9, 1e-6])
+def test_groups_of_close_eigenvalues(cuda_handle, gap):
+    rng = np.random.default_rng(3)
+    Q, _ = np.linalg.qr(rng.standard_normal((150, 150)))
+    lam = np.concatenate([5.0 + gap * np.arange(40), [4.0, 4.0, 3.0], rng.uniform(-1.0, 1.0, 107)])
+    _check(cuda_handle, (Q * lam) @ Q.T, 48)
+
+
+def test_one_eigenvalue(cuda_handle):
+    _check(cuda_handle, 3.0 * np.eye(96), 16)

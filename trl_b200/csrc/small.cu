@@ -319,15 +319,12 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
 //     3.7 ms at N = 384 on B200.)
 //  2. k_bisect: all eigenvalues of T by bisection on Sturm counts, one warp per eigenvalue,
 //     each lane evaluating one of 32 points of the interval per iteration (multisection).
-//  3. k_tri_factor / k_tri_solve / k_tri_gs: eigenvectors of T for the kvec selected
+//  3. k_tri_factor / k_tri_solve / k_gs_apply: eigenvectors of T for the kvec selected
 //     eigenvalues by inverse iteration (partial-pivoting LU of T - lambda I, tiny pivots
-//     replaced by eps * ||T||), all vectors at once, then classical Gram-Schmidt applied
-//     twice in ascending eigenvalue order. A solve shrinks the component along an eigenvalue
-//     at distance g by eps * ||T|| / g relative to the wanted one, so three solves separate
-//     every pair with g above ~1e-10 ||T|| to working accuracy; closer pairs (and exactly
-//     equal ones) span their eigenspace and the Gram-Schmidt step makes them orthonormal.
-//     The wanted end of a Lanczos T is one tight cluster (48 values within 5e-4 ||T|| at the
-//     96^3 workload), so vectors are not iterated one after another.
+//     replaced by eps * ||T||), all vectors at once. A solve shrinks the component along an
+//     eigenvalue at distance g by eps * ||T|| / g relative to the wanted one; the wanted end of
+//     a Lanczos T is one tight cluster (48 values within 5e-4 ||T|| at the 96^3 workload), so
+//     vectors are not iterated one after another but orthonormalised at the end (k_tri_cluster).
 //  4. k_wy_factor / k_backtransform: x = Q z with the stored reflectors in compact WY
 //     chunks (Q restricted to a chunk = I - V T V^T).
 // Otherwise it falls back to trl_cuda_small_eigen and zeroes the columns from kvec on.
@@ -346,7 +343,6 @@ constexpr int kTriMaxN = 1024;
 constexpr int kTriMaxVec = 256;    // vectors by inverse iteration
 constexpr int kTriIters = 3;       // inverse-iteration sweeps
 constexpr int kBisectMaxN = kTriMaxN;
-constexpr size_t kTriGsMaxBytes = 200 * 1024; // the K vectors of N entries in one CTA's shared memory (else in global memory)
 
 enum TriRows { kTriRegs, kTriShared, kTriGlobal };
 
@@ -362,7 +358,7 @@ __device__ __forceinline__ double warp_sum(double v)
   return v;
 }
 
-// block sum over kTriThreads threads; `red` holds 32 doubles; all threads get the result
+// block sum over the CTA; `red` holds 32 doubles; all threads get the result
 __device__ double block_sum(double v, double* red)
 {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1038,48 +1034,151 @@ __global__ void __launch_bounds__(32) k_tri_solve(int N, const double* __restric
   for (int i = lane; i < N; i += 32) Z[static_cast<size_t>(t) * N + i] = x[i] * inv;
 }
 
-// classical Gram-Schmidt applied twice, column by column in ascending eigenvalue order, on
-// the K vectors held in shared memory (kGlobal: in place in Z, for K x N beyond one CTA's
-// shared memory); one CTA of kTriThreads threads
-template <bool kGlobal>
-__global__ void __launch_bounds__(kTriThreads) k_tri_gs(int N, int K, double* __restrict__ Z)
+// Orthonormalisation of the K vectors (rows of Z, ascending eigenvalues). Inverse iteration
+// leaves an overlap of about eps ||T|| / gap between two vectors, so the vectors of eigenvalues
+// further apart than kClusterGap ||T|| are orthogonal to 1e-5, and one step
+//   z_j <- z_j - (E_jj / 2) z_j - sum_{i<j} E_ij z_i,   E = Z Z^T - I,
+// which is Gram-Schmidt in this order to first order, squares what is left: two steps reach
+// rounding. They are matrix products spread over the SMs, where Gram-Schmidt vector by vector
+// is a chain of K steps in one CTA (B200, N = 384, K = 40: 165 us in shared memory; N = 512, K =
+// 112: 3,610 us in global memory; now 38 and 59 us in all).
+//  1. k_tri_cluster: Gram-Schmidt twice within each group of closer eigenvalues, a CTA per group;
+//     it also scales every vector to unit length;
+//  2. k_gs_gram, k_gs_apply twice;
+//  3. k_tri_gs, where the first step left more than kGsLimit (never seen): Gram-Schmidt twice
+//     over all vectors.
+constexpr double kClusterGap = 1e-10;
+constexpr double kGsLimit = 1e-8;
+
+// Gram-Schmidt twice of z_j against z_first .. z_{j-1}, then unit length, by one CTA; coef: K
+// doubles of shared memory
+__device__ void gs_column(int N, int first, int j, double* __restrict__ Z, double* coef, double* red)
 {
-  ::trl_detail::pdl_enter();
-  extern __shared__ __align__(16) double zsm[]; // K x N
-  double* const zs = kGlobal ? Z : zsm;
-  __shared__ double coef[kTriMaxVec];
-  __shared__ double red[32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int NW = kTriThreads / 32;
-  if (!kGlobal) stage(zs, Z, K * N);
-  __syncthreads();
-  for (int j = 0; j < K; ++j) {
-    double* zj = zs + static_cast<size_t>(j) * N;
-    for (int pass = 0; pass < 2 && j > 0; ++pass) {
-      for (int i = warp; i < j; i += NW) {
-        const double* zi = zs + static_cast<size_t>(i) * N;
-        double s = 0.0;
-        for (int n = lane; n < N; n += 32) s = fma(zi[n], zj[n], s);
-        s = warp_sum(s);
-        if (lane == 0) coef[i] = s;
-      }
-      __syncthreads();
-      for (int n = tid; n < N; n += kTriThreads) {
-        double v = zj[n];
-        for (int i = 0; i < j; ++i) v = fma(-coef[i], zs[static_cast<size_t>(i) * N + n], v);
-        zj[n] = v;
-      }
-      __syncthreads();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  double* zj = Z + static_cast<size_t>(j) * N;
+  for (int pass = 0; pass < 2 && j > first; ++pass) {
+    for (int i = first + warp; i < j; i += nw) {
+      const double* zi = Z + static_cast<size_t>(i) * N;
+      double s = 0.0;
+      for (int n = lane; n < N; n += 32) s = fma(zi[n], zj[n], s);
+      s = warp_sum(s);
+      if (lane == 0) coef[i - first] = s;
     }
-    double s = 0.0;
-    for (int n = tid; n < N; n += kTriThreads) s = fma(zj[n], zj[n], s);
-    s = block_sum(s, red);
-    const double inv = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
-    for (int n = tid; n < N; n += kTriThreads) zj[n] *= inv;
+    __syncthreads();
+    for (int n = tid; n < N; n += blockDim.x) {
+      double v = zj[n];
+      for (int i = first; i < j; ++i) v = fma(-coef[i - first], Z[static_cast<size_t>(i) * N + n], v);
+      zj[n] = v;
+    }
     __syncthreads();
   }
-  if (!kGlobal)
-    for (int idx = tid; idx < K * N; idx += kTriThreads) Z[idx] = zs[idx];
+  double s = 0.0;
+  for (int n = tid; n < N; n += blockDim.x) s = fma(zj[n], zj[n], s);
+  s = block_sum(s, red);
+  const double inv = s > 0.0 ? 1.0 / sqrt(s) : 0.0;
+  for (int n = tid; n < N; n += blockDim.x) zj[n] *= inv;
+  __syncthreads();
+}
+
+constexpr int kClusterThreads = 256;
+
+__global__ void __launch_bounds__(kClusterThreads) k_tri_cluster(int N, int K, const double* __restrict__ w, const int* __restrict__ sel, double* __restrict__ Z)
+{
+  ::trl_detail::pdl_enter();
+  __shared__ double coef[kTriMaxVec];
+  __shared__ double red[32];
+  const int t = blockIdx.x;
+  const double tol = kClusterGap * fmax(fabs(w[0]), fabs(w[N - 1]));
+  if (t > 0 && w[sel[t]] - w[sel[t - 1]] <= tol) return; // in the group of the vector before
+  gs_column(N, t, t, Z, coef, red);
+  for (int j = t + 1; j < K && w[sel[j]] - w[sel[j - 1]] <= tol; ++j) gs_column(N, t, j, Z, coef, red);
+}
+
+// E(i, j) = z_i . z_j - delta_ij (row-major K x K) for the 8 x 8 tiles on and above the
+// diagonal: a CTA per tile, its 8 warps take every 8th group of 4 entries of the vectors
+// (DMMA), summed in warp order. emax (may be null): the largest |E| as an ordered bit pattern.
+__global__ void __launch_bounds__(256) k_gs_gram(int N, int K, const double* __restrict__ Z, double* __restrict__ E, unsigned long long* emax)
+{
+  ::trl_detail::pdl_enter();
+  __shared__ double part[8][64];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  int tj = 0, ti = blockIdx.x; // tile (ti <= tj): column tj holds tj + 1 tiles
+  while (ti > tj) ti -= ++tj;
+  const int i = ti * 8 + g, j = tj * 8 + g;
+  const double* zi = Z + static_cast<size_t>(i < K ? i : 0) * N;
+  const double* zj = Z + static_cast<size_t>(j < K ? j : 0) * N;
+  double d0[2] = {0.0, 0.0}, d1[2] = {0.0, 0.0};
+  constexpr int U = 4; // loads in flight
+  for (int n0 = warp * 4; n0 < N; n0 += 32 * U) {
+    double a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int n = n0 + u * 32 + t4;
+      a[u] = (n < N && i < K) ? zi[n] : 0.0;
+      b[u] = (n < N && j < K) ? zj[n] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) dmma_m8n8k4(d0[u & 1], d1[u & 1], a[u], b[u]);
+  }
+  part[warp][g * 8 + 2 * t4] = d0[0] + d0[1];
+  part[warp][g * 8 + 2 * t4 + 1] = d1[0] + d1[1];
+  __syncthreads();
+  if (tid < 64) {
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) s += part[q][tid];
+    const int ei = ti * 8 + (tid >> 3), ej = tj * 8 + (tid & 7);
+    double big = 0.0;
+    if (ei < K && ej < K) {
+      if (ei == ej) s -= 1.0;
+      E[static_cast<size_t>(ei) * K + ej] = s;
+      if (ei <= ej) big = fabs(s);
+    }
+    for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+    if (emax && (tid & 31) == 0) atomicMax(emax, static_cast<unsigned long long>(__double_as_longlong(big)));
+  }
+}
+
+// out_j = z_j - (E_jj / 2) z_j - sum_{i<j} E_ij z_i: a warp per 8 vectors x 32 entries (DMMA).
+// With emax above kGsLimit: out = z.
+__global__ void __launch_bounds__(128) k_gs_apply(int N, int K, const double* __restrict__ Z, const double* __restrict__ E, const unsigned long long* emax, double* __restrict__ out)
+{
+  ::trl_detail::pdl_enter();
+  const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+  const int j0 = blockIdx.x * 8, n0 = (blockIdx.y * 4 + (threadIdx.x >> 5)) * 32;
+  if (n0 >= N) return;
+  const int iend = (emax && __longlong_as_double(static_cast<long long>(*emax)) > kGsLimit) ? 0 : min(j0 + 8, K);
+  double d0[4] = {0.0, 0.0, 0.0, 0.0}, d1[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+  for (int i0 = 0; i0 < iend; i0 += 4) {
+    const int i = i0 + t4, j = j0 + g; // A(g, t4) = -U(i, j), B(t4, g) = z_i[n]
+    double a = (i < iend && j < K && i <= j) ? -E[static_cast<size_t>(i) * K + j] : 0.0;
+    if (i == j) a *= 0.5;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int n = n0 + c * 8 + g;
+      const double b = (i < iend && n < N) ? Z[static_cast<size_t>(i) * N + n] : 0.0;
+      dmma_m8n8k4(d0[c], d1[c], a, b);
+    }
+  }
+  const int j = j0 + g;
+  if (j >= K) return;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int n = n0 + c * 8 + 2 * t4;
+    if (n < N) out[static_cast<size_t>(j) * N + n] = Z[static_cast<size_t>(j) * N + n] + d0[c];
+    if (n + 1 < N) out[static_cast<size_t>(j) * N + n + 1] = Z[static_cast<size_t>(j) * N + n + 1] + d1[c];
+  }
+}
+
+// Gram-Schmidt twice over all vectors, one CTA, if *emax is above kGsLimit
+__global__ void __launch_bounds__(kTriThreads) k_tri_gs(int N, int K, double* __restrict__ Z, const unsigned long long* emax)
+{
+  ::trl_detail::pdl_enter();
+  if (!(__longlong_as_double(static_cast<long long>(*emax)) > kGsLimit)) return;
+  __shared__ double coef[kTriMaxVec];
+  __shared__ double red[32];
+  for (int j = 0; j < K; ++j) gs_column(N, 0, j, Z, coef, red);
 }
 
 // Back-transform X = Q Z, Q = H_0 ... H_{N-3}, in chunks of kWyRows reflectors: a chunk
@@ -1300,8 +1399,7 @@ const TriVariant* tri_variant(int device, int N)
   std::lock_guard<std::mutex> g(lock);
   if (!checked[device]) {
     checked[device] = true;
-    const bool common = cudaFuncSetAttribute(k_tri_gs<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kTriGsMaxBytes)) == cudaSuccess &&
-                        cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kFactorRows + 1) * kTriMaxN)) == cudaSuccess &&
+    const bool common = cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kFactorRows + 1) * kTriMaxN)) == cudaSuccess &&
                         cudaFuncSetAttribute(k_tri_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * kFactorRows * kTriMaxN)) == cudaSuccess &&
                         cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kWyRows + kWyVecs) * kTriMaxN)) == cudaSuccess &&
                         cudaFuncSetAttribute(k_wy_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * kWyRows * kTriMaxN)) == cudaSuccess;
@@ -1363,8 +1461,10 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   int* slot = sel + N;
   int* flags = slot + N; // [0] = 0 (no solver error), [1] = converged count
   double* tmax = reinterpret_cast<double*>(ws + (sizeof(double) * doubles + sizeof(int) * ints + 15) / 16 * 16);
+  auto* emax = reinterpret_cast<unsigned long long*>(tmax + 1);
 
   const unsigned g = grid_for(h, static_cast<int64_t>(N) * N, 256, 4);
+  cudaMemsetAsync(emax, 0, sizeof *emax, h->stream);
   launch(k_max_abs, 1, 1024, 0, h->stream, T, static_cast<int64_t>(N) * N, tmax);
   launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, 1, A);
   if (int st = after_launch(h, "assemble")) return st;
@@ -1388,8 +1488,20 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
     launch(k_tri_solve, K, 32, sizeof(double) * (kFactorRows + 1) * N, h->stream, N, F, Z);
     if (int st = after_launch(h, "inverse iteration")) return st;
   }
-  if (sizeof(double) * NK > kTriGsMaxBytes) launch(k_tri_gs<true>, 1, kTriThreads, 0, h->stream, N, K, Z);
-  else launch(k_tri_gs<false>, 1, kTriThreads, sizeof(double) * NK, h->stream, N, K, Z);
+  launch(k_tri_cluster, K, kClusterThreads, 0, h->stream, N, K, w, sel, Z);
+  if (int st = after_launch(h, "gram-schmidt")) return st;
+  const int kt = (K + 7) / 8;
+  const dim3 apply_grid(kt, (N + 127) / 128);
+  for (int round = 0; round < 2; ++round) {
+    double* from = round == 0 ? Z : X;
+    double* to = round == 0 ? X : Z;
+    unsigned long long* check = round == 0 ? nullptr : emax;
+    launch(k_gs_gram, kt * (kt + 1) / 2, 256, 0, h->stream, N, K, from, F, check); // F: the factors are done with
+    if (int st = after_launch(h, "overlaps")) return st;
+    launch(k_gs_apply, apply_grid, 128, 0, h->stream, N, K, from, F, check, to);
+    if (int st = after_launch(h, "orthogonalise")) return st;
+  }
+  launch(k_tri_gs, 1, kTriThreads, 0, h->stream, N, K, Z, emax);
   if (int st = after_launch(h, "gram-schmidt")) return st;
   const int nch = (N - 2 + kWyRows - 1) / kWyRows;
   launch(k_wy_factor, nch, 256, sizeof(double) * kWyRows * N, h->stream, refl, tau, N, Tw);
