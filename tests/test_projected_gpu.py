@@ -24,6 +24,8 @@ def _check(cuda_handle, D, kvec, bs=1, scale=1.0):
     ev = ev / scale
     assert np.abs(np.abs(ev) - np.abs(w)).max() <= 1e-12 * nrm
     assert np.abs(np.sort(ev) - np.sort(w)).max() <= 1e-12 * nrm
+    if kvec == 0:
+        return
     assert np.abs(D @ X - X * ev[:kvec]).max() <= 1e-11 * nrm
     assert np.abs(X.T @ X - np.eye(kvec)).max() <= 1e-11
 
@@ -74,3 +76,14 @@ def test_groups_of_close_eigenvalues(cuda_handle, gap):
 
 def test_one_eigenvalue(cuda_handle):
     _check(cuda_handle, 3.0 * np.eye(96), 16)
+
+
+@pytest.mark.parametrize("N", [3, 4, 5, 6, 7, 8, 9, 10, 11, 64, 201])
+def test_counts_at_exact_zeros(cuda_handle, N):
+    """Integer and singular tridiagonals: pivots and products that are exactly zero at the
+    points the bisection tries, repeated blocks, and entries of very different size."""
+    i = np.arange(N)
+    for d, e in ((np.zeros(N), np.ones(N - 1)), (2.0 * np.ones(N), -np.ones(N - 1)), (i % 3 - 1.0, (i[:-1] % 2) * 1.0), (1.0 * (i == 0), np.zeros(N - 1)),
+                 (10.0 ** -(i % 20), 10.0 ** -(i[:-1] % 17)), (np.zeros(N), 1e-25 * np.ones(N - 1) + (i[:-1] == 0))):
+        D = np.diag(d) + np.diag(e, 1) + np.diag(e, -1)
+        _check(cuda_handle, D, 0 if N > 100 else 1)

@@ -317,8 +317,8 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
 //     CTAs that exchange one column per step through distributed shared memory.
 //     (cuSOLVER's tridiagonalisation of the same matrix is a sequence of small kernels, about
 //     3.7 ms at N = 384 on B200.)
-//  2. k_bisect: all eigenvalues of T by bisection on Sturm counts, one warp per eigenvalue,
-//     each lane evaluating one of 32 points of the interval per iteration (multisection).
+//  2. k_bisect: all eigenvalues of T by bisection on Sturm counts, a CTA per eigenvalue whose
+//     threads evaluate one of 64 points of the interval each per round (multisection).
 //  3. k_tri_factor / k_tri_solve / k_gs_apply: eigenvectors of T for the kvec selected
 //     eigenvalues by inverse iteration (partial-pivoting LU of T - lambda I, tiny pivots
 //     replaced by eps * ||T||), all vectors at once. A solve shrinks the component along an
@@ -342,7 +342,6 @@ constexpr int kTriMaxShared = 624; // 39 rows and 7 vectors of N doubles in one 
 constexpr int kTriMaxN = 1024;
 constexpr int kTriMaxVec = 256;    // vectors by inverse iteration
 constexpr int kTriIters = 3;       // inverse-iteration sweeps
-constexpr int kBisectMaxN = kTriMaxN;
 
 enum TriRows { kTriRegs, kTriShared, kTriGlobal };
 
@@ -845,65 +844,149 @@ __global__ void __launch_bounds__(kTriThreads, 1)
   cluster.sync(); // no CTA leaves while another may still store into its shared memory
 }
 
-// number of eigenvalues of the tridiagonal (d, e2 = e^2) below sigma
-__device__ __forceinline__ int sturm_count(const double* d, const double* e2, int N, double sigma, double pivmin)
+// ---- eigenvalues of the tridiagonal by bisection on Sturm counts
+// The number of eigenvalues below sigma is the number of negative pivots of T - sigma I, that is of
+// sign changes in p_j = (d_j - sigma) p_{j-1} - e_{j-1}^2 p_{j-2} (the pivots are p_j / p_{j-1}).
+// The products need no division, which leaves one dependent FMA per row (17 cycles, against
+// about 190 for a row of pivots), and are kept in range by powers of two. Elimination runs from
+// both ends to row h = N / 2 at once, whose pivot is
+// (d_h - sigma) - e_{h-1}^2 p_{h-2} / p_{h-1} - (the same from below).
+// Where they vanish all the same (a pivot of exactly zero beside a zero coupling, or several
+// minute ones in a row), the pivots themselves are counted.
+constexpr double kPivMin = 0x1p-900; // smallest pivot of the division form
+
+// number of eigenvalues below sigma, counted on pivots; row j = (d_j, e_{j-1}^2)
+__device__ __noinline__ int sturm_count_pivots(const double2* up, const double2* down, int N, double sigma)
 {
-  double q = d[0] - sigma;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int c = q < 0.0;
-  for (int j = 1; j < N; ++j) {
-    q = (d[j] - sigma) - e2[j - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
+  const int h = N / 2;
+  double q = 1.0;
+  int c = 0;
+  for (int j = 0; j < N; ++j) {
+    const double d = j < h ? up[j].x : (j == h ? up[h].x : down[N - 1 - j].x);
+    const double e2 = j <= h ? up[j].y : down[N - j].y; // coupling to row j - 1
+    q = (d - sigma) - (j > 0 ? e2 / q : 0.0);
+    if (fabs(q) < kPivMin) q = -kPivMin;
     c += q < 0.0;
   }
   return c;
 }
 
-// w[i] = i-th smallest eigenvalue of the tridiagonal (d, e); one warp per eigenvalue
-__global__ void __launch_bounds__(256) k_bisect(const double* __restrict__ dg, const double* __restrict__ eg, int N, double* __restrict__ w)
+// One step of the recurrence for row r = (d, e^2 to the row before): p1 the newest product
+__device__ __forceinline__ void sturm_step(double2 r, double sigma, double& p1, double& p0, int& c)
+{
+  const double p = fma(r.x - sigma, p1, -(r.y * p0));
+  c += static_cast<int>(static_cast<unsigned>(__double2hiint(p) ^ __double2hiint(p1)) >> 31);
+  p0 = p1;
+  p1 = p;
+}
+
+// Keeps a pair of products in range: both by the same power of two (their signs and ratio
+// stay). Sets `lost` where they are too small to tell.
+__device__ __forceinline__ void sturm_rescale(double& p1, double& p0, bool& lost)
+{
+  const int top = max(__double2hiint(p1) & 0x7fffffff, __double2hiint(p0) & 0x7fffffff); // exponent in the upper 11 bits
+  if (top < ((1023 - 300) << 20)) {
+    lost |= top < ((1023 - 900) << 20);
+    p1 *= 0x1p300;
+    p0 *= 0x1p300;
+  }
+  else if (top > ((1023 + 300) << 20)) {
+    p1 *= 0x1p-300;
+    p0 *= 0x1p-300;
+  }
+}
+
+// number of eigenvalues below sigma. up[j] = (d_j, e_{j-1}^2) for rows 0 .. h from the top,
+// down[i] = (d, e^2 to the row below) of row N - 1 - i for rows N - 1 .. h + 1 from the bottom
+// (down[N - 1 - h].y: the coupling of rows h and h + 1).
+__device__ __forceinline__ int sturm_count(const double2* up, const double2* down, int N, double sigma)
+{
+  const int h = N / 2, m = N - 1 - h; // rows from the top, from the bottom: h = m or m + 1
+  double p1 = 1.0, p0 = 0.0, r1 = 1.0, r0 = 0.0;
+  int c = 0;
+  bool lost = false;
+  int j = 0;
+  for (; j + 4 <= m; j += 4) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      sturm_step(up[j + u], sigma, p1, p0, c);
+      sturm_step(down[j + u], sigma, r1, r0, c);
+    }
+    sturm_rescale(p1, p0, lost);
+    sturm_rescale(r1, r0, lost);
+  }
+  for (; j < m; ++j) {
+    sturm_step(up[j], sigma, p1, p0, c);
+    sturm_step(down[j], sigma, r1, r0, c);
+  }
+  if (j < h) sturm_step(up[j], sigma, p1, p0, c);
+  sturm_rescale(p1, p0, lost);
+  sturm_rescale(r1, r0, lost);
+  // pivot of row h times p1 r1
+  const double g = fma((up[h].x - sigma) * p1, r1, -fma(up[h].y * p0, r1, down[m].y * r0 * p1));
+  if (lost || !(fabs(p1) > 0.0) || !(fabs(r1) > 0.0) || !(fabs(g) > 0.0)) return sturm_count_pivots(up, down, N, sigma);
+  return c + static_cast<int>(static_cast<unsigned>(__double2hiint(g) ^ __double2hiint(p1) ^ __double2hiint(r1)) >> 31);
+}
+
+// w[i] = i-th smallest eigenvalue of the tridiagonal (d, e): a CTA of two warps per eigenvalue,
+// which evaluates the count at 64 points of the interval at a time (multisection). Bound by the
+// latency of the recurrence: N / 2 rows x 9 rounds.
+// Measured on B200: N = 384 94 us, N = 512 123 us (before, on pivots from one end, one warp and 32
+// points per eigenvalue, and the Gershgorin bounds summed by one thread: 427 and 568 us).
+constexpr int kBisectPoints = 64;
+
+__global__ void __launch_bounds__(kBisectPoints) k_bisect(const double* __restrict__ dg, const double* __restrict__ eg, int N, double* __restrict__ w)
 {
   ::trl_detail::pdl_enter();
-  __shared__ double d[kBisectMaxN], e2[kBisectMaxN];
-  __shared__ double bounds[3];
-  for (int j = threadIdx.x; j < N; j += blockDim.x) {
-    d[j] = dg[j];
-    e2[j] = j + 1 < N ? eg[j] * eg[j] : 0.0;
+  extern __shared__ __align__(16) double2 rows[]; // up: N / 2 + 1, then down: N - N / 2
+  __shared__ double red[3][2];
+  __shared__ unsigned above[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = N / 2;
+  double2* up = rows;
+  double2* down = rows + h + 1;
+  double lo = INFINITY, hi = -INFINITY;
+  for (int j = tid; j < N; j += kBisectPoints) {
+    const double d = dg[j], eb = j > 0 ? fabs(eg[j - 1]) : 0.0, ea = j + 1 < N ? fabs(eg[j]) : 0.0;
+    if (j <= h) up[j] = make_double2(d, eb * eb);
+    if (j >= h) down[N - 1 - j] = make_double2(d, ea * ea);
+    lo = fmin(lo, d - (eb + ea));
+    hi = fmax(hi, d + (eb + ea));
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) {
+    red[0][warp] = lo;
+    red[1][warp] = hi;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double lo = d[0], hi = d[0], emax = 0.0;
-    for (int j = 0; j < N; ++j) {
-      const double rad = (j > 0 ? sqrt(e2[j - 1]) : 0.0) + (j + 1 < N ? sqrt(e2[j]) : 0.0);
-      lo = fmin(lo, d[j] - rad);
-      hi = fmax(hi, d[j] + rad);
-      if (j + 1 < N) emax = fmax(emax, e2[j]);
-    }
-    const double nrm = fmax(fabs(lo), fabs(hi));
-    bounds[0] = lo - 2.0 * DBL_EPSILON * nrm * N - DBL_MIN;
-    bounds[1] = hi + 2.0 * DBL_EPSILON * nrm * N + DBL_MIN;
-    bounds[2] = DBL_MIN * fmax(1.0, emax); // pivmin
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= N) return;
-  double lo = bounds[0], hi = bounds[1];
-  const double pivmin = bounds[2];
+  lo = fmin(red[0][0], red[0][1]);
+  hi = fmax(red[1][0], red[1][1]);
+  const double margin = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) * N + kPivMin;
+  lo -= margin;
+  hi += margin;
+  const int i = blockIdx.x;
   for (int it = 0; it < 64; ++it) {
     const double width = hi - lo;
-    if (width <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 2.0 * pivmin) break;
-    const double sigma = lo + width * (lane + 1) / 33.0;
-    const int c = sturm_count(d, e2, N, sigma, pivmin);
-    // smallest lane whose point has more than i eigenvalues below it
-    const unsigned above = __ballot_sync(0xffffffffu, c > i);
-    const int q = above ? __ffs(above) - 1 : 32;
-    const double nlo = q == 0 ? lo : lo + width * q / 33.0;
-    const double nhi = q == 32 ? hi : lo + width * (q + 1) / 33.0;
+    if (width <= 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + 2.0 * kPivMin) break;
+    constexpr double parts = kBisectPoints + 1;
+    const double sigma = lo + width * (tid + 1) / parts;
+    const int c = sturm_count(up, down, N, sigma);
+    const unsigned mask = __ballot_sync(0xffffffffu, c > i);
+    if (lane == 0) above[warp] = mask;
+    __syncthreads();
+    // smallest point with more than i eigenvalues below it
+    const int q = above[0] ? __ffs(above[0]) - 1 : (above[1] ? 31 + __ffs(above[1]) : kBisectPoints);
+    __syncthreads();
+    const double nlo = q == 0 ? lo : lo + width * q / parts;
+    const double nhi = q == kBisectPoints ? hi : lo + width * (q + 1) / parts;
     if (!(nhi < hi || nlo > lo)) break; // no progress in floating point
     lo = nlo;
     hi = nhi;
   }
-  if (lane == 0) w[i] = 0.5 * (lo + hi);
+  if (tid == 0) w[i] = 0.5 * (lo + hi);
 }
 
 __device__ __forceinline__ double hash_unit(unsigned a, unsigned b)
@@ -1476,7 +1559,7 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
     cudaLaunchKernelEx(&cfg, tv->fn, A, N, d, e, tau, refl, h->d_status);
     if (int st = after_launch(h, "tridiagonalise")) return st;
   }
-  launch(k_bisect, (N + 7) / 8, 256, 0, h->stream, d, e, N, w);
+  launch(k_bisect, N, kBisectPoints, sizeof(double2) * (N + 1), h->stream, d, e, N, w);
   if (int st = after_launch(h, "bisect")) return st;
   launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, tmax, perm, evals, flags, h->d_status);
   if (int st = after_launch(h, "rank")) return st;
