@@ -319,7 +319,7 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
 //     3.7 ms at N = 384 on B200.)
 //  2. k_bisect: all eigenvalues of T by bisection on Sturm counts, a CTA per eigenvalue whose
 //     threads evaluate one of 64 points of the interval each per round (multisection).
-//  3. k_tri_factor / k_tri_solve / k_gs_apply: eigenvectors of T for the kvec selected
+//  3. k_tri_vectors, k_gs_apply: eigenvectors of T for the kvec selected
 //     eigenvalues by inverse iteration (partial-pivoting LU of T - lambda I, tiny pivots
 //     replaced by eps * ||T||), all vectors at once. A solve shrinks the component along an
 //     eigenvalue at distance g by eps * ||T|| / g relative to the wanted one; the wanted end of
@@ -1001,120 +1001,162 @@ __device__ __forceinline__ double hash_unit(unsigned a, unsigned b)
 }
 
 // Inverse iteration for the eigenvectors of the tridiagonal (d, e) at the K eigenvalues
-// w[sel[t]] (sel ascending). Vectors: Z[t * N + i]. Per vector t the factorisation
-// P L U = T - lambda_t I (general tridiagonal LU with partial pivoting; pivots below
-// eps * ||T|| replaced by +-eps * ||T||) is stored as F[t][5][N]: multipliers, 1 / U diagonal,
-// U first and second superdiagonal, pivot flags. The recurrences are sequential: one lane
-// runs them on the vector's shared-memory copy.
-constexpr int kFactorRows = 5;
+// w[sel[t]] (sel ascending): a warp per vector t, kTriIters solves with T - lambda_t I from a random
+// start, into Z[t * N + i] (not scaled; k_tri_cluster does that).
+// Elimination with partial pivoting runs from both ends to the middle at once, lane 0 from row 0
+// and lane 1 from row N - 1 (a side sees the matrix in its own order, so both run the same
+// code), and leaves two equations in the two middle unknowns; substitution runs outwards. The
+// recurrences are chains of one reciprocal (factorisation) or one FMA (substitution) per row;
+// everything else is prepared by all lanes. Pivots below eps * ||T|| are replaced by +-eps * ||T||.
+// Position i of side s is stored at 2 i + s.
+// Measured on B200 (K = 40, N = 384 / K = 112, N = 512): 51 / 63 us (before,
+// one lane from one end, a kernel for the factors and one per solve: 177 / 227 us).
+constexpr int kVectorArrays = 5; // diagonal -> U1, coupling -> U2, multiplier, 1 / pivot, vector
 
-__global__ void __launch_bounds__(32) k_tri_factor(const double* __restrict__ dg, const double* __restrict__ eg, int N, const double* __restrict__ w, const int* __restrict__ sel,
-                                                   double* __restrict__ F, double* __restrict__ Z)
+size_t vectors_smem(int N) { return (sizeof(double) * kVectorArrays + 1) * static_cast<size_t>(N + 1); }
+
+__global__ void __launch_bounds__(32) k_tri_vectors(const double* __restrict__ dg, const double* __restrict__ eg, int N, const double* __restrict__ w, const int* __restrict__ sel,
+                                                    double* __restrict__ Z)
 {
   ::trl_detail::pdl_enter();
-  extern __shared__ __align__(16) double fs[]; // 5 x N
+  extern __shared__ __align__(16) double vs[];
+  const int M = N + 1; // odd N: side 1 is one shorter
+  double* U1 = vs;          // diagonal; then the pivot row's next entry times 1 / pivot
+  double* U2 = vs + M;      // coupling to the next position; then the entry after it, times 1 / pivot
+  double* F = vs + 2 * M;   // multiplier
+  double* RP = vs + 3 * M;  // 1 / pivot
+  double* X = vs + 4 * M;   // right-hand side, solution
+  unsigned char* SW = reinterpret_cast<unsigned char*>(vs + 5 * M); // rows exchanged
   const int t = blockIdx.x, lane = threadIdx.x;
-  // ||T||_inf (Gershgorin) for the pivot floor
+  const int h0 = (N + 1) / 2, h1 = N / 2;
+  const double lam = w[sel[t]];
   double nrm = 0.0;
-  for (int i = lane; i < N; i += 32) nrm = fmax(nrm, fabs(dg[i]) + (i > 0 ? fabs(eg[i - 1]) : 0.0) + (i + 1 < N ? fabs(eg[i]) : 0.0));
+  for (int i = lane; i < N; i += 32) {
+    const double eb = i > 0 ? eg[i - 1] : 0.0, ea = i + 1 < N ? eg[i] : 0.0, d = dg[i];
+    nrm = fmax(nrm, fabs(d) + fabs(eb) + fabs(ea));
+    const int at = i < h0 ? 2 * i : 2 * (N - 1 - i) + 1;
+    U1[at] = d - lam;
+    U2[at] = i < h0 ? ea : eb;
+    X[at] = hash_unit(static_cast<unsigned>(t), static_cast<unsigned>(i));
+  }
   for (int o = 16; o > 0; o >>= 1) nrm = fmax(nrm, __shfl_xor_sync(0xffffffffu, nrm, o));
   if (!(nrm > 0.0)) nrm = 1.0;
-  double* DL = fs;
-  double* D = fs + N;
-  double* DU = fs + 2 * N;
-  double* DU2 = fs + 3 * N;
-  double* PV = fs + 4 * N;
-  const double lam = w[sel[t]];
-  for (int i = lane; i < N; i += 32) {
-    D[i] = dg[i] - lam;
-    DL[i] = i + 1 < N ? eg[i] : 0.0;
-    DU[i] = i + 1 < N ? eg[i] : 0.0;
-    DU2[i] = 0.0;
-    PV[i] = 0.0;
-    Z[static_cast<size_t>(t) * N + i] = hash_unit(static_cast<unsigned>(t), static_cast<unsigned>(i));
-  }
+  const double tiny = DBL_EPSILON * nrm;
+  const auto floored = [tiny](double p) { return fabs(p) < tiny ? (p < 0.0 ? -tiny : tiny) : p; };
   __syncwarp();
-  if (lane == 0) {
-    const double tiny = DBL_EPSILON * nrm;
-    for (int i = 0; i + 1 < N; ++i) {
-      if (fabs(D[i]) >= fabs(DL[i])) {
-        if (fabs(D[i]) < tiny) D[i] = D[i] < 0.0 ? -tiny : tiny;
-        const double fact = DL[i] / D[i];
-        DL[i] = fact;
-        D[i + 1] -= fact * DU[i];
-      }
-      else {
-        const double fact = D[i] / DL[i];
-        D[i] = DL[i];
-        DL[i] = fact;
-        const double temp = DU[i];
-        DU[i] = D[i + 1];
-        D[i + 1] = temp - fact * D[i + 1];
-        if (i + 2 < N) {
-          DU2[i] = DU[i + 1];
-          DU[i + 1] = -fact * DU[i + 1];
+  const int side = lane & 1, len = side ? h1 : h0;
+  double D = 0.0, U = 0.0, c = 0.0; // the equation carried along: D x_i + U x_{i+1} = c
+  if (lane < 2) { // factorisation, with the first forward elimination
+    D = U1[side];
+    U = U2[side];
+    c = X[side];
+    double d1 = U1[2 + side], e1 = U2[2 + side], b1 = X[2 + side]; // (position 1; read past the side's end where len is 1, not used)
+    double L = U;
+    for (int i = 0; i + 1 < len; ++i) {
+      const int at = 2 * i + side;
+      const int nx = i + 2 < len ? at + 4 : at + 2;
+      const double d2 = U1[nx], e2 = U2[nx], b2 = X[nx]; // the next round's row
+      const bool sw = fabs(D) < fabs(L);
+      const double piv = sw ? L : floored(D);
+      const double rp = 1.0 / piv;
+      const double f = (sw ? D : L) * rp;
+      const double u1 = sw ? d1 : U, u2 = sw ? e1 : 0.0, y = sw ? b1 : c;
+      c = fma(-f, y, sw ? c : b1);
+      D = fma(-f, u1, sw ? U : d1);
+      U = sw ? -f * e1 : e1;
+      L = e1;
+      F[at] = f;
+      RP[at] = rp;
+      U1[at] = u1;
+      U2[at] = u2;
+      X[at] = y;
+      SW[at] = sw;
+      d1 = d2;
+      e1 = e2;
+      b1 = b2;
+    }
+  }
+  // the two middle equations D x_own + U x_other = c, eliminated with pivoting on x of side 0
+  const double D0 = __shfl_sync(0xffffffffu, D, 0), U0 = __shfl_sync(0xffffffffu, U, 0);
+  const double D1 = __shfl_sync(0xffffffffu, D, 1), V1 = __shfl_sync(0xffffffffu, U, 1);
+  const bool mid = fabs(D0) < fabs(V1); // the equation of side 1 is the pivot row
+  const double mr = 1.0 / (mid ? V1 : floored(D0));
+  const double mf = (mid ? D0 : V1) * mr;
+  const double mu = mid ? D1 : U0; // the pivot row's entry of x of side 1
+  const double ms = 1.0 / floored(fma(-mf, mu, mid ? U0 : D1));
+  __syncwarp();
+  for (int at = lane; at < N + 1; at += 32) // entries of positions without a pivot are not read
+    if (at / 2 + 1 < ((at & 1) ? h1 : h0)) {
+      const double rp = RP[at];
+      U1[at] *= rp;
+      U2[at] *= rp;
+    }
+  __syncwarp();
+  for (int it = 0; it < kTriIters; ++it) {
+    if (it > 0 && lane < 2) { // forward elimination
+      c = X[side];
+      int i = 0;
+      for (; i + 4 < len; i += 4) {
+        double f[4], b[4];
+        unsigned char sw[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int at = 2 * (i + u) + side;
+          f[u] = F[at];
+          sw[u] = SW[at];
+          b[u] = X[at + 2];
         }
-        PV[i] = 1.0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double y = sw[u] ? b[u] : c;
+          c = fma(-f[u], y, sw[u] ? c : b[u]);
+          X[2 * (i + u) + side] = y;
+        }
+      }
+      for (; i + 1 < len; ++i) {
+        const int at = 2 * i + side;
+        const double b = X[at + 2];
+        const bool sw = SW[at];
+        const double y = sw ? b : c;
+        c = fma(-F[at], y, sw ? c : b);
+        X[at] = y;
       }
     }
-    if (fabs(D[N - 1]) < tiny) D[N - 1] = D[N - 1] < 0.0 ? -tiny : tiny;
-    for (int i = 0; i < N; ++i) D[i] = 1.0 / D[i];
+    const double c0 = __shfl_sync(0xffffffffu, c, 0), c1 = __shfl_sync(0xffffffffu, c, 1);
+    const double xb = fma(-mf, mid ? c1 : c0, mid ? c0 : c1) * ms; // x of side 1
+    const double xa = fma(-mu, xb, mid ? c1 : c0) * mr;            // x of side 0
+    if (lane < 2) { // substitution, outwards
+      double x1 = side ? xb : xa, x2 = side ? xa : xb; // x_{i+1}, x_{i+2}
+      X[2 * (len - 1) + side] = x1;
+      int i = len - 2;
+      for (; i >= 3; i -= 4) {
+        double y[4], a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int at = 2 * (i - u) + side;
+          y[u] = X[at] * RP[at];
+          a[u] = U1[at];
+          b[u] = U2[at];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const double v = fma(-a[u], x1, fma(-b[u], x2, y[u]));
+          X[2 * (i - u) + side] = v;
+          x2 = x1;
+          x1 = v;
+        }
+      }
+      for (; i >= 0; --i) {
+        const int at = 2 * i + side;
+        const double v = fma(-U1[at], x1, fma(-U2[at], x2, X[at] * RP[at]));
+        X[at] = v;
+        x2 = x1;
+        x1 = v;
+      }
+    }
+    __syncwarp();
   }
-  __syncwarp();
-  for (int idx = lane; idx < kFactorRows * N; idx += 32) F[static_cast<size_t>(t) * kFactorRows * N + idx] = fs[idx];
-}
-
-// z_t <- (T - lambda_t I)^{-1} z_t, scaled to unit max-norm
-__global__ void __launch_bounds__(32) k_tri_solve(int N, const double* __restrict__ F, double* __restrict__ Z)
-{
-  ::trl_detail::pdl_enter();
-  extern __shared__ __align__(16) double fs[]; // 5 x N factors, N vector
-  const int t = blockIdx.x, lane = threadIdx.x;
-  for (int idx = lane; idx < kFactorRows * N; idx += 32) fs[idx] = F[static_cast<size_t>(t) * kFactorRows * N + idx];
-  double* x = fs + kFactorRows * N;
-  for (int i = lane; i < N; i += 32) x[i] = Z[static_cast<size_t>(t) * N + i];
-  __syncwarp();
-  if (lane == 0) {
-    const double* DL = fs;
-    const double* RD = fs + N;
-    const double* DU = fs + 2 * N;
-    const double* DU2 = fs + 3 * N;
-    const double* PV = fs + 4 * N;
-    double xi = x[0];
-    for (int i = 0; i + 1 < N; ++i) { // apply P and L, carrying x[i] in a register
-      const double xn = x[i + 1];
-      if (PV[i] == 0.0) {
-        x[i] = xi;
-        xi = xn - DL[i] * xi;
-      }
-      else {
-        x[i] = xn;
-        xi = xi - DL[i] * xn;
-      }
-    }
-    x[N - 1] = xi;
-    double x1 = x[N - 1] * RD[N - 1]; // x[i+1]
-    x[N - 1] = x1;
-    double x2 = 0.0; // x[i+2]
-    if (N > 1) {
-      const double v = (x[N - 2] - DU[N - 2] * x1) * RD[N - 2];
-      x[N - 2] = v;
-      x2 = x1;
-      x1 = v;
-    }
-    for (int i = N - 3; i >= 0; --i) {
-      const double v = (x[i] - DU[i] * x1 - DU2[i] * x2) * RD[i];
-      x[i] = v;
-      x2 = x1;
-      x1 = v;
-    }
-  }
-  __syncwarp();
-  double mx = 0.0;
-  for (int i = lane; i < N; i += 32) mx = fmax(mx, fabs(x[i]));
-  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const double inv = mx > 0.0 ? 1.0 / mx : 1.0;
-  for (int i = lane; i < N; i += 32) Z[static_cast<size_t>(t) * N + i] = x[i] * inv;
+  for (int i = lane; i < N; i += 32) Z[static_cast<size_t>(t) * N + i] = X[i < h0 ? 2 * i : 2 * (N - 1 - i) + 1];
 }
 
 // Orthonormalisation of the K vectors (rows of Z, ascending eigenvalues). Inverse iteration
@@ -1482,9 +1524,7 @@ const TriVariant* tri_variant(int device, int N)
   std::lock_guard<std::mutex> g(lock);
   if (!checked[device]) {
     checked[device] = true;
-    const bool common = cudaFuncSetAttribute(k_tri_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kFactorRows + 1) * kTriMaxN)) == cudaSuccess &&
-                        cudaFuncSetAttribute(k_tri_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * kFactorRows * kTriMaxN)) == cudaSuccess &&
-                        cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kWyRows + kWyVecs) * kTriMaxN)) == cudaSuccess &&
+    const bool common = cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kWyRows + kWyVecs) * kTriMaxN)) == cudaSuccess &&
                         cudaFuncSetAttribute(k_wy_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * kWyRows * kTriMaxN)) == cudaSuccess;
     for (int i = 0; i < kNumTriVariants && common; ++i) {
       const TriVariant& v = kTriVariants[i];
@@ -1522,10 +1562,10 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   ProfScope prof(h, PROF_SMALL_EIGEN, 16.0 * N * N);
   const int K = kvec > 0 ? kvec : 1;
   // workspace: A (N*N) | refl (N*N) | d | e | tau | w (N each) | Z (N*K) | X (N*K) |
-  // factors (5 N*K) | perm, sel, slot (N ints each) | zero flag, count
+  // E (K*K overlaps) | perm, sel, slot (N ints each) | zero flag, count
   const size_t NN = static_cast<size_t>(N) * N, NK = static_cast<size_t>(N) * K;
   const size_t nchunks = static_cast<size_t>(N - 2 + kWyRows - 1) / kWyRows;
-  const size_t doubles = 2 * NN + 4 * static_cast<size_t>(N) + (2 + kFactorRows) * NK + nchunks * kWyRows * kWyRows;
+  const size_t doubles = 2 * NN + 4 * static_cast<size_t>(N) + 2 * NK + static_cast<size_t>(K) * K + nchunks * kWyRows * kWyRows;
   const size_t ints = 3 * static_cast<size_t>(N) + 8;
   char* ws = static_cast<char*>(workspace(h, sizeof(double) * (doubles + 1) + sizeof(int) * ints + 256));
   if (!ws) return TRL_ENOMEM;
@@ -1537,8 +1577,8 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   double* w = tau + N;
   double* Z = w + N;
   double* X = Z + NK;
-  double* F = X + NK;
-  double* Tw = F + kFactorRows * NK;
+  double* E = X + NK;
+  double* Tw = E + static_cast<size_t>(K) * K;
   int* perm = reinterpret_cast<int*>(Tw + nchunks * kWyRows * kWyRows);
   int* sel = perm + N;
   int* slot = sel + N;
@@ -1565,12 +1605,8 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   if (int st = after_launch(h, "rank")) return st;
   launch(k_select, 1, kTriMaxVec, 0, h->stream, perm, K, sel, slot);
   if (int st = after_launch(h, "select")) return st;
-  launch(k_tri_factor, K, 32, sizeof(double) * kFactorRows * N, h->stream, d, e, N, w, sel, F, Z);
-  if (int st = after_launch(h, "tridiagonal factor")) return st;
-  for (int it = 0; it < kTriIters; ++it) {
-    launch(k_tri_solve, K, 32, sizeof(double) * (kFactorRows + 1) * N, h->stream, N, F, Z);
-    if (int st = after_launch(h, "inverse iteration")) return st;
-  }
+  launch(k_tri_vectors, K, 32, vectors_smem(N), h->stream, d, e, N, w, sel, Z);
+  if (int st = after_launch(h, "inverse iteration")) return st;
   launch(k_tri_cluster, K, kClusterThreads, 0, h->stream, N, K, w, sel, Z);
   if (int st = after_launch(h, "gram-schmidt")) return st;
   const int kt = (K + 7) / 8;
@@ -1579,9 +1615,9 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
     double* from = round == 0 ? Z : X;
     double* to = round == 0 ? X : Z;
     unsigned long long* check = round == 0 ? nullptr : emax;
-    launch(k_gs_gram, kt * (kt + 1) / 2, 256, 0, h->stream, N, K, from, F, check); // F: the factors are done with
+    launch(k_gs_gram, kt * (kt + 1) / 2, 256, 0, h->stream, N, K, from, E, check);
     if (int st = after_launch(h, "overlaps")) return st;
-    launch(k_gs_apply, apply_grid, 128, 0, h->stream, N, K, from, F, check, to);
+    launch(k_gs_apply, apply_grid, 128, 0, h->stream, N, K, from, E, check, to);
     if (int st = after_launch(h, "orthogonalise")) return st;
   }
   launch(k_tri_gs, 1, kTriThreads, 0, h->stream, N, K, Z, emax);
