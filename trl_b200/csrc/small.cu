@@ -433,7 +433,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 
 // Householder tridiagonalisation. A: N x N symmetric (full storage, max|A| in [0.5, 1)).
 // Outputs: d[N], e[N-1] of Q^T A Q with Q = H_0 ... H_{N-3}, H_k = I - tau_k u_k u_k^T, u_k
-// stored in refl[k*N + k+1 .. N-1] (not normalised).
+// stored in refl[k*ld + k+1 .. N-1] (not normalised).
 //
 // One cluster of kTriC CTAs of kTriW warps; row g belongs to CTA g % 16 and there to warp
 // (g / 16) % 8, which holds it in registers (lane l: columns l, l + 32, ...): row i of a warp
@@ -472,7 +472,7 @@ struct TriState {
 };
 
 struct TriArgs {
-  int N, g0, glast; // matrix size; this warp's first and last row
+  int N, ld, g0, glast; // matrix size, length of a reflector's row; this warp's first and last row
   bool keeper;
   uint32_t to_pairs, to_bar; // lane q: addresses in CTA q
   const double2* pairs;
@@ -503,7 +503,7 @@ __device__ __forceinline__ bool tri_steps(TriState<RPW>& st, const TriArgs& k)
 #pragma unroll
         for (int q = Q0; q < Q; ++q) {
           const int j = q * 32 + lane;
-          if (j >= s && j < N) k.refl[static_cast<size_t>(s - 1) * N + j] = st.u[q];
+          if (j >= s && j < N) k.refl[static_cast<size_t>(s - 1) * k.ld + j] = st.u[q];
         }
       }
       if (lane == 0) {
@@ -622,7 +622,7 @@ __device__ __forceinline__ void tri_phases(TriState<RPW>& st, const TriArgs& k)
 
 template <int RPW>
 __global__ void __launch_bounds__(kTriW * 32, 1)
-    k_tridiag(double* __restrict__ A, int N, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out,
+    k_tridiag(double* __restrict__ A, int N, int ld, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out,
               double* __restrict__ refl, int* status)
 {
   ::trl_detail::pdl_enter();
@@ -640,6 +640,7 @@ __global__ void __launch_bounds__(kTriW * 32, 1)
   }
   TriArgs k;
   k.N = N;
+  k.ld = ld;
   k.g0 = r + kTriC * warp;
   k.glast = k.g0 < N ? k.g0 + (N - 1 - k.g0) / kTriStride * kTriStride : -1;
   const int cta_rows = r < N ? (N - 1 - r) / kTriC + 1 : 0;
@@ -697,7 +698,7 @@ __device__ __forceinline__ double tri_block_sum(double v, double* slot)
 
 template <int C, int RPW, bool kGlobalRows>
 __global__ void __launch_bounds__(kTriThreads, 1)
-    k_tridiag_mem(double* __restrict__ A, int N, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out,
+    k_tridiag_mem(double* __restrict__ A, int N, int ld, double* __restrict__ dout, double* __restrict__ eout, double* __restrict__ tau_out,
                   double* __restrict__ refl, int* status)
 {
   ::trl_detail::pdl_enter();
@@ -832,7 +833,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
       if (j < N) {
         vn[j] = vj[e];
         wbuf[j] = w[e];
-        if (r == s % C && j > s && s < N - 2) refl[static_cast<size_t>(s) * N + j] = vj[e];
+        if (r == s % C && j > s && s < N - 2) refl[static_cast<size_t>(s) * ld + j] = vj[e];
       }
     }
     if (r == 0 && tid == 0) {
@@ -1309,111 +1310,164 @@ __global__ void __launch_bounds__(kTriThreads) k_tri_gs(int N, int K, double* __
 // Back-transform X = Q Z, Q = H_0 ... H_{N-3}, in chunks of kWyRows reflectors: a chunk
 // H_a ... H_b equals I - V T V^T (compact WY form, T upper triangular: T_ii = tau_i,
 // T[0:i, i] = -tau_i T[0:i, 0:i] V[:, 0:i]^T v_i), so a chunk is three small matrix
-// products on the vectors instead of kWyRows dependent reflector applications.
+// products on the vectors instead of kWyRows dependent reflector applications. Reflectors are
+// rows of `ld` doubles (an even number: 16-byte aligned rows).
 constexpr int kWyRows = 16;
-constexpr int kWyVecs = 1; // vectors per CTA: the chunk products are latency-bound, so one vector per CTA spreads them over K SMs
+constexpr int kWyThreads = 256;
+constexpr size_t kWyStageMax = 200 * 1024; // two chunks of reflectors in shared memory, or one
 
-// T of chunk c (reflectors c * kWyRows ...) into Tw[c][kWyRows][kWyRows]
-__global__ void __launch_bounds__(256) k_wy_factor(const double* __restrict__ refl, const double* __restrict__ tau, int N, double* __restrict__ Tw)
+__host__ __device__ __forceinline__ int refl_ld(int N) { return N + (N & 1); }
+
+// T of chunk c (reflectors c * kWyRows ...) into Tw[c][kWyRows][kWyRows], and the zeros of the
+// chunk's reflectors up to their first entry (from the multiple of 32 at or below it) into refl
+__global__ void __launch_bounds__(kWyThreads) k_wy_factor(double* __restrict__ refl, const double* __restrict__ tau, int N, int ld, double* __restrict__ Tw)
 {
   ::trl_detail::pdl_enter();
-  extern __shared__ __align__(16) double vs[]; // kWyRows x N
-  __shared__ double G[kWyRows][kWyRows], Tt[kWyRows][kWyRows];
+  constexpr int NW = kWyThreads / 32;
+  __shared__ double part[NW][3][64];
+  __shared__ double G[kWyRows][kWyRows + 1];
   const int R = N - 2;
   const int k0 = blockIdx.x * kWyRows;
   const int b = R - k0 < kWyRows ? R - k0 : kWyRows;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  stage(vs, refl + static_cast<size_t>(k0) * N, b * N);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int start = k0 & ~31;
+  for (int rr = warp; rr < b; rr += NW)
+    for (int i = start + lane; i <= k0 + rr; i += 32) refl[static_cast<size_t>(k0 + rr) * ld + i] = 0.0;
+  // G = V^T V: tiles (0, 0), (0, 1), (1, 1) of 8 x 8 on the tensor cores, entries split over the warps
+  double d0[3] = {0.0, 0.0, 0.0}, d1[3] = {0.0, 0.0, 0.0};
+  const double* v0 = refl + static_cast<size_t>(k0 + (g < b ? g : 0)) * ld;
+  const double* v1 = refl + static_cast<size_t>(k0 + (g + 8 < b ? g + 8 : 0)) * ld;
+#pragma unroll 4
+  for (int n0 = start + warp * 4; n0 < N; n0 += NW * 4) {
+    const int n = n0 + t4;
+    const double a0 = (g < b && n > k0 + g && n < N) ? v0[n] : 0.0; // v_k is zero up to entry k
+    const double a1 = (g + 8 < b && n > k0 + g + 8 && n < N) ? v1[n] : 0.0;
+    dmma_m8n8k4(d0[0], d1[0], a0, a0);
+    dmma_m8n8k4(d0[1], d1[1], a0, a1);
+    dmma_m8n8k4(d0[2], d1[2], a1, a1);
+  }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    part[warp][q][g * 8 + 2 * t4] = d0[q];
+    part[warp][q][g * 8 + 2 * t4 + 1] = d1[q];
+  }
   __syncthreads();
-  for (int rr = 0; rr < b; ++rr) // v_k is zero up to row k (refl holds nothing there)
-    for (int i = tid; i <= k0 + rr; i += blockDim.x) vs[rr * N + i] = 0.0;
-  __syncthreads();
-  for (int pq = warp; pq < b * b; pq += blockDim.x >> 5) {
-    const int p = pq / b, q = pq % b;
-    if (p >= q) continue; // strictly upper part: G[p][q] = v_p . v_q
+  if (tid < 192) {
     double s = 0.0;
-    for (int i = lane; i < N; i += 32) s = fma(vs[p * N + i], vs[q * N + i], s);
-    s = warp_sum(s);
-    if (lane == 0) G[p][q] = s;
+#pragma unroll
+    for (int q = 0; q < NW; ++q) s += part[q][tid >> 6][tid & 63];
+    const int tile = tid >> 6, e = tid & 63;
+    G[(tile == 2 ? 8 : 0) + (e >> 3)][(tile == 0 ? 0 : 8) + (e & 7)] = s;
   }
   __syncthreads();
-  if (warp == 0) {
-    for (int i = 0; i < b; ++i) {
-      const double ti = tau[k0 + i];
-      // lane j < i: T[j][i] = -tau_i sum_{m=j}^{i-1} T[j][m] G[m][i]
-      double v = 0.0;
-      if (lane < i) {
-        for (int m = lane; m < i; ++m) v = fma(Tt[lane][m], G[m][i], v);
-        v = -ti * v;
-      }
-      __syncwarp();
-      if (lane < i) Tt[lane][i] = v;
-      if (lane == i) Tt[i][i] = ti;
-      if (lane > i && lane < kWyRows) Tt[lane][i] = 0.0;
-      __syncwarp();
+  if (warp == 0 && lane < kWyRows) { // lane j: row j of T
+    double row[kWyRows];
+#pragma unroll
+    for (int i = 0; i < kWyRows; ++i) {
+      const double ti = i < b ? tau[k0 + i] : 0.0;
+      double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int m = 0; m < i; ++m) s4[m & 3] = fma(row[m], G[m][i], s4[m & 3]); // row[m] = 0 for m < lane
+      const double s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      row[i] = i < lane || i >= b ? 0.0 : (i == lane ? ti : -ti * s);
+      Tw[(static_cast<size_t>(blockIdx.x) * kWyRows + lane) * kWyRows + i] = row[i];
     }
-  }
-  __syncthreads();
-  for (int e = tid; e < kWyRows * kWyRows; e += blockDim.x) {
-    const int p = e / kWyRows, q = e % kWyRows;
-    Tw[static_cast<size_t>(blockIdx.x) * kWyRows * kWyRows + e] = (p < b && q < b) ? Tt[p][q] : 0.0;
   }
 }
 
-__global__ void __launch_bounds__(256) k_backtransform(const double* __restrict__ Z, int K, int N, const double* __restrict__ refl, const double* __restrict__ Tw,
-                                                       double* __restrict__ X)
+__device__ __forceinline__ void cp_async16(void* dst, const void* src)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
+}
+
+// One vector per CTA (the chunks are a chain, so the vectors spread over the SMs). While a chunk
+// is applied, the next one's reflectors arrive in the other half of the stage.
+// Measured on B200 with k_wy_factor (K = 40, N = 384 / K = 112, N = 512): 72 / 98 us
+// (before, each chunk loaded after the last was applied and T applied between barriers: 208 /
+// 315 us).
+__global__ void __launch_bounds__(kWyThreads) k_backtransform(const double* __restrict__ Z, int N, int ld, int stages, const double* __restrict__ refl, const double* __restrict__ Tw,
+                                                              double* __restrict__ X)
 {
   ::trl_detail::pdl_enter();
-  extern __shared__ __align__(16) double sm[]; // kWyRows x N reflectors | kWyVecs x N vectors
-  double* vs = sm;
-  double* xs = sm + kWyRows * N;
-  __shared__ double W[kWyRows][kWyVecs], W2[kWyRows][kWyVecs], Ts[kWyRows][kWyRows];
+  extern __shared__ __align__(16) double sm[]; // stages x kWyRows x ld reflectors | vector
+  constexpr int NW = kWyThreads / 32;
+  __shared__ double W[kWyRows], W2[NW][kWyRows];
+  double* const xs = sm + static_cast<size_t>(stages) * kWyRows * ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int t0 = blockIdx.x * kWyVecs;
-  const int nv = K - t0 < kWyVecs ? K - t0 : kWyVecs;
-  stage(xs, Z + static_cast<size_t>(t0) * N, nv * N);
+  for (int i = tid; i < N; i += kWyThreads) xs[i] = Z[static_cast<size_t>(blockIdx.x) * N + i];
   const int R = N - 2;
   const int nch = (R + kWyRows - 1) / kWyRows;
+  const auto fetch = [&](int c) { // chunk c's rows, entries from the multiple of 32 below its first
+    const int k0 = c * kWyRows, b = R - k0 < kWyRows ? R - k0 : kWyRows, start = k0 & ~31;
+    double* to = sm + static_cast<size_t>(c % stages) * kWyRows * ld;
+    for (int rr = warp; rr < b; rr += NW)
+      for (int i = start + 2 * lane; i < ld; i += 64) cp_async16(to + static_cast<size_t>(rr) * ld + i, refl + static_cast<size_t>(k0 + rr) * ld + i);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (stages > 1) fetch(nch - 1);
   for (int c = nch - 1; c >= 0; --c) {
-    const int k0 = c * kWyRows;
-    const int b = R - k0 < kWyRows ? R - k0 : kWyRows;
-    __syncthreads(); // previous chunk done with vs, Ts, W2
-    stage(vs, refl + static_cast<size_t>(k0) * N, b * N);
-    for (int e = tid; e < kWyRows * kWyRows; e += blockDim.x) Ts[e / kWyRows][e % kWyRows] = Tw[static_cast<size_t>(c) * kWyRows * kWyRows + e];
-    __syncthreads();
-    for (int rr = 0; rr < b; ++rr) // v_k is zero up to row k (refl holds nothing there)
-      for (int i = tid; i <= k0 + rr; i += blockDim.x) vs[rr * N + i] = 0.0;
-    __syncthreads();
-    // W = V^T X: warp per (row, vector) pair
-    for (int pv = warp; pv < b * nv; pv += blockDim.x >> 5) {
-      const int rr = pv / nv, v = pv % nv;
-      double s0 = 0.0, s1 = 0.0;
-      int i = lane;
+    const int k0 = c * kWyRows, b = R - k0 < kWyRows ? R - k0 : kWyRows, start = k0 & ~31;
+    if (stages > 1 && c > 0) {
+      fetch(c - 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    }
+    else {
+      if (stages == 1) fetch(c);
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    double tr[kWyRows]; // lane m < 16: row m of T
+#pragma unroll
+    for (int q = 0; q < kWyRows; ++q) tr[q] = lane < kWyRows ? __ldg(Tw + (static_cast<size_t>(c) * kWyRows + lane) * kWyRows + q) : 0.0;
+    __syncthreads(); // the chunk is there for all; the vector is as the last chunk left it
+    const double* vs = sm + static_cast<size_t>(c % stages) * kWyRows * ld;
+    // W = V^T x: warp w takes rows w and w + 8
+    {
+      const double* va = vs + static_cast<size_t>(warp) * ld;
+      const double* vb = vs + static_cast<size_t>(warp + NW) * ld;
+      const bool oka = warp < b, okb = warp + NW < b;
+      double sa0 = 0.0, sa1 = 0.0, sb0 = 0.0, sb1 = 0.0;
+      int i = start + lane;
+#pragma unroll 2
       for (; i + 32 < N; i += 64) {
-        s0 = fma(vs[rr * N + i], xs[v * N + i], s0);
-        s1 = fma(vs[rr * N + i + 32], xs[v * N + i + 32], s1);
+        const double x0 = xs[i], x1 = xs[i + 32];
+        sa0 = fma(oka ? va[i] : 0.0, x0, sa0);
+        sb0 = fma(okb ? vb[i] : 0.0, x0, sb0);
+        sa1 = fma(oka ? va[i + 32] : 0.0, x1, sa1);
+        sb1 = fma(okb ? vb[i + 32] : 0.0, x1, sb1);
       }
-      if (i < N) s0 = fma(vs[rr * N + i], xs[v * N + i], s0);
-      const double s = warp_sum(s0 + s1);
-      if (lane == 0) W[rr][v] = s;
+      if (i < N) {
+        sa0 = fma(oka ? va[i] : 0.0, xs[i], sa0);
+        sb0 = fma(okb ? vb[i] : 0.0, xs[i], sb0);
+      }
+      double s0 = sa0 + sa1, s1 = sb0 + sb1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      }
+      if (lane == 0) {
+        W[warp] = s0;
+        W[warp + NW] = s1;
+      }
     }
     __syncthreads();
-    if (tid < b * nv) { // W2 = T W
-      const int rr = tid / nv, v = tid % nv;
-      double s = 0.0;
-      for (int m = rr; m < b; ++m) s = fma(Ts[rr][m], W[m][v], s);
-      W2[rr][v] = s;
+    { // W2 = T W, by every warp for itself
+      double s4[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int q = 0; q < kWyRows; ++q) s4[q & 3] = fma(tr[q], W[q], s4[q & 3]);
+      if (lane < kWyRows) W2[warp][lane] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+      __syncwarp();
     }
-    __syncthreads();
-    for (int idx = tid; idx < nv * N; idx += blockDim.x) { // X -= V W2
-      const int v = idx / N, i = idx % N;
-      double x = xs[idx];
-      for (int rr = 0; rr < b; ++rr) x = fma(-vs[rr * N + i], W2[rr][v], x);
-      xs[idx] = x;
+    for (int i = start + tid; i < N; i += kWyThreads) { // x -= V W2
+      double s4[4] = {xs[i], 0.0, 0.0, 0.0};
+#pragma unroll
+      for (int rr = 0; rr < kWyRows; ++rr)
+        if (rr < b) s4[rr & 3] = fma(-vs[static_cast<size_t>(rr) * ld + i], W2[warp][rr], s4[rr & 3]);
+      xs[i] = (s4[0] + s4[1]) + (s4[2] + s4[3]);
     }
+    __syncthreads(); // done with the stage and with W
   }
-  __syncthreads();
-  for (int idx = tid; idx < nv * N; idx += blockDim.x) X[static_cast<size_t>(t0) * N + idx] = xs[idx];
+  for (int i = tid; i < N; i += kWyThreads) X[static_cast<size_t>(blockIdx.x) * N + i] = xs[i];
 }
 
 // selected ascending indices: sel[t] (ascending), slot[c] = t for rank c < K
@@ -1477,7 +1531,7 @@ __global__ void k_zero_cols(double* __restrict__ Y, int nblk, int bs, int K)
   }
 }
 
-using TriKernel = void (*)(double*, int, double*, double*, double*, double*, int*);
+using TriKernel = void (*)(double*, int, int, double*, double*, double*, double*, int*);
 
 struct TriVariant {
   TriKernel fn;
@@ -1524,8 +1578,7 @@ const TriVariant* tri_variant(int device, int N)
   std::lock_guard<std::mutex> g(lock);
   if (!checked[device]) {
     checked[device] = true;
-    const bool common = cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * (kWyRows + kWyVecs) * kTriMaxN)) == cudaSuccess &&
-                        cudaFuncSetAttribute(k_wy_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(double) * kWyRows * kTriMaxN)) == cudaSuccess;
+    const bool common = cudaFuncSetAttribute(k_backtransform, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kWyStageMax + sizeof(double) * kTriMaxN)) == cudaSuccess;
     for (int i = 0; i < kNumTriVariants && common; ++i) {
       const TriVariant& v = kTriVariants[i];
       if (cudaFuncSetAttribute(v.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(tridiag_smem(v.max_n, v.C, v.rows))) != cudaSuccess) continue;
@@ -1561,17 +1614,18 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   }
   ProfScope prof(h, PROF_SMALL_EIGEN, 16.0 * N * N);
   const int K = kvec > 0 ? kvec : 1;
-  // workspace: A (N*N) | refl (N*N) | d | e | tau | w (N each) | Z (N*K) | X (N*K) |
+  // workspace: refl (N*ld) | A (N*N) | d | e | tau | w (N each) | Z (N*K) | X (N*K) |
   // E (K*K overlaps) | perm, sel, slot (N ints each) | zero flag, count
   const size_t NN = static_cast<size_t>(N) * N, NK = static_cast<size_t>(N) * K;
   const size_t nchunks = static_cast<size_t>(N - 2 + kWyRows - 1) / kWyRows;
-  const size_t doubles = 2 * NN + 4 * static_cast<size_t>(N) + 2 * NK + static_cast<size_t>(K) * K + nchunks * kWyRows * kWyRows;
+  const int ld = refl_ld(N);
+  const size_t doubles = NN + static_cast<size_t>(N) * ld + 4 * static_cast<size_t>(N) + 2 * NK + static_cast<size_t>(K) * K + nchunks * kWyRows * kWyRows;
   const size_t ints = 3 * static_cast<size_t>(N) + 8;
   char* ws = static_cast<char*>(workspace(h, sizeof(double) * (doubles + 1) + sizeof(int) * ints + 256));
   if (!ws) return TRL_ENOMEM;
-  double* A = reinterpret_cast<double*>(ws);
-  double* refl = A + NN;
-  double* d = refl + NN;
+  double* refl = reinterpret_cast<double*>(ws);
+  double* A = refl + static_cast<size_t>(N) * ld;
+  double* d = A + NN;
   double* e = d + N;
   double* tau = e + N;
   double* w = tau + N;
@@ -1596,7 +1650,7 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
     tri_config(*tv, N, h->stream, cfg, attr);
-    cudaLaunchKernelEx(&cfg, tv->fn, A, N, d, e, tau, refl, h->d_status);
+    cudaLaunchKernelEx(&cfg, tv->fn, A, N, ld, d, e, tau, refl, h->d_status);
     if (int st = after_launch(h, "tridiagonalise")) return st;
   }
   launch(k_bisect, N, kBisectPoints, sizeof(double2) * (N + 1), h->stream, d, e, N, w);
@@ -1623,9 +1677,11 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   launch(k_tri_gs, 1, kTriThreads, 0, h->stream, N, K, Z, emax);
   if (int st = after_launch(h, "gram-schmidt")) return st;
   const int nch = (N - 2 + kWyRows - 1) / kWyRows;
-  launch(k_wy_factor, nch, 256, sizeof(double) * kWyRows * N, h->stream, refl, tau, N, Tw);
+  launch(k_wy_factor, nch, kWyThreads, 0, h->stream, refl, tau, N, ld, Tw);
   if (int st = after_launch(h, "wy factor")) return st;
-  launch(k_backtransform, (K + kWyVecs - 1) / kWyVecs, 256, sizeof(double) * (kWyRows + kWyVecs) * N, h->stream, Z, K, N, refl, Tw, X);
+  const size_t chunk = sizeof(double) * kWyRows * ld;
+  const int stages = 2 * chunk <= kWyStageMax ? 2 : 1;
+  launch(k_backtransform, K, kWyThreads, stages * chunk + sizeof(double) * N, h->stream, Z, N, ld, stages, refl, Tw, X);
   if (int st = after_launch(h, "back-transform")) return st;
   launch(k_scatter_partial, g, 256, 0, h->stream, X, slot, nblk, bs, kvec, evecs);
   if (int st = after_launch(h, "scatter")) return st;
