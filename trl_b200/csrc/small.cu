@@ -454,7 +454,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // warp leaves when its last row has been sent; the warp with the CTA's last row arms the
 // barrier of each step. Steps [128 F, 128 F + 127] run a body of their own without the rows
 // and columns before 128 F, so that the body has no branches and its chains overlap.
-// Measured on B200 (ncu, us a launch): N = 384 525, N = 512 920, N = 160 120. The kernel before
+// Measured on B200 (ncu, us a launch): N = 384 535, N = 512 965, N = 160 120. The kernel before
 // this one (rows in shared memory, two cluster barriers and three CTA barriers a step, the
 // sums over all CTAs' partials): 1,719, 2,604, 480. At N = 384 a step is about 2,300 cycles:
 // sending and waiting 660, reading the pairs and the first sum 440, rows and columns 750, the
@@ -568,7 +568,9 @@ __device__ __forceinline__ bool tri_steps(TriState<RPW>& st, const TriArgs& k)
       n4[q & 3] = fma(xq, xq, n4[q & 3]);
 #pragma unroll
       for (int i = F; i < RPW; ++i) {
-        const double aq = fma(-st.ug[i], wq, fma(-wg[i], uq, st.a[i][q]));
+        // the two products summed before they are subtracted: subtracted one after the other
+        // they lose half a digit of the eigenvalues where A is near a multiple of I
+        const double aq = st.a[i][q] - fma(st.ug[i], wq, wg[i] * uq);
         st.a[i][q] = aq;
         t2[i][q & 1] = fma(aq, xq, t2[i][q & 1]);
         if (q == Q0) st.col[i] = aq;
@@ -606,7 +608,7 @@ __device__ __forceinline__ bool tri_steps(TriState<RPW>& st, const TriArgs& k)
       st.t[i] = fma(st.col[i], st.us, tn[i]);
       if (k.g0 + i * kTriStride == s + 1) st.ug[i] = st.us;
     }
-    st.half = norm * (norm + fabs(x0));
+    st.half = norm > 0.0 ? 0.5 * fma(st.us, st.us, xnorm2) : 0.0;
     st.eprev = beta;
   }
   return true;
@@ -767,7 +769,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
 #pragma unroll
         for (int i = 0; i < RPW; ++i)
           if (on[i]) {
-            a[i] = fma(-vg[i], wpj, fma(-wg[i], vpj, a[i]));
+            a[i] -= fma(vg[i], wpj, wg[i] * vpj);
             rl[i][j] = a[i];
             acc[i] = fma(a[i], vjj, acc[i]);
             if (j == s) col[i] = a[i];
