@@ -48,21 +48,17 @@ __global__ void k_mb_set_diag(double* __restrict__ dst, DiagValues d, int bs)
   if (i < bs) dst[i * bs + i] = d.v[i];
 }
 
-// max |T_ij| over the block matrix (one CTA) into *out
-__global__ void __launch_bounds__(1024) k_max_abs(const double* __restrict__ T, int64_t count, double* __restrict__ out)
+// max |T_ij| over the block matrix into *out, which holds zero before: non-negative doubles order
+// like their bit patterns. Spread over the SMs (one CTA took 27 us for 384 x 384 entries).
+__global__ void __launch_bounds__(256) k_max_abs(const double* __restrict__ T, int64_t count, unsigned long long* __restrict__ out)
 {
   ::trl_detail::pdl_enter();
-  __shared__ double red[32];
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   double m = 0.0;
-  for (int64_t e = threadIdx.x; e < count; e += blockDim.x) m = fmax(m, fabs(T[e]));
+#pragma unroll 4
+  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < count; e += stride) m = fmax(m, fabs(T[e]));
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0) *out = m;
-  }
+  if ((threadIdx.x & 31) == 0 && m > 0.0) atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(m)));
 }
 
 // Entries below kFlushRel * max|T| are set to zero when the dense copy is assembled: they
@@ -108,15 +104,20 @@ __global__ void k_rank(const double* __restrict__ w, int N, const double* __rest
   ::trl_detail::pdl_enter();
   const double unscale = tmax ? scalbn(1.0, scale_exponent(*tmax)) : 1.0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && *syevd_info != 0) atomicOr(status, TRL_DEV_EIGEN);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    const double ai = fabs(w[i]);
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int i = blockIdx.x * nw + (threadIdx.x >> 5); i < N; i += gridDim.x * nw) { // a warp per eigenvalue
+    // |w| ordered by bit pattern: the order of the values, and a permutation even with NaNs
+    const long long ai = __double_as_longlong(fabs(w[i]));
     int r = 0;
-    for (int j = 0; j < N; ++j) {
-      const double aj = fabs(w[j]);
+    for (int j = lane; j < N; j += 32) {
+      const long long aj = __double_as_longlong(fabs(w[j]));
       r += (aj > ai) || (aj == ai && j < i);
     }
-    perm[r] = i;
-    evals_sorted[r] = w[i] * unscale;
+    r = __reduce_add_sync(0xffffffffu, r);
+    if (lane == 0) {
+      perm[r] = i;
+      evals_sorted[r] = w[i] * unscale;
+    }
   }
 }
 
@@ -142,16 +143,16 @@ __global__ void k_count_converged(const double* __restrict__ A, const int* __res
 {
   ::trl_detail::pdl_enter();
   const int N = nblk * bs;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncheck; c += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c = blockIdx.x * nw + (threadIdx.x >> 5); c < ncheck; c += gridDim.x * nw) { // a warp per pair, a lane per entry of beta y
     const double* y = A + static_cast<int64_t>(perm[c]) * N + (nblk - 1) * bs;
-    double nrm2 = 0.0;
-    for (int i = 0; i < bs; ++i) {
-      double s = 0.0;
-      for (int k = 0; k < bs; ++k) s += beta[i * bs + k] * y[k];
-      nrm2 += s * s;
-    }
+    double v = 0.0;
+    if (lane < bs)
+      for (int k = 0; k < bs; ++k) v = fma(beta[lane * bs + k], y[k], v);
+    double nrm2 = v * v;
+    for (int o = 16; o > 0; o >>= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
     const double denom = fmax(fabs(evals_sorted[c]), DBL_EPSILON);
-    if (sqrt(nrm2) / denom < tol) atomicAdd(count, 1);
+    if (lane == 0 && sqrt(nrm2) / denom < tol) atomicAdd(count, 1);
   }
 }
 
@@ -280,19 +281,20 @@ int trl_cuda_small_eigen(trl_cuda_handle h, const double* T, int nblk, int bs, c
   }
 
   const unsigned g = grid_for(h, static_cast<int64_t>(N) * N, 256, 4);
-  launch(k_max_abs, 1, 1024, 0, h->stream, T, static_cast<int64_t>(N) * N, tmax);
+  cudaMemsetAsync(tmax, 0, sizeof *tmax, h->stream);
+  launch(k_max_abs, grid_for(h, static_cast<int64_t>(N) * N, 1024, 1), 256, 0, h->stream, T, static_cast<int64_t>(N) * N, reinterpret_cast<unsigned long long*>(tmax));
   launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, 0, A);
   if (int st = after_launch(h, "assemble")) return st;
   cs = cusolverDnDsyevd(sh, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, N, A, N, w, static_cast<double*>(h->syevd_work), lwork, info);
   if (cs != CUSOLVER_STATUS_SUCCESS) return set_error(h, TRL_ECUDA, "syevd failed (%d)", static_cast<int>(cs));
-  launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, static_cast<const double*>(nullptr), perm, evals, info, h->d_status);
+  launch(k_rank, (N + 7) / 8, 256, 0, h->stream, w, N, static_cast<const double*>(nullptr), perm, evals, info, h->d_status);
   if (int st = after_launch(h, "rank")) return st;
   launch(k_scatter_evecs, g, 256, 0, h->stream, A, perm, nblk, bs, evecs);
   if (int st = after_launch(h, "scatter")) return st;
   cudaMemsetAsync(count, 0, sizeof(int), h->stream);
   const int ncheck = nev < N ? nev : N;
   if (ncheck > 0) {
-    launch(k_count_converged, (ncheck + 127) / 128, 128, 0, h->stream, A, perm, evals, beta, nblk, bs, ncheck, tol, count);
+    launch(k_count_converged, (ncheck + 3) / 4, 128, 0, h->stream, A, perm, evals, beta, nblk, bs, ncheck, tol, count);
     if (int st = after_launch(h, "count")) return st;
   }
   char* pin = static_cast<char*>(pinned(h, w_bytes + 64));
@@ -1507,16 +1509,16 @@ __global__ void k_count_partial(const double* __restrict__ X, const int* __restr
 {
   ::trl_detail::pdl_enter();
   const int N = nblk * bs;
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < ncheck; c += gridDim.x * blockDim.x) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int c = blockIdx.x * nw + (threadIdx.x >> 5); c < ncheck; c += gridDim.x * nw) { // a warp per pair, a lane per entry of beta y
     const double* y = X + static_cast<int64_t>(slot[c]) * N + (nblk - 1) * bs;
-    double nrm2 = 0.0;
-    for (int i = 0; i < bs; ++i) {
-      double s = 0.0;
-      for (int k = 0; k < bs; ++k) s += beta[i * bs + k] * y[k];
-      nrm2 += s * s;
-    }
+    double v = 0.0;
+    if (lane < bs)
+      for (int k = 0; k < bs; ++k) v = fma(beta[lane * bs + k], y[k], v);
+    double nrm2 = v * v;
+    for (int o = 16; o > 0; o >>= 1) nrm2 += __shfl_xor_sync(0xffffffffu, nrm2, o);
     const double denom = fmax(fabs(evals_sorted[c]), DBL_EPSILON);
-    if (sqrt(nrm2) / denom < tol) atomicAdd(count, 1);
+    if (lane == 0 && sqrt(nrm2) / denom < tol) atomicAdd(count, 1);
   }
 }
 
@@ -1617,12 +1619,12 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   ProfScope prof(h, PROF_SMALL_EIGEN, 16.0 * N * N);
   const int K = kvec > 0 ? kvec : 1;
   // workspace: refl (N*ld) | A (N*N) | d | e | tau | w (N each) | Z (N*K) | X (N*K) |
-  // E (K*K overlaps) | perm, sel, slot (N ints each) | zero flag, count
+  // E (K*K overlaps) | perm, sel, slot (N ints each) | max|T|, largest overlap, flags
   const size_t NN = static_cast<size_t>(N) * N, NK = static_cast<size_t>(N) * K;
   const size_t nchunks = static_cast<size_t>(N - 2 + kWyRows - 1) / kWyRows;
   const int ld = refl_ld(N);
   const size_t doubles = NN + static_cast<size_t>(N) * ld + 4 * static_cast<size_t>(N) + 2 * NK + static_cast<size_t>(K) * K + nchunks * kWyRows * kWyRows;
-  const size_t ints = 3 * static_cast<size_t>(N) + 8;
+  const size_t ints = 3 * static_cast<size_t>(N);
   char* ws = static_cast<char*>(workspace(h, sizeof(double) * (doubles + 1) + sizeof(int) * ints + 256));
   if (!ws) return TRL_ENOMEM;
   double* refl = reinterpret_cast<double*>(ws);
@@ -1638,16 +1640,15 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   int* perm = reinterpret_cast<int*>(Tw + nchunks * kWyRows * kWyRows);
   int* sel = perm + N;
   int* slot = sel + N;
-  int* flags = slot + N; // [0] = 0 (no solver error), [1] = converged count
   double* tmax = reinterpret_cast<double*>(ws + (sizeof(double) * doubles + sizeof(int) * ints + 15) / 16 * 16);
   auto* emax = reinterpret_cast<unsigned long long*>(tmax + 1);
+  int* flags = reinterpret_cast<int*>(tmax + 2); // [0] = 0 (no solver error), [1] = converged count
 
   const unsigned g = grid_for(h, static_cast<int64_t>(N) * N, 256, 4);
-  cudaMemsetAsync(emax, 0, sizeof *emax, h->stream);
-  launch(k_max_abs, 1, 1024, 0, h->stream, T, static_cast<int64_t>(N) * N, tmax);
+  cudaMemsetAsync(tmax, 0, 2 * sizeof(double) + 2 * sizeof(int), h->stream); // tmax, emax, flags
+  launch(k_max_abs, grid_for(h, static_cast<int64_t>(N) * N, 1024, 1), 256, 0, h->stream, T, static_cast<int64_t>(N) * N, reinterpret_cast<unsigned long long*>(tmax));
   launch(k_assemble_dense, g, 256, 0, h->stream, T, nblk, bs, tmax, 1, A);
   if (int st = after_launch(h, "assemble")) return st;
-  cudaMemsetAsync(flags, 0, 2 * sizeof(int), h->stream);
   {
     cudaLaunchConfig_t cfg{};
     cudaLaunchAttribute attr{};
@@ -1657,7 +1658,7 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   }
   launch(k_bisect, N, kBisectPoints, sizeof(double2) * (N + 1), h->stream, d, e, N, w);
   if (int st = after_launch(h, "bisect")) return st;
-  launch(k_rank, (N + 255) / 256, 256, 0, h->stream, w, N, tmax, perm, evals, flags, h->d_status);
+  launch(k_rank, (N + 7) / 8, 256, 0, h->stream, w, N, tmax, perm, evals, flags, h->d_status);
   if (int st = after_launch(h, "rank")) return st;
   launch(k_select, 1, kTriMaxVec, 0, h->stream, perm, K, sel, slot);
   if (int st = after_launch(h, "select")) return st;
@@ -1689,7 +1690,7 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
   if (int st = after_launch(h, "scatter")) return st;
   const int ncheck = nev < kvec ? nev : kvec;
   if (ncheck > 0) {
-    launch(k_count_partial, (ncheck + 127) / 128, 128, 0, h->stream, X, slot, evals, beta, nblk, bs, ncheck, tol, flags + 1);
+    launch(k_count_partial, (ncheck + 3) / 4, 128, 0, h->stream, X, slot, evals, beta, nblk, bs, ncheck, tol, flags + 1);
     if (int st = after_launch(h, "count")) return st;
   }
   const size_t w_bytes = sizeof(double) * N;
