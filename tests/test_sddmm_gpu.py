@@ -1,0 +1,40 @@
+"""SDDMM and eigenvalue adjoint over the forms their kernel distinguishes: columns per lane and
+lanes per row (k odd and even, below, at and above the 16 of one round), coefficients by value
+(k <= 256) and from memory, rows of 0 entries to more than a warp sweeps, X aligned to 8 bytes only.
+
+Tolerance: each output sums k products of three factors in 64 bits, in some order: an error of at
+most (k + 2) eps times the sum of magnitudes (k - 1 additions, 2 multiplications, and the last
+rounding); 2 (k + 2) eps leaves room for the reference's own.
+"""
+import numpy as np
+import pytest
+import torch
+
+from trl_b200 import native
+from trl_b200 import problems as P
+
+from test_kernels_gpu import _long_row_csr, dev, host
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+
+
+@pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 9, 16, 17, 18, 33, 256, 300])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_sddmm_forms(cuda_handle, k, offset):
+    rng = np.random.default_rng(k)
+    for A in (_long_row_csr(rng, 700), P.laplace2d(9), P.diagonal(3)):
+        X = rng.standard_normal((A.n, k))
+        w = rng.uniform(0.5, 2.0, k)
+        Xd = torch.zeros(A.n * k + offset, dtype=torch.float64, device="cuda")[offset:].view(A.n, k)
+        Xd.copy_(torch.from_numpy(X))
+        rows = A.row_indices()
+        terms = w * X[rows] * X[A.colind]
+        bound = 2 * (k + 2) * EPS * np.abs(terms).sum(1)
+        Ad = native.DeviceCSRTensors.from_host(A)
+        out = torch.full((A.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+        cuda_handle.sddmm(Ad, Xd, dev(w), out)
+        assert np.all(np.abs(host(out) - terms.sum(1)) <= bound)
+        out.fill_(float("nan"))
+        cuda_handle.eigen_adjoint(Ad, Xd, np.arange(1.0, k + 1.0), w, out)
+        assert np.all(np.abs(host(out) - terms.sum(1)) <= bound)
