@@ -20,7 +20,7 @@ EPS = np.finfo(np.float64).eps
 
 
 @pytest.mark.parametrize("k", [1, 2, 3, 4, 5, 8, 9, 16, 17, 18, 33, 256, 300])
-@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("offset", [0, 1, 2])
 def test_sddmm_forms(cuda_handle, k, offset):
     rng = np.random.default_rng(k)
     for A in (_long_row_csr(rng, 700), P.laplace2d(9), P.diagonal(3)):

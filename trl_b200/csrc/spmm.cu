@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -222,110 +223,126 @@ __global__ void __launch_bounds__(kThreads, SpmmShape<T, BS>::MINB) k_spmm(int64
 }
 
 // ---- SDDMM: out[p] = sum_c w[c] X[row(p), c] X[col(p), c]
-// A group of L lanes owns a row; a lane carries VEC adjacent columns of the k at a time, so a
-// gathered row of X is one request of L * VEC * 8 bytes. A group takes its row's entries L at a
-// time: one coalesced load of their columns, L gathers in flight, then the L sums over the L lanes
-// by halving exchanges (lane q ends with entry q: L - 1 shuffles instead of L log L, and a
-// coalesced store). Rows longer than kSddmmLong are finished by all groups of the warp.
-// Bound by the gathers' L1/L2 traffic, nnz * k * 8 bytes.
-// Measured on B200, 512^2 five-point pattern (nnz = 1.31 M), k = 16: SDDMM_FIGURES
+// A warp owns `rpw` rows and takes their entries 32 at a time, whatever rows they belong to (a lane
+// finds its entry's row by bisection among the row starts the warp's lanes hold), so short rows
+// leave no lane idle and long ones are shared. Of the 32 entries a group of L lanes takes L: a lane
+// carries VEC adjacent columns of the k at a time, so a gathered row of X is one request of
+// L * VEC * 8 bytes, and the L sums over the L lanes go by halving exchanges (lane q ends with entry
+// q: L - 1 shuffles instead of L log L, and a coalesced store).
+// Bound by the L1/L2 traffic of the rows of X, 2 nnz * k * 8 bytes.
+// Measured on B200, 512^2 five-point pattern (nnz = 1.31 M) and its diagonal, k = 16, together:
+// 41 us (a lane per entry of one row per warp, X uncoalesced: 255 us with its copies and waits; a row
+// per group of 8 lanes and 16-byte pieces: 63 us; entries 32 at a time, 16-byte pieces: 57 us).
 constexpr int kSddmmMaxCoef = 256; // coefficients passed by value (2 KB of kernel parameters)
-constexpr int kSddmmLong = 32;
 
 struct SddmmCoef {
   double v[kSddmmMaxCoef];
 };
 
+template <int VEC>
+__device__ __forceinline__ void load_cols(const double* p, double (&out)[VEC])
+{
+  if constexpr (VEC == 4)
+    asm volatile("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(out[0]), "=d"(out[1]), "=d"(out[2]), "=d"(out[3]) : "l"(p));
+  else
+    load_vec<double, VEC>(p, out);
+}
+
 // w in device memory, or (null) by value in cf; the CTA keeps them in shared memory either way
 // as far as they fit kSddmmMaxCoef
 template <int L, int VEC>
 __global__ void __launch_bounds__(kThreads) k_sddmm(int64_t n, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, const double* __restrict__ X, int k,
-                                                    const double* __restrict__ w, const __grid_constant__ SddmmCoef cf, double* __restrict__ out)
+                                                    const double* __restrict__ w, const __grid_constant__ SddmmCoef cf, int rpw, double* __restrict__ out)
 {
   ::trl_detail::pdl_enter();
   __shared__ double ws[kSddmmMaxCoef];
   for (int c = threadIdx.x; c < k && c < kSddmmMaxCoef; c += kThreads) ws[c] = w ? w[c] : cf.v[c];
   __syncthreads();
   const auto coef = [&](int c) { return c < kSddmmMaxCoef ? ws[c] : __ldg(w + c); };
-  constexpr int RPW = 32 / L; // rows per warp step
-  const int lane = threadIdx.x & 31, sub = lane % L, grp = lane / L;
-  const unsigned gmask = L == 32 ? 0xffffffffu : ((1u << L) - 1u) << (grp * L);
-  const int64_t step = static_cast<int64_t>(gridDim.x) * (kThreads / 32) * RPW;
-
-  // out[p] for the cnt <= L entries p .. of row `row`
-  const auto entries = [&](int64_t row, int p, int cnt) {
-    const int mycol = sub < cnt ? __ldg(colind + p + sub) : 0;
-    double s[L];
+  const int lane = threadIdx.x & 31, sub = lane % L;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * (kThreads / 32) * rpw;
+  for (int64_t r0 = (static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5)) * rpw; r0 < n; r0 += step) {
+    const int start = __ldg(rowptr + min(r0 + lane, n)); // lane l < rpw: start of row r0 + l (rows past n are empty)
+    const int pend = __ldg(rowptr + min(r0 + rpw, n));
+    const int first = __shfl_sync(0xffffffffu, start, 0);
+    int col = lane < pend - first ? __ldg(colind + first + lane) : 0;
+    for (int left = pend - first; left > 0; left -= 32) { // entries not taken yet
+      const int p = pend - left + lane;
+      const int next = lane + 32 < left ? __ldg(colind + p + 32) : 0;
+      int at = 0; // the last row that starts at or before p
 #pragma unroll
-    for (int e = 0; e < L; ++e) s[e] = 0.0;
-    for (int c0 = sub * VEC; c0 - sub * VEC < k; c0 += L * VEC) { // the same number of rounds for all lanes of the group
-      double xr[VEC];
-#pragma unroll
-      for (int v = 0; v < VEC; ++v) xr[v] = 0.0;
-      if (c0 < k) {
-        load_vec<double, VEC>(X + row * k + c0, xr);
-#pragma unroll
-        for (int v = 0; v < VEC; ++v) xr[v] *= coef(c0 + v);
+      for (int h = 16; h > 0; h >>= 1) {
+        const int v = __shfl_sync(0xffffffffu, start, at + h);
+        if (at + h < rpw && v <= p) at += h;
       }
+      const int row = static_cast<int>(r0) + at;
+      const int cnt = min(max(left - (lane - sub), 0), L); // entries of this group
+      double s[L];
 #pragma unroll
-      for (int e = 0; e < L; ++e) {
-        const int col = __shfl_sync(gmask, mycol, e, L);
-        if (e < cnt && c0 < k) {
-          double xc[VEC];
-          load_vec<double, VEC>(X + static_cast<int64_t>(col) * k + c0, xc);
+      for (int e = 0; e < L; ++e) s[e] = 0.0;
+      for (int c0 = sub * VEC; c0 - sub * VEC < k; c0 += L * VEC) { // the same number of rounds for all lanes
+        double cw[VEC];
 #pragma unroll
-          for (int v = 0; v < VEC; ++v) s[e] = fma(xr[v], xc[v], s[e]);
+        for (int v = 0; v < VEC; ++v) cw[v] = c0 < k ? coef(c0 + v) : 0.0;
+        int held = -1; // the row whose products with the coefficients are in xw
+        double xw[VEC];
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) xw[v] = 0.0;
+#pragma unroll
+        for (int e = 0; e < L; ++e) {
+          const int er = __shfl_sync(0xffffffffu, row, e, L), ec = __shfl_sync(0xffffffffu, col, e, L);
+          if (e < cnt && c0 < k) {
+            double xc[VEC];
+            load_cols<VEC>(X + static_cast<int64_t>(ec) * k + c0, xc);
+            if (er != held) {
+              load_cols<VEC>(X + static_cast<int64_t>(er) * k + c0, xw);
+#pragma unroll
+              for (int v = 0; v < VEC; ++v) xw[v] *= cw[v];
+              held = er;
+            }
+#pragma unroll
+            for (int v = 0; v < VEC; ++v) s[e] = fma(xw[v], xc[v], s[e]);
+          }
         }
       }
-    }
 #pragma unroll
-    for (int h = L / 2; h > 0; h >>= 1) { // lanes with bit h keep the upper half of the entries
-      const bool up = (sub & h) != 0;
+      for (int h = L / 2; h > 0; h >>= 1) { // lanes with bit h keep the upper half of the entries
+        const bool up = (sub & h) != 0;
 #pragma unroll
-      for (int e = 0; e < h; ++e) {
-        const double give = up ? s[e] : s[e + h];
-        const double got = __shfl_xor_sync(gmask, give, h);
-        s[e] = (up ? s[e + h] : s[e]) + got;
+        for (int e = 0; e < h; ++e) {
+          const double give = up ? s[e] : s[e + h];
+          const double got = __shfl_xor_sync(0xffffffffu, give, h);
+          s[e] = (up ? s[e + h] : s[e]) + got;
+        }
       }
-    }
-    if (sub < cnt) out[p + sub] = s[0];
-  };
-
-  for (int64_t r0 = (static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5)) * RPW; r0 < n; r0 += step) {
-    const int64_t row = r0 + grp;
-    const int kb = row < n ? __ldg(rowptr + row) : 0, ke = row < n ? __ldg(rowptr + row + 1) : 0;
-    const int ks = min(ke, kb + kSddmmLong);
-    for (int p = kb; p < ks; p += L) entries(row, p, min(L, ks - p));
-    __syncwarp();
-    for (unsigned m = __ballot_sync(0xffffffffu, sub == 0 && ks < ke); m != 0; m &= m - 1) {
-      const int src = __ffs(m) - 1; // first lane of a group with a long row
-      const int rb = __shfl_sync(0xffffffffu, ks, src), re = __shfl_sync(0xffffffffu, ke, src);
-      for (int p = rb + grp * L; p < re; p += 32) entries(r0 + src / L, p, min(L, re - p));
-      __syncwarp();
+      if (lane < left) out[p] = s[0];
+      col = next;
     }
   }
 }
 
-// lanes per row by k: a lane's VEC columns at a time cover k in one round up to k = 8 VEC
+// lanes per entry by k: a lane's VEC columns at a time cover k in one round up to k = 8 VEC
 int launch_sddmm(trl_cuda_context* h, const trl_csr* P, const double* X, int k, const double* w, const SddmmCoef& cf, double* out)
 {
-  const bool vec = k % 2 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0; // 16-byte rows
-  const int need = vec ? k / 2 : k;
-  const auto run = [&](auto kernel, int rpw) {
-    launch(kernel, grid_for(h, (P->n + rpw - 1) / rpw, kThreads / 32, 8), kThreads, 0, h->stream, P->n, P->rowptr, P->colind, X, k, w, cf, out);
+  const auto aligned = [&](int v) { return k % v == 0 && reinterpret_cast<uintptr_t>(X) % (v * sizeof(double)) == 0; }; // every row of X
+  const int vec = aligned(4) ? 4 : (aligned(2) ? 2 : 1);
+  const int need = k / vec;
+  // rows per warp: 32, fewer where that would leave SMs without two warps per scheduler
+  int rpw = 32;
+  while (rpw > 4 && P->n < static_cast<int64_t>(rpw) * h->num_sms * 8) rpw /= 2;
+  const auto run = [&](auto kernel) {
+    launch(kernel, grid_for(h, (P->n + rpw - 1) / rpw, kThreads / 32, 8), kThreads, 0, h->stream, P->n, P->rowptr, P->colind, X, k, w, cf, rpw, out);
   };
-  if (vec) {
-    if (need <= 1) run(k_sddmm<1, 2>, 32);
-    else if (need <= 2) run(k_sddmm<2, 2>, 16);
-    else if (need <= 4) run(k_sddmm<4, 2>, 8);
-    else run(k_sddmm<8, 2>, 4);
-  }
-  else {
-    if (need <= 1) run(k_sddmm<1, 1>, 32);
-    else if (need <= 3) run(k_sddmm<2, 1>, 16);
-    else if (need <= 5) run(k_sddmm<4, 1>, 8);
-    else run(k_sddmm<8, 1>, 4);
-  }
+  const auto lanes = [&](auto v) {
+    constexpr int VEC = decltype(v)::value;
+    if (need <= 1) run(k_sddmm<1, VEC>);
+    else if (need <= 2) run(k_sddmm<2, VEC>);
+    else if (need <= 4) run(k_sddmm<4, VEC>);
+    else run(k_sddmm<8, VEC>);
+  };
+  if (vec == 4) lanes(std::integral_constant<int, 4>{});
+  else if (vec == 2) lanes(std::integral_constant<int, 2>{});
+  else lanes(std::integral_constant<int, 1>{});
   return after_launch(h, "sddmm");
 }
 
