@@ -1,0 +1,76 @@
+"""The kernels of a Lanczos step that add their partial sums up themselves and keep the block in
+registers between the passes of a CholQR: row counts at the edges of their tiles, of a group of CTAs,
+and of the switch to a second kernel; repeated calls (the ticket counters start at zero again);
+blocks aligned to one element only; breakdowns.
+
+Tolerances: sums of n products in 64 bits in any order, n eps sum|terms| (as in test_kernels_gpu.py,
+1e-12 of the magnitude for n <= 300,000); CholQR2 leaves |Q^T Q - I| and |Q R - X| at a modest multiple
+of the storage's eps (2.2e-16, 6e-8), held to 1e-13 and 1e-6 of the magnitude.
+"""
+import numpy as np
+import pytest
+import torch
+
+from trl_b200 import native
+
+from test_kernels_gpu import BS, DT, as_dt, close, dev, host
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("n", [1, 255, 257, 512 * 32, 512 * 32 + 1, 131072, 131073])
+def test_single_dot_rows(cuda_handle, bs, dtype, n):
+    rng = np.random.default_rng(n + bs)
+    X, Y = (as_dt(rng.standard_normal((n, bs)), dtype) for _ in range(2))
+    Xd, Yd = dev(X, dtype), dev(Y, dtype)
+    ref, scale = X.T @ Y, (np.abs(X).T @ np.abs(Y)).max()
+    first = None
+    for _ in range(3):
+        C = torch.full((1, bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+        cuda_handle.block_dot(Xd[None], Yd, C)
+        close(host(C)[0], ref, scale)
+        first = C if first is None else first
+        assert torch.equal(C, first)  # one order of additions, whichever CTA adds
+
+
+@pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("passes", [1, 2, 3, 4])
+@pytest.mark.parametrize("n,offset", [(16, 0), (33, 0), (4099, 1), (70001, 0)])
+def test_cholqr_passes(cuda_handle, bs, dtype, passes, n, offset):
+    rng = np.random.default_rng(n + bs)
+    X = as_dt(rng.standard_normal((n, bs)) @ (np.eye(bs) + 0.1 * rng.standard_normal((bs, bs))), dtype)
+    Xd = torch.zeros(n * bs + offset, dtype=dtype, device="cuda")[offset:].view(n, bs)
+    Xd.copy_(dev(X, dtype))
+    G0 = dev(X.T @ X)
+    R = torch.full((bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+    cuda_handle.cholqr_gram(Xd, passes, R, G0)
+    cuda_handle.sync()
+    Q, Rh = host(Xd), host(R)
+    eps = 1e-13 if dtype == torch.float64 else 1e-6
+    assert np.array_equal(np.tril(Rh, -1), np.zeros((bs, bs)))
+    assert np.abs(Q.T @ Q - np.eye(bs)).max() < (eps if passes > 1 else 100 * eps)
+    assert np.abs(Q @ Rh - X).max() < eps * np.abs(X).max()
+
+
+@pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("passes", [1, 2])
+def test_cholqr_breakdown_leaves_block_and_factor(cuda_handle, bs, passes):
+    X = torch.randn((1000, bs), dtype=torch.float64, device="cuda")
+    R = torch.full((bs, bs), 7.0, dtype=torch.float64, device="cuda")
+    G0 = -torch.eye(bs, dtype=torch.float64, device="cuda")
+    Y = X.clone()
+    cuda_handle.cholqr_gram(Y, 1, R, G0)
+    with pytest.raises(native.TrlError) as e:
+        cuda_handle.sync()
+    assert e.value.status == native.TRL_ECHOLESKY
+    assert torch.equal(X, Y) and torch.all(R == 7.0)
+    if passes == 2:  # the second pass works from the block itself
+        R.copy_(torch.eye(bs))
+        cuda_handle.cholqr_gram(Y, 2, R, G0)
+        with pytest.raises(native.TrlError):
+            cuda_handle.sync()
+        close(host(Y).T @ host(Y), np.eye(bs), 1.0, 1e-12)
+        close(host(Y) @ host(R), host(X), host(X.abs()).max(), 1e-12)

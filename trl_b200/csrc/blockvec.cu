@@ -79,16 +79,170 @@ __global__ void __launch_bounds__(kThreads) k_convert(D* __restrict__ dst, const
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) dst[i] = static_cast<D>(src[i]);
 }
 
+// ---------------------------------------------------------------- sums over the CTAs of a kernel
+// A kernel that leaves one row of LEN partial sums per CTA can also add them up: the CTA that
+// finishes last does it, found by ticket counters (zero between launches), so the short
+// results of single-block dots and Grams need no second launch. The rows are added in groups of
+// kTicketGroup, each by the last CTA of its group, and the groups' sums by the last group's: two
+// rounds of loads, however many CTAs there are. Which CTA adds depends on scheduling, the order
+// of the additions does not.
+constexpr int kTicketGroup = 32;
+constexpr int kTickets = 128; // counters of a handle: one for the groups, one per group
+
+struct Tickets {
+  unsigned* count; // [kTickets]
+  double* groups;  // [number of groups][LEN]
+};
+
+// sum[e] = sum of a[r * LEN + e] over the rows r < rows, by a CTA of kThreads; scratch: kThreads doubles
+template <int LEN>
+__device__ __forceinline__ void sum_rows(const double* a, int rows, double* sum, double* scratch)
+{
+  constexpr int SL = LEN >= kThreads ? 1 : (kThreads / LEN < 16 ? kThreads / LEN : 16); // threads per entry
+  constexpr int U = 8;                                    // loads in flight
+  const int tid = threadIdx.x;
+  for (int e = SL > 1 ? (tid < LEN * SL ? tid % LEN : LEN) : tid; e < LEN; e += kThreads) {
+    double t[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) t[u] = 0.0;
+    for (int r = tid / LEN; r < rows; r += U * SL) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) t[u] += r + u * SL < rows ? __ldcg(a + static_cast<int64_t>(r + u * SL) * LEN + e) : 0.0; // L2: other CTAs wrote it
+    }
+    const double v = ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+    if constexpr (SL == 1) sum[e] = v;
+    else scratch[tid] = v;
+  }
+  if constexpr (SL > 1) {
+    __syncthreads();
+    if (tid < LEN) {
+      double v = 0.0;
+#pragma unroll
+      for (int q = 0; q < SL; ++q) v += scratch[q * LEN + tid];
+      sum[tid] = v;
+    }
+  }
+  __syncthreads();
+}
+
+// Called by every CTA after it wrote its row `chunk` of partial[chunks][LEN]; true in the one CTA
+// that then has the totals in sum[LEN] (shared memory, as scratch).
+template <int LEN>
+__device__ __forceinline__ bool last_cta_sum(const double* partial, int chunks, int chunk, const Tickets& t, double* sum, double* scratch)
+{
+  __shared__ int last;
+  const int group = chunk / kTicketGroup, ngroups = (chunks + kTicketGroup - 1) / kTicketGroup;
+  const int members = min(kTicketGroup, chunks - group * kTicketGroup);
+  // the barrier and thread 0's fence order this CTA's row before its ticket, and the rows of
+  // the CTAs that came before it after the ticket
+  const auto take = [](unsigned* counter, int count) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(counter, 1u) == static_cast<unsigned>(count - 1);
+      __threadfence();
+    }
+    __syncthreads();
+    return last != 0;
+  };
+  if (!take(&t.count[1 + group], members)) return false;
+  sum_rows<LEN>(partial + static_cast<int64_t>(group) * kTicketGroup * LEN, members, sum, scratch);
+  if (threadIdx.x == 0) t.count[1 + group] = 0u;
+  if (ngroups == 1) return true;
+  for (int e = threadIdx.x; e < LEN; e += kThreads) t.groups[static_cast<int64_t>(group) * LEN + e] = sum[e];
+  if (!take(&t.count[0], ngroups)) return false;
+  sum_rows<LEN>(t.groups, ngroups, sum, scratch);
+  if (threadIdx.x == 0) t.count[0] = 0u;
+  return true;
+}
+
+// What the last CTA does with the totals (all its threads call it).
+struct FinishNone { // partial sums only
+  static constexpr bool kOn = false;
+  __device__ void operator()(const double*) const {}
+};
+
+template <int LEN>
+struct FinishStore {
+  static constexpr bool kOn = true;
+  double* out;
+  __device__ void operator()(const double* sum) const
+  {
+    for (int e = threadIdx.x; e < LEN; e += kThreads) out[e] = sum[e];
+  }
+};
+
+// Gram matrix of an updated block, and (flag) the DGKS criterion (Daniel, Gragg, Kaufman &
+// Stewart 1976): a second Gram-Schmidt pass is needed when some column kept less than eta of
+// its norm through the first pass.
+template <int BS>
+struct FinishGram {
+  static constexpr bool kOn = true;
+  double* G;
+  const double* before; // Gram matrix before the pass
+  double eta2;
+  int* flag; // null: no test
+  __device__ void operator()(const double* sum) const
+  {
+    for (int e = threadIdx.x; e < BS * BS; e += kThreads) G[e] = sum[e];
+    if (flag && threadIdx.x < 32) {
+      const int c = threadIdx.x;
+      const bool lost = c < BS && sum[c * BS + c] < eta2 * before[c * BS + c];
+      const unsigned any = __ballot_sync(0xffffffffu, lost);
+      if (c == 0) *flag = any != 0;
+    }
+  }
+};
+
+// sum = [E; G] = [S, W]^T W. flag = ||E||_F^2 > thr2 * trace(G): the sketch S^T W says W's components
+// along the basis exceed thr relative to W's norm. With `pair` (a word kept across calls), a step
+// whose test fired also projects the next one: pair = this step's test. G goes to both outputs
+// (G: the answer unless a pass runs; before: what the DGKS test compares with), and flag2 (the
+// second pass) is cleared, since the first pass may not run.
+template <int BS>
+struct FinishSketch {
+  static constexpr bool kOn = true;
+  double *G, *before;
+  double thr2;
+  int *flag, *flag2, *pair;
+  __device__ void operator()(const double* sum) const
+  {
+    constexpr int BB = BS * BS;
+    for (int e = threadIdx.x; e < BB; e += kThreads) G[e] = before[e] = sum[BB + e];
+    if (threadIdx.x < 32) {
+      const int lane = threadIdx.x;
+      double e2 = 0.0, tr = 0.0;
+      for (int e = lane; e < BB; e += 32) e2 = fma(sum[e], sum[e], e2);
+      for (int c = lane; c < BS; c += 32) tr += sum[BB + c * BS + c];
+      for (int o = 16; o > 0; o >>= 1) {
+        e2 += __shfl_xor_sync(0xffffffffu, e2, o);
+        tr += __shfl_xor_sync(0xffffffffu, tr, o);
+      }
+      if (lane == 0) {
+        const int fired = !(e2 <= thr2 * tr); // NaN counts as loss
+        int f = fired;
+        if (pair) {
+          f |= (*pair != 0) ? 2 : 0; // bit 1: forced by the previous step
+          *pair = fired;
+        }
+        *flag = f;
+        *flag2 = 0;
+      }
+    }
+  }
+};
+
 // ---------------------------------------------------------------- block dot
 // C_j = V_j^T W, j < nblk. Grid: x = chunk of JC blocks, y = chunk of rows.
 // A warp takes G groups of 4 rows per iteration. All operand loads of the iteration are
 // issued before the first DMMA (block indices beyond nblk are clamped to a valid block and
 // their products discarded), so each warp keeps G*(JC+1)*NT 256-byte loads in flight.
 // Per group: one DMMA m8n8k4 per (j, 8x8 output tile). Per-CTA sums go to
-// partial[row_chunk][j][BS*BS]; k_reduce_partials adds the row chunks in a fixed order.
-template <typename T, int BS, int JC, int G>
+// partial[row_chunk][j][BS*BS]; k_reduce_partials adds the row chunks in a fixed order, or (Fin,
+// nblk = JC, one chunk of blocks) the last CTA does.
+template <typename T, int BS, int JC, int G, class Fin>
 __global__ void __launch_bounds__(kThreads) k_block_dot(const T* __restrict__ V, int64_t vstride, int nblk, const T* __restrict__ W, int64_t n, int64_t rows_per_cta,
-                                                        double* __restrict__ partial, const int* __restrict__ cond = nullptr)
+                                                        double* __restrict__ partial, const int* __restrict__ cond, Tickets tickets, Fin fin)
 {
   ::trl_detail::pdl_enter();
   if (cond && *cond == 0) return; // device-side skip (uniform over the grid)
@@ -170,6 +324,12 @@ __global__ void __launch_bounds__(kThreads) k_block_dot(const T* __restrict__ V,
       }
     }
     __syncthreads();
+  }
+  if constexpr (Fin::kOn) {
+    constexpr int LEN = JC * BB;
+    static_assert(LEN + kThreads <= kWarps * NT * NT * 64, "totals and scratch fit the reduction buffer");
+    double* sum = &red[0][0];
+    if (last_cta_sum<LEN>(partial, static_cast<int>(gridDim.y), static_cast<int>(blockIdx.y), tickets, sum, sum + LEN)) fin(sum);
   }
 }
 
@@ -595,14 +755,18 @@ __device__ __forceinline__ void load_cols(const T* p, T (&v)[KS])
 // and in the same pass the Gram matrix out^T out of the values as stored (rounded to T):
 // each warp stages its finished rows in shared memory, re-reads them in DMMA fragment
 // layout (k = rows) and accumulates the BS x BS Gram; per-CTA sums go to
-// gram_partial[blockIdx.x][BS*BS]. When cond is given and *cond == 0 the kernel does
-// nothing (a device-side decision: no host round trip). `in` and `out` may alias for MB = 1.
-template <typename T, int BS, int RT, int U>
-__global__ void __launch_bounds__(kThreads) k_update_gram(const T* in, int64_t istride, int MB, const double* __restrict__ coef, T* out, int64_t n, int accumulate, double sign,
-                                                          double* __restrict__ gram_partial, const int* __restrict__ cond)
+// gram_partial[blockIdx.x][BS*BS], added up by the last CTA. When cond is given and *cond == 0
+// the kernel does nothing (a device-side decision: no host round trip).
+template <typename T, int BS, int RT, int U, class Fin>
+__global__ void __launch_bounds__(kThreads) k_update_gram(const T* in, int64_t istride, int MB, const double* __restrict__ coef, T* out, int64_t n,
+                                                          int accumulate, double sign, double* __restrict__ gram_partial, const int* __restrict__ cond, Tickets tickets, Fin fin)
 {
   ::trl_detail::pdl_enter();
   if (cond && *cond == 0) return;
+  // input blocks per loop body, without which ptxas picks worse ones from kernel to kernel.
+  // Measured on B200 (one projection, 884,736 rows, 2 / 3 blocks): FP64 bs 1 250 / 214 us, 2 175 / 183,
+  // 4 285 / 319, 8 462 / 511; FP32 bs 1 195 / 182, 2 415 / 393, 4 265 / 220, 8 286 / 295.
+  constexpr int kUnroll = (sizeof(T) == 4 ? BS <= 4 : BS == 1) ? 3 : 2;
   constexpr int NT = (BS + 7) / 8;
   constexpr int KS = (BS + 3) / 4;
   __shared__ double stage[kWarps][RT * 8 * BS];
@@ -630,6 +794,7 @@ __global__ void __launch_bounds__(kThreads) k_update_gram(const T* in, int64_t i
           acc[r][t][i] = (accumulate && row < n && col < BS) ? static_cast<double>(out[row * BS + col]) : 0.0;
         }
     }
+#pragma unroll(kUnroll)
     for (int ib0 = 0; ib0 < MB; ib0 += U) {
       // k is permuted so that lane t4 owns the KS adjacent columns t4*KS .. t4*KS+KS-1 of
       // its row (one vector load); the values stay in the storage type until the DMMA
@@ -714,177 +879,292 @@ __global__ void __launch_bounds__(kThreads) k_update_gram(const T* in, int64_t i
       gram_partial[static_cast<int64_t>(blockIdx.x) * BS * BS + row * BS + col] = s;
     }
   }
-}
-
-// DGKS criterion (Daniel, Gragg, Kaufman & Stewart 1976): a second Gram-Schmidt pass is
-// needed when some column kept less than eta of its norm through the first pass.
-template <int BS>
-__global__ void k_dgks_flag(const double* __restrict__ G_before, const double* __restrict__ G_after, double eta2, int* __restrict__ flag)
-{
-  ::trl_detail::pdl_enter();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int f = 0;
-  for (int c = 0; c < BS; ++c) f |= (G_after[c * BS + c] < eta2 * G_before[c * BS + c]);
-  *flag = f;
-}
-
-// flag = ||E||_F^2 > thr2 * trace(G): the sketch S^T W (E) says W's components along the
-// basis exceed thr relative to W's norm (G = W^T W). With `pair` (a word kept across calls),
-// a step whose test fired also projects the next one: pair = this step's test.
-template <int BS>
-__global__ void k_sketch_flag(const double* __restrict__ E, const double* __restrict__ G, double thr2, int* __restrict__ flag, int* __restrict__ pair)
-{
-  ::trl_detail::pdl_enter();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double e2 = 0.0, tr = 0.0;
-  for (int i = 0; i < BS * BS; ++i) e2 = fma(E[i], E[i], e2);
-  for (int c = 0; c < BS; ++c) tr += G[c * BS + c];
-  const int fired = !(e2 <= thr2 * tr); // NaN counts as loss
-  int f = fired;
-  if (pair) {
-    f |= (*pair != 0) ? 2 : 0; // bit 1: forced by the previous step
-    *pair = fired;
-  }
-  *flag = f;
-}
-
-// flag2 = flag1 && (a column kept less than eta of its norm through pass 1)
-template <int BS>
-__global__ void k_dgks_flag_after(const int* __restrict__ flag1, const double* __restrict__ G_before, const double* __restrict__ G_after, double eta2, int* __restrict__ flag2)
-{
-  ::trl_detail::pdl_enter();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int f = 0;
-  if (*flag1)
-    for (int c = 0; c < BS; ++c) f |= (G_after[c * BS + c] < eta2 * G_before[c * BS + c]);
-  *flag2 = f;
-}
-
-// dst = *f2 ? c : (*f1 ? b : a)  (BS x BS)
-__global__ void k_select_block3(const int* __restrict__ f1, const int* __restrict__ f2, const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-                                double* __restrict__ dst, int count)
-{
-  ::trl_detail::pdl_enter();
-  const int e = threadIdx.x;
-  if (e < count) dst[e] = *f2 ? c[e] : (*f1 ? b[e] : a[e]);
-}
-
-// dst = *flag ? a : b  (BS x BS)
-__global__ void k_select_block(const int* __restrict__ flag, const double* __restrict__ a, const double* __restrict__ b, double* __restrict__ dst, int count)
-{
-  ::trl_detail::pdl_enter();
-  const int e = threadIdx.x;
-  if (e < count) dst[e] = *flag ? a[e] : b[e];
-}
-
-// ---------------------------------------------------------------- small Cholesky
-// Gram matrix G from `chunks` partial sums (chunks = 0: G given), then G = L L^T reading
-// the lower triangle, Uinv = L^{-T} for the apply, and R <- L^T (first pass) or
-// R <- L^T R (so that X_in = X_out R across passes). All in shared memory; the factor and
-// the inverse are column-parallel over one warp. A pivot <= 0 (or NaN) records
-// TRL_DEV_CHOLESKY and writes Uinv = I, leaving the apply a no-op.
-// With partial sums the reduction is spread over ceil(BS^2 / kFactorOPC) CTAs, each
-// summing kFactorOPC entries of G in a fixed order into gsum; the CTA that finishes last
-// (a ticket counter, left at zero again) factors. Every entry is summed by one CTA in one
-// order, so the result does not depend on scheduling.
-constexpr int kFactorOPC = 8;
-template <int BS>
-__global__ void __launch_bounds__(kRedThreads) k_gram_factor(const double* __restrict__ src, int chunks, double* __restrict__ Uinv, double* __restrict__ R, int first,
-                                                             int* status, double* gsum, unsigned* ticket)
-{
-  ::trl_detail::pdl_enter();
-  constexpr int OPC = kFactorOPC;
-  constexpr int SL = kRedThreads / OPC; // slices of the chunk range per entry
-  __shared__ double G[BS * BS], L[BS][BS + 1], Li[BS][BS + 1], Ro[BS * BS];
-  __shared__ double part[SL][OPC + 1];
-  __shared__ int bad, last;
-  const int tid = threadIdx.x;
-  // 1. G (the same fixed-order reduction as k_reduce_partials<8>)
-  if (chunks > 0) {
-    const int o = tid % OPC, s = tid / OPC, e = static_cast<int>(blockIdx.x) * OPC + o;
-    part[s][o] = e < BS * BS ? slice_sum<SL>(src, chunks, BS * BS, e, s) : 0.0;
-    __syncthreads();
-    if (s == 0 && e < BS * BS) {
-      double t = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < SL; ++q) t += part[q][o];
-      gsum[e] = t;
-    }
-    if (gridDim.x > 1) {
-      __threadfence(); // this CTA's entries of gsum are visible before its ticket is taken
-      __syncthreads();
-      if (tid == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-      __syncthreads();
-      if (!last) return;
-      __threadfence();
-      if (tid == 0) *ticket = 0u;
-    }
-    else
-      __syncthreads();
-    for (int e = tid; e < BS * BS; e += blockDim.x) G[e] = __ldcg(gsum + e); // L2: written by other CTAs
-  }
-  else {
-    for (int e = tid; e < BS * BS; e += blockDim.x) G[e] = src[e];
-  }
-  for (int e = tid; e < BS * BS; e += blockDim.x) Ro[e] = R[e];
-  if (tid == 0) bad = 0;
   __syncthreads();
-  if (tid < 32) {
-    const int lane = tid;
-    // 2. L: column by column; lane i < BS owns row i
-    for (int j = 0; j < BS; ++j) {
-      if (lane == j) {
-        double d = G[j * BS + j];
-        for (int k = 0; k < j; ++k) d -= L[j][k] * L[j][k];
-        if (!(d > 0.0)) bad = 1;
-        L[j][j] = d > 0.0 ? sqrt(d) : 1.0;
-      }
-      __syncwarp();
-      if (lane > j && lane < BS) {
-        double s = G[lane * BS + j];
-        for (int k = 0; k < j; ++k) s -= L[lane][k] * L[j][k];
-        L[lane][j] = s / L[j][j];
-      }
-      if (lane < j) L[lane][j] = 0.0;
-      __syncwarp();
+  static_assert(BS * BS + kThreads <= kWarps * NT * NT * 64, "totals and scratch fit the reduction buffer");
+  double* sum = &red[0][0];
+  if (last_cta_sum<BS * BS>(gram_partial, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), tickets, sum, sum + BS * BS)) fin(sum);
+}
+
+// ---------------------------------------------------------------- Cholesky-QR
+// One warp: G = L L^T (reading the lower triangle), Ui = L^{-T}; L is left in shared memory. Lane i
+// owns row i of G, then column i of L^{-1}; chains of one square root or division per column.
+// false (uniform): a pivot was <= 0 or NaN; Ui is then the identity, which leaves an apply a no-op.
+template <int BS>
+__device__ __forceinline__ bool warp_factor(const double* G, double (*L)[BS + 1], double* Ui)
+{
+  const int lane = threadIdx.x & 31;
+  double row[BS];
+  bool ok = true;
+#pragma unroll
+  for (int j = 0; j < BS; ++j) row[j] = lane < BS ? G[lane * BS + j] : 0.0;
+#pragma unroll
+  for (int j = 0; j < BS; ++j) {
+    const double piv = __shfl_sync(0xffffffffu, row[j], j);
+    ok = ok && piv > 0.0;
+    const double l = piv > 0.0 ? sqrt(piv) : 1.0;
+    row[j] = lane == j ? l : (lane > j ? row[j] / l : 0.0);
+#pragma unroll
+    for (int k = j + 1; k < BS; ++k) {
+      const double lk = __shfl_sync(0xffffffffu, row[j], k);
+      row[k] = fma(-row[j], lk, row[k]);
     }
-    // 3. Li = L^{-1} (lower): lane c owns column c, forward substitution
-    if (lane < BS) {
-      const int c = lane;
-      for (int i = 0; i < BS; ++i) {
-        if (i < c) {
-          Li[i][c] = 0.0;
-          continue;
-        }
-        double s = (i == c) ? 1.0 : 0.0;
-        for (int k = c; k < i; ++k) s -= L[i][k] * Li[k][c];
-        Li[i][c] = s / L[i][i];
-      }
+  }
+  if (lane < BS) {
+#pragma unroll
+    for (int j = 0; j < BS; ++j) L[lane][j] = row[j];
+  }
+  __syncwarp();
+  if (lane < BS) {
+    double x[BS]; // column `lane` of the identity, then of L^{-1}
+#pragma unroll
+    for (int i = 0; i < BS; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < BS; ++i) {
+      x[i] = x[i] / L[i][i];
+#pragma unroll
+      for (int m = i + 1; m < BS; ++m) x[m] = fma(-L[m][i], x[i], x[m]);
     }
-    __syncwarp();
-    // 4. outputs: Uinv = Li^T; R (lane i owns row i)
-    if (lane < BS) {
-      const int i = lane;
-      for (int c = 0; c < BS; ++c) Uinv[i * BS + c] = bad ? (i == c ? 1.0 : 0.0) : Li[c][i];
-      if (!bad) {
-        for (int c = 0; c < BS; ++c) {
-          double s;
-          if (first) {
-            s = (c >= i) ? L[c][i] : 0.0;
-          }
-          else {
-            s = 0.0;
-            for (int k = i; k <= c; ++k) s += L[k][i] * Ro[k * BS + c];
-            if (c < i) s = 0.0;
-          }
-          R[i * BS + c] = s;
-        }
+#pragma unroll
+    for (int c = 0; c < BS; ++c) Ui[lane * BS + c] = ok ? x[c] : (c == lane ? 1.0 : 0.0);
+  }
+  __syncwarp();
+  return ok;
+}
+
+// The factor's outputs, by the same warp: Ui to global memory, and R <- L^T (first pass) or
+// R <- L^T R (X_in = X_out R across passes). A breakdown leaves R and records TRL_DEV_CHOLESKY.
+template <int BS>
+__device__ __forceinline__ void warp_factor_store(bool ok, const double (*L)[BS + 1], const double* Ui, double* Uout, double* R, bool first, int* status)
+{
+  const int lane = threadIdx.x & 31;
+  for (int e = lane; e < BS * BS; e += 32) Uout[e] = Ui[e];
+  if (!ok) {
+    if (lane == 0) atomicOr(status, TRL_DEV_CHOLESKY);
+    return;
+  }
+  double r[BS]; // column `lane` of R before
+  if (lane < BS && !first) {
+#pragma unroll
+    for (int k = 0; k < BS; ++k) r[k] = __ldcg(R + k * BS + lane); // L2: another CTA may have written it
+  }
+  __syncwarp();
+  if (lane < BS) {
+#pragma unroll
+    for (int i = 0; i < BS; ++i) { // entry (i, lane)
+      double v = 0.0;
+      if (first) v = L[lane][i]; // zero above the diagonal of L: R is upper triangular
+      else {
+#pragma unroll
+        for (int k = i; k < BS; ++k)
+          if (k <= lane) v = fma(L[k][i], r[k], v);
       }
+      R[i * BS + lane] = i <= lane ? v : 0.0;
     }
-    if (lane == 0 && bad) atomicOr(status, TRL_DEV_CHOLESKY);
   }
 }
 
+// X's rows as a warp holds them: lane (g, t4) columns 8 t + 2 t4 and the next one of row g of an
+// 8-row tile, which is at once the accumulator layout of a DMMA and, with the k dimension
+// permuted, its A operand: the product with a factor feeds the next one without a move.
+template <typename T, int BS>
+struct CholTile {
+  static constexpr int NT = (BS + 7) / 8;
+  // pairs: X is aligned to two elements, so that a lane's two columns are one load
+  static __device__ __forceinline__ void load(const T* X, int64_t row, int64_t n, int t4, bool pairs, double (&x)[NT][2])
+  {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      const int col = t * 8 + 2 * t4;
+      x[t][0] = x[t][1] = 0.0;
+      if (row < n && col < BS) {
+        if constexpr (BS >= 2) {
+          T v[2];
+          if (pairs) load_cols<T, 2>(X + row * BS + col, v);
+          else {
+            v[0] = X[row * BS + col];
+            v[1] = X[row * BS + col + 1];
+          }
+          x[t][0] = static_cast<double>(v[0]);
+          x[t][1] = static_cast<double>(v[1]);
+        }
+        else
+          x[t][0] = static_cast<double>(X[row]);
+      }
+    }
+  }
+  // this lane's fragments of a factor U (shared memory, row-major)
+  static __device__ __forceinline__ void fragments(const double* U, int g, int t4, double (&b)[NT][2][NT])
+  {
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < NT; ++c) {
+          const int k = t * 8 + 2 * t4 + i, col = c * 8 + g;
+          b[t][i][c] = (k < BS && col < BS) ? U[k * BS + col] : 0.0;
+        }
+  }
+  // x <- x U, rounded to T as a stored block would be
+  static __device__ __forceinline__ void apply(double (&x)[NT][2], const double (&b)[NT][2][NT])
+  {
+    double acc[NT][2];
+#pragma unroll
+    for (int c = 0; c < NT; ++c) acc[c][0] = acc[c][1] = 0.0;
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < NT; ++c) dmma_m8n8k4(acc[c][0], acc[c][1], x[t][i], b[t][i][c]);
+#pragma unroll
+    for (int c = 0; c < NT; ++c) {
+      x[c][0] = static_cast<double>(static_cast<T>(acc[c][0]));
+      x[c][1] = static_cast<double>(static_cast<T>(acc[c][1]));
+    }
+  }
+};
+
+constexpr int kCholMaxPasses = 4;
+
+// CholQR without storing the block between passes: the factors so far, U_0 ... U_{nf-1}, are applied to
+// each row tile in registers (rounded to T after each, so the values are those of a stored
+// block). With G0, nf is 1 and every CTA factors G0 for itself first (a few microseconds in
+// place of a launch); CTA 0 keeps the outputs.
+// GRAM: forms the Gram matrix of the result, and the last CTA factors it into U_nf. Otherwise the
+// result is stored in place, and CholQR2 has read the block twice and written it once.
+// Measured on B200, CholQR2 of 884,736 x 8 FP64 / 100,003 x 16 FP32: 40 / 45 us (before, with a
+// launch per factor and the block stored between the passes: 57 / 61 us).
+template <typename T, int BS, int RT, bool GRAM>
+__global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const double* __restrict__ G0, int nf, double* U, double* R, int* status, double* __restrict__ partial,
+                                                     Tickets tickets)
+{
+  ::trl_detail::pdl_enter();
+  using Tile = CholTile<T, BS>;
+  constexpr int NT = Tile::NT;
+  constexpr int BB = BS * BS;
+  __shared__ double Us[kCholMaxPasses][BB];
+  __shared__ double Ls[BS][BS + 1];
+  __shared__ double stage[GRAM ? kWarps : 1][GRAM ? RT * 8 * BS : 1];
+  __shared__ double red[GRAM ? kWarps : 1][GRAM ? NT * NT * 64 : BB];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t4 = lane & 3;
+  if (G0) {
+    double* Gs = &red[0][0];
+    for (int e = threadIdx.x; e < BB; e += kThreads) Gs[e] = G0[e];
+    __syncthreads();
+    if (warp == 0) {
+      const bool ok = warp_factor<BS>(Gs, Ls, Us[0]);
+      if (blockIdx.x == 0) warp_factor_store<BS>(ok, Ls, Us[0], U, R, true, status);
+    }
+  }
+  else
+    for (int e = threadIdx.x; e < nf * BB; e += kThreads) Us[e / BB][e % BB] = U[e];
+  __syncthreads();
+  const bool pairs = reinterpret_cast<uintptr_t>(X) % (2 * sizeof(T)) == 0;
+  double b0[NT][2][NT], b1[NT][2][NT]; // the first two factors in registers
+  Tile::fragments(Us[0], g, t4, b0);
+  if (nf > 1) Tile::fragments(Us[1], g, t4, b1);
+
+  double gacc[NT][NT][2];
+#pragma unroll
+  for (int a = 0; a < NT; ++a)
+#pragma unroll
+    for (int b = 0; b < NT; ++b) gacc[a][b][0] = gacc[a][b][1] = 0.0;
+  const int64_t warp_stride = static_cast<int64_t>(gridDim.x) * kWarps * 8 * RT;
+  for (int64_t r0 = (static_cast<int64_t>(blockIdx.x) * kWarps + warp) * 8 * RT; r0 < n; r0 += warp_stride) {
+    double x[RT][NT][2];
+#pragma unroll
+    for (int r = 0; r < RT; ++r) Tile::load(X, r0 + r * 8 + g, n, t4, pairs, x[r]);
+#pragma unroll
+    for (int r = 0; r < RT; ++r) Tile::apply(x[r], b0);
+    if (nf > 1) {
+#pragma unroll
+      for (int r = 0; r < RT; ++r) Tile::apply(x[r], b1);
+    }
+    for (int f = 2; f < nf; ++f) {
+      double bf[NT][2][NT];
+      Tile::fragments(Us[f], g, t4, bf);
+#pragma unroll
+      for (int r = 0; r < RT; ++r) Tile::apply(x[r], bf);
+    }
+    if constexpr (!GRAM) {
+#pragma unroll
+      for (int r = 0; r < RT; ++r) {
+        const int64_t row = r0 + r * 8 + g;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int col = t * 8 + 2 * t4;
+          if (row < n && col < BS) {
+            if constexpr (BS >= 2) {
+              const T v[2] = {static_cast<T>(x[r][t][0]), static_cast<T>(x[r][t][1])};
+              if (pairs) ::trl_detail::store_vec<T, 2>(X + row * BS + col, v);
+              else {
+                X[row * BS + col] = v[0];
+                X[row * BS + col + 1] = v[1];
+              }
+            }
+            else
+              X[row] = static_cast<T>(x[r][t][0]);
+          }
+        }
+      }
+    }
+    else {
+      // rows past n are zero: they add nothing to the Gram
+#pragma unroll
+      for (int r = 0; r < RT; ++r)
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int col = t * 8 + 2 * t4 + i;
+            if (col < BS) stage[warp][(r * 8 + g) * BS + col] = x[r][t][i];
+          }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 2 * RT; ++q) { // groups of 4 staged rows = the DMMA k dimension
+        const int lr = q * 4 + t4;
+        double bf[NT];
+#pragma unroll
+        for (int tk = 0; tk < NT; ++tk) bf[tk] = (tk * 8 + g < BS) ? stage[warp][lr * BS + tk * 8 + g] : 0.0;
+#pragma unroll
+        for (int ti = 0; ti < NT; ++ti)
+#pragma unroll
+          for (int tk = 0; tk < NT; ++tk) dmma_m8n8k4(gacc[ti][tk][0], gacc[ti][tk][1], bf[ti], bf[tk]);
+      }
+      __syncwarp();
+    }
+  }
+  if constexpr (GRAM) {
+    __syncthreads(); // red held G0
+#pragma unroll
+    for (int ti = 0; ti < NT; ++ti)
+#pragma unroll
+      for (int tk = 0; tk < NT; ++tk) {
+        red[warp][(ti * NT + tk) * 64 + g * 8 + 2 * t4 + 0] = gacc[ti][tk][0];
+        red[warp][(ti * NT + tk) * 64 + g * 8 + 2 * t4 + 1] = gacc[ti][tk][1];
+      }
+    __syncthreads();
+    for (int e = threadIdx.x; e < NT * NT * 64; e += kThreads) {
+      const int tile = e >> 6, within = e & 63;
+      const int row = (tile / NT) * 8 + (within >> 3);
+      const int col = (tile % NT) * 8 + (within & 7);
+      if (row < BS && col < BS) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) v += red[w][e];
+        partial[static_cast<int64_t>(blockIdx.x) * BB + row * BS + col] = v;
+      }
+    }
+    __syncthreads();
+    double* sum = &red[0][0];
+    if (last_cta_sum<BB>(partial, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), tickets, sum, sum + BB) && warp == 0) {
+      const bool ok = warp_factor<BS>(sum, Ls, Us[0]);
+      warp_factor_store<BS>(ok, Ls, Us[0], U + nf * BB, R, false, status);
+    }
+  }
+}
 
 } // namespace
 
@@ -893,53 +1173,60 @@ using namespace trl_detail;
 // ---------------------------------------------------------------- launchers
 namespace trl_detail {
 
+// Workspace of a kernel whose last CTA adds up `chunks` rows of `len` partial sums; null on failure.
+inline double* ticket_workspace(trl_cuda_context* h, int64_t chunks, int64_t len, Tickets& t)
+{
+  const int64_t groups = (chunks + kTicketGroup - 1) / kTicketGroup;
+  double* small = static_cast<double*>(small_scratch(h));
+  if (!small || groups + 1 > kTickets) return nullptr;
+  double* partial = static_cast<double*>(workspace(h, static_cast<size_t>(chunks + groups) * len * sizeof(double)));
+  t.count = reinterpret_cast<unsigned*>(small + kSmallTickets);
+  t.groups = partial ? partial + chunks * len : nullptr;
+  return partial;
+}
+
+// Row chunks of the register-fed dot: about 4 CTAs per SM in total, 512+ rows per CTA.
+template <int G>
+int64_t dot_chunks(int num_sms, int gj, int64_t n, int64_t& rows_per_cta)
+{
+  int64_t chunks = static_cast<int64_t>(num_sms) * 4 / gj;
+  const int64_t max_chunks = (n + 511) / 512;
+  if (chunks > max_chunks) chunks = max_chunks;
+  if (chunks < 1) chunks = 1;
+  rows_per_cta = (n + chunks - 1) / chunks;
+  constexpr int step = kWarps * 4 * G; // rows one CTA iteration covers
+  rows_per_cta = (rows_per_cta + step - 1) / step * step;
+  return (n + rows_per_cta - 1) / rows_per_cta;
+}
+
+// C = [V_0, V_vstride, ...]^T W for JC blocks `vstride` elements apart, reading W once; fin gets the
+// JC * BS * BS totals in the same launch.
+template <typename T, int BS, int JC, int G, class Fin>
+int launch_block_dot_finish(trl_cuda_context* h, const T* V, int64_t vstride, const T* W, int64_t n, const int* cond, const Fin& fin)
+{
+  int64_t rows_per_cta = 0;
+  const int64_t chunks = dot_chunks<G>(h->num_sms, 1, n, rows_per_cta);
+  Tickets t{};
+  double* partial = ticket_workspace(h, chunks, static_cast<int64_t>(JC) * BS * BS, t);
+  if (!partial) return TRL_ENOMEM;
+  launch(k_block_dot<T, BS, JC, G, Fin>, dim3(1, static_cast<unsigned>(chunks)), kThreads, 0, h->stream, V, vstride, JC, W, n, rows_per_cta, partial, cond, t, fin);
+  return after_launch(h, "block_dot");
+}
+
 template <typename T, int BS, int JC, int G>
 int launch_block_dot_jc(trl_cuda_context* h, const T* V, int nblk, const T* W, int64_t n, double* C, const int* cond)
 {
   const int64_t len = static_cast<int64_t>(nblk) * BS * BS;
   const int gj = (nblk + JC - 1) / JC;
-  // about 4 CTAs per SM in total, 512+ rows per CTA
-  int64_t target = static_cast<int64_t>(h->num_sms) * 4 / gj;
-  if (target < 1) target = 1;
-  int64_t max_chunks = (n + 511) / 512;
-  int64_t chunks = target < max_chunks ? target : max_chunks;
-  if (chunks < 1) chunks = 1;
-  int64_t rows_per_cta = (n + chunks - 1) / chunks;
-  constexpr int step = kWarps * 4 * G; // rows one CTA iteration covers
-  rows_per_cta = (rows_per_cta + step - 1) / step * step;
-  chunks = (n + rows_per_cta - 1) / rows_per_cta;
+  int64_t rows_per_cta = 0;
+  const int64_t chunks = dot_chunks<G>(h->num_sms, gj, n, rows_per_cta);
   double* partial = static_cast<double*>(workspace(h, static_cast<size_t>(chunks) * len * sizeof(double)));
   if (!partial) return TRL_ENOMEM;
-  dim3 grid(gj, static_cast<unsigned>(chunks));
-  launch(k_block_dot<T, BS, JC, G>, grid, kThreads, 0, h->stream, V, n * BS, nblk, W, n, rows_per_cta, partial, cond);
+  launch(k_block_dot<T, BS, JC, G, FinishNone>, dim3(gj, static_cast<unsigned>(chunks)), kThreads, 0, h->stream, V, n * BS, nblk, W, n, rows_per_cta, partial, cond, Tickets{},
+         FinishNone{});
   int st = after_launch(h, "block_dot");
   if (st) return st;
   launch_reduce(h->stream, partial, chunks, len, C, cond);
-  return after_launch(h, "block_dot reduce");
-}
-
-// C = [A, B]^T W (2 blocks of bs x bs) for two blocks anywhere in memory, reading W once:
-// the register kernel's blocks are V and V + vstride.
-template <typename T, int BS>
-int launch_block_dot_two(trl_cuda_context* h, const T* A, const T* B, const T* W, int64_t n, double* C)
-{
-  constexpr int JC = 2, G = 4;
-  constexpr int64_t len = 2 * BS * BS;
-  int64_t target = static_cast<int64_t>(h->num_sms) * 4;
-  int64_t max_chunks = (n + 511) / 512;
-  int64_t chunks = target < max_chunks ? target : max_chunks;
-  if (chunks < 1) chunks = 1;
-  int64_t rows_per_cta = (n + chunks - 1) / chunks;
-  constexpr int step = kWarps * 4 * G;
-  rows_per_cta = (rows_per_cta + step - 1) / step * step;
-  chunks = (n + rows_per_cta - 1) / rows_per_cta;
-  double* partial = static_cast<double*>(workspace(h, static_cast<size_t>(chunks) * len * sizeof(double)));
-  if (!partial) return TRL_ENOMEM;
-  const int64_t vstride = B - A; // elements between the two blocks
-  launch(k_block_dot<T, BS, JC, G>, dim3(1, static_cast<unsigned>(chunks)), kThreads, 0, h->stream, A, vstride, 2, W, n, rows_per_cta, partial, nullptr);
-  int st = after_launch(h, "block_dot");
-  if (st) return st;
-  launch_reduce(h->stream, partial, chunks, len, C, nullptr);
   return after_launch(h, "block_dot reduce");
 }
 
@@ -976,6 +1263,8 @@ int launch_block_dot_bulk(trl_cuda_context* h, const T* V, int nblk, const T* W,
   return after_launch(h, "block_dot reduce");
 }
 
+constexpr int64_t kTicketDotRows = 131072;
+
 // Bulk-copy pipeline when a row of the block is a whole number of 16-byte units; otherwise
 // the register-prefetch kernel with JC blocks and G row groups per warp iteration (about
 // 16-20 independent loads in flight per warp).
@@ -993,7 +1282,14 @@ int launch_block_dot(trl_cuda_context* h, const T* V, int nblk, const T* W, int6
   // A single block (the driver's T_ii = V_i^T W, both operands usually still in L2 from the
   // SpMM): the register-fed kernel with 8 (FP64) / 4 (FP32) row groups per warp and 4 CTAs
   // per SM measured 6,851 / 5,682 GB/s against 4,759 / 4,562 for the bulk pipeline.
-  if (nblk == 1 && BS <= 8) return launch_block_dot_jc<T, BS, 1, (sizeof(T) == 8 ? 8 : 4)>(h, V, nblk, W, n, C, cond);
+  // Up to kTicketDotRows rows its last CTA adds the partial sums up (B200, 16,384 x 8 FP64: 10.0 -> 7.3 us,
+  // the second launch's host time); beyond that the wider second kernel is faster (884,736 x 8: FP64
+  // 20.8 against 19.6 us, FP32 15.5 against 12.0).
+  if (nblk == 1 && BS <= 8) {
+    constexpr int G1 = sizeof(T) == 8 ? 8 : 4;
+    if (n <= kTicketDotRows) return launch_block_dot_finish<T, BS, 1, G1>(h, V, n * BS, W, n, cond, FinishStore<BS * BS>{C});
+    return launch_block_dot_jc<T, BS, 1, G1>(h, V, nblk, W, n, C, cond);
+  }
   if constexpr ((BS * sizeof(T)) % 16 == 0) {
     constexpr int TBS = (BS * sizeof(T) <= 64) ? 2048 : 4096; // small tiles where 32 rows fit
     constexpr int JCL = BS >= 16 ? 4 : 8;
@@ -1010,11 +1306,9 @@ int launch_block_dot(trl_cuda_context* h, const T* V, int nblk, const T* W, int6
   return launch_block_dot_jc<T, BS, (BS >= 16 ? 4 : 8), 2>(h, V, nblk, W, n, C, cond);
 }
 
-// Launches k_update_gram; the per-CTA Gram partial sums are left in the workspace
-// (*partial, *chunks) for the caller to reduce.
-template <typename T, int BS>
-int launch_update_gram_partials(trl_cuda_context* h, const T* in, int MB, const double* coef, T* out, int64_t n, int accumulate, double sign, const int* cond,
-                                double** partial, int* chunks)
+// out -= V C over MB blocks and the Gram matrix of the result, which fin gets
+template <typename T, int BS, class Fin>
+int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* coef, T* out, int64_t n, const int* cond, const Fin& fin)
 {
   constexpr int NT = (BS + 7) / 8;
   // Measured on B200 (24 blocks of 884,736 x 8, GB/s of algorithmic bytes; copy peak
@@ -1024,26 +1318,36 @@ int launch_update_gram_partials(trl_cuda_context* h, const T* in, int MB, const 
   constexpr int RT = NT >= 2 ? 1 : (sizeof(T) == 8 ? 4 : 2);
   static int resident = 0;
   if (resident == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_update_gram<T, BS, RT, 1>, kThreads, 0) != cudaSuccess || resident < 1) resident = 4;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_update_gram<T, BS, RT, 1, Fin>, kThreads, 0) != cudaSuccess || resident < 1) resident = 4;
     cudaGetLastError();
   }
   const unsigned grid = grid_for(h, (n + 8 * RT - 1) / (8 * RT), kWarps, 2 * resident);
-  *partial = static_cast<double*>(workspace(h, static_cast<size_t>(grid) * BS * BS * sizeof(double)));
-  *chunks = static_cast<int>(grid);
-  if (!*partial) return TRL_ENOMEM;
-  launch(k_update_gram<T, BS, RT, 1>, grid, kThreads, 0, h->stream, in, n * BS, MB, coef, out, n, accumulate, sign, *partial, cond);
+  Tickets t{};
+  double* partial = ticket_workspace(h, grid, BS * BS, t);
+  if (!partial) return TRL_ENOMEM;
+  launch(k_update_gram<T, BS, RT, 1, Fin>, grid, kThreads, 0, h->stream, in, n * BS, MB, coef, out, n, 1, -1.0, partial, cond, t, fin);
   return after_launch(h, "update_gram");
 }
 
-template <typename T, int BS>
-int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* coef, T* out, int64_t n, int accumulate, double sign, double* G, const int* cond)
+// One pass of k_cholqr over the block: GRAM factors the Gram matrix of X U_0 ... U_{nf-1}, otherwise
+// X <- X U_0 ... U_{nf-1}.
+template <typename T, int BS, bool GRAM>
+int launch_cholqr(trl_cuda_context* h, T* X, int64_t n, const double* G0, int nf, double* U, double* R)
 {
+  constexpr int NT = (BS + 7) / 8;
+  constexpr int RT = NT >= 2 ? 2 : 4;
+  static int resident = 0;
+  if (resident == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cholqr<T, BS, RT, GRAM>, kThreads, 0) != cudaSuccess || resident < 1) resident = 4;
+    cudaGetLastError();
+  }
+  // one resident wave: every CTA prepares its factors once
+  const unsigned grid = grid_for(h, (n + 8 * RT - 1) / (8 * RT), kWarps, resident);
+  Tickets t{};
   double* partial = nullptr;
-  int chunks = 0;
-  int st = launch_update_gram_partials<T, BS>(h, in, MB, coef, out, n, accumulate, sign, cond, &partial, &chunks);
-  if (st) return st;
-  launch_reduce(h->stream, partial, chunks, BS * BS, G, cond);
-  return after_launch(h, "update_gram reduce");
+  if (GRAM && !(partial = ticket_workspace(h, grid, BS * BS, t))) return TRL_ENOMEM;
+  launch(k_cholqr<T, BS, RT, GRAM>, grid, kThreads, 0, h->stream, X, n, G0, nf, U, R, h->d_status, partial, t);
+  return after_launch(h, "cholqr");
 }
 
 template <typename T, int BS, int NBMAX>
@@ -1298,40 +1602,26 @@ int trl_cuda_cholqr(trl_cuda_handle h, int dtype, void* X, int64_t n, int bs, in
   return trl_cuda_cholqr_gram(h, dtype, X, n, bs, passes, R, G);
 }
 
-// Per pass: one-CTA factor of the Gram matrix, then the apply X <- X U^{-1}, which also
-// forms the partial Gram sums of the result for the next pass's factor.
+// passes - 1 launches that each add a factor (the first one factors G0 too), and one that applies
+// them all.
 int trl_cuda_cholqr_gram(trl_cuda_handle h, int dtype, void* X, int64_t n, int bs, int passes, double* R, const double* G0)
 {
   TRL_CHECK_HANDLE(h);
   if (!G0) return trl_cuda_cholqr(h, dtype, X, n, bs, passes, R);
   if (int st = check_common(h, dtype, n, bs)) return st;
-  if (passes < 1 || passes > 4) return set_error(h, TRL_EINVAL, "passes must be in [1, 4]");
+  if (passes < 1 || passes > kCholMaxPasses) return set_error(h, TRL_EINVAL, "passes must be in [1, 4]");
   if (!X || !R) return set_error(h, TRL_EINVAL, "null pointer");
   double* small = static_cast<double*>(small_scratch(h));
   if (!small) return TRL_ENOMEM;
-  double* Uinv = small + 256;
-  double* gsum = small + 512;                                // the factor's reduced Gram entries
-  unsigned* ticket = reinterpret_cast<unsigned*>(small + 768); // zero between launches
+  double* U = small + kSmallFactors;
   ProfScope prof(h, PROF_CHOLQR, 2.0 * passes * n * bs * elt_size(dtype), 4.0 * passes * n * bs * bs);
-  const double* src = G0; // the Gram matrix, or per-CTA partial sums of it
-  int chunks = 0;
-  for (int p = 0; p < passes; ++p) {
-    int st = TRL_OK;
-    TRL_DISPATCH_BS(bs, launch(k_gram_factor<BS>, chunks > 0 ? static_cast<unsigned>((BS * BS + kFactorOPC - 1) / kFactorOPC) : 1u, kRedThreads, 0, h->stream, src, chunks,
-                               Uinv, R, p == 0, h->d_status, gsum, ticket));
-    st = after_launch(h, "cholqr factor");
-    if (st) return st;
-    if (p + 1 < passes) {
-      double* partial = nullptr;
-      TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, st = launch_update_gram_partials<T, BS>(h, static_cast<const T*>(X), 1, Uinv, static_cast<T*>(X), n, 0, 1.0, nullptr, &partial, &chunks)));
-      src = partial;
-    }
-    else {
-      TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, st = launch_block_gemm<T, BS>(h, static_cast<const T*>(X), 1, Uinv, 1, 0, static_cast<T*>(X), 1, n, 0, 1.0)));
-    }
-    if (st) return st;
-  }
-  return TRL_OK;
+  int st = TRL_OK;
+  TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
+    T* Xt = static_cast<T*>(X);
+    for (int q = 1; q < passes && !st; ++q) st = launch_cholqr<T, BS, true>(h, Xt, n, q == 1 ? G0 : nullptr, q, U, R);
+    if (!st) st = launch_cholqr<T, BS, false>(h, Xt, n, passes == 1 ? G0 : nullptr, passes, U, R);
+  }));
+  return st;
 }
 
 int trl_cuda_project_out(trl_cuda_handle h, int dtype, const void* V, int nblk, void* W, int64_t n, int bs, int mode, double eta, double* G)
@@ -1344,15 +1634,13 @@ int trl_cuda_project_out(trl_cuda_handle h, int dtype, const void* V, int nblk, 
   if (n == 0) return trl_cuda_memset_zero(h, G, sizeof(double) * BB);
   if (!V || !W) return set_error(h, TRL_EINVAL, "null pointer");
   const size_t es = elt_size(dtype);
-  // coefficient storage: C1 (nblk+1 blocks) | C2 (nblk blocks) | Gw0 | Gw1 | Gw2 | flag
-  double* base = static_cast<double*>(workspace2(h, sizeof(double) * (static_cast<size_t>(2 * nblk + 4) * BB) + 64));
+  // coefficient storage: C1 (nblk+1 blocks) | C2 (nblk blocks) | Gw0 | flag
+  double* base = static_cast<double*>(workspace2(h, sizeof(double) * (static_cast<size_t>(2 * nblk + 2) * BB) + 64));
   if (!base) return TRL_ENOMEM;
   double* C1 = base;
   double* C2 = C1 + static_cast<size_t>(nblk + 1) * BB;
   double* Gw0 = C2 + static_cast<size_t>(nblk) * BB;
-  double* Gw1 = Gw0 + BB;
-  double* Gw2 = Gw1 + BB;
-  int* flag = reinterpret_cast<int*>(Gw2 + BB);
+  int* flag = reinterpret_cast<int*>(Gw0 + BB);
   const bool contiguous = static_cast<const char*>(W) == static_cast<const char*>(V) + static_cast<size_t>(nblk) * n * bs * es;
   int st = TRL_OK;
   TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
@@ -1361,39 +1649,24 @@ int trl_cuda_project_out(trl_cuda_handle h, int dtype, const void* V, int nblk, 
     // pass 1: C1 = V^T w (and w^T w, for free when w is the block right after V)
     {
       ProfScope prof(h, PROF_DOT, (nblk + (contiguous ? 1.0 : 2.0)) * n * bs * es, 2.0 * (nblk + 1) * n * bs * bs);
-      if (contiguous) {
-        st = launch_block_dot<T, BS>(h, Vt, nblk + 1, Wt, n, C1);
-        if (!st) st = trl_cuda_memcpy(h, Gw0, C1 + static_cast<size_t>(nblk) * BB, sizeof(double) * BB, TRL_D2D);
-      }
-      else {
-        st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C1);
-        if (!st) st = launch_block_dot<T, BS>(h, Wt, 1, Wt, n, Gw0);
-      }
+      st = launch_block_dot<T, BS>(h, Vt, nblk + (contiguous ? 1 : 0), Wt, n, C1);
+      if (contiguous) Gw0 = C1 + static_cast<size_t>(nblk) * BB;
+      else if (!st) st = launch_block_dot<T, BS>(h, Wt, 1, Wt, n, Gw0);
     }
     if (st) return st;
     {
       ProfScope prof(h, PROF_UPDATE, (nblk + 2.0) * n * bs * es, 2.0 * nblk * n * bs * bs + 2.0 * n * bs * bs);
-      st = launch_update_gram<T, BS>(h, Vt, nblk, C1, Wt, n, 1, -1.0, Gw1, nullptr);
+      st = launch_update_gram<T, BS>(h, Vt, nblk, C1, Wt, n, nullptr, FinishGram<BS>{G, Gw0, eta * eta, mode == TRL_CGS_IFNEEDED ? flag : nullptr});
     }
-    if (st) return st;
-    if (mode == TRL_CGS_ONE) return trl_cuda_memcpy(h, G, Gw1, sizeof(double) * BB, TRL_D2D);
-    if (mode == TRL_CGS_TWO) {
-      cudaMemsetAsync(flag, 0x01, sizeof(int), h->stream);
-    }
-    else {
-      launch(k_dgks_flag<BS>, 1, 32, 0, h->stream, Gw0, Gw1, eta * eta, flag);
-      if ((st = after_launch(h, "dgks"))) return st;
-    }
-    // pass 2, only where the flag is set (decided on the device; its bytes are not credited
-    // to the profile because the host does not know whether it ran)
+    if (st || mode == TRL_CGS_ONE) return st;
+    // pass 2, always or only where the flag is set (decided on the device; its bytes are not
+    // credited to the profile because the host does not know whether it ran)
     {
       ProfScope prof(h, PROF_REORTH2, 0.0);
-      st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C2, flag);
-      if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C2, Wt, n, 1, -1.0, Gw2, flag);
+      const int* cond = mode == TRL_CGS_IFNEEDED ? flag : nullptr;
+      st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C2, cond);
+      if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C2, Wt, n, cond, FinishGram<BS>{G, nullptr, 0.0, nullptr});
     }
-    if (st) return st;
-    launch(k_select_block, 1, 256, 0, h->stream, flag, Gw2, Gw1, G, BB);
-    st = after_launch(h, "select");
   }));
   return st;
 }
@@ -1407,16 +1680,13 @@ int trl_cuda_project_out_sketch(trl_cuda_handle h, int dtype, const void* V, int
   const int BB = bs * bs;
   if (n == 0) return trl_cuda_memset_zero(h, G, sizeof(double) * BB);
   if (!V || !W || !S) return set_error(h, TRL_EINVAL, "null pointer");
-  // coefficient storage: C1 (nblk blocks) | C2 (nblk blocks) | E | Gw0 | Gw1 | Gw2 | flags
-  double* base = static_cast<double*>(workspace2(h, sizeof(double) * (static_cast<size_t>(2 * nblk + 4) * BB) + 64));
+  // coefficient storage: C1 (nblk blocks) | C2 (nblk blocks) | Gw0 | flags
+  double* base = static_cast<double*>(workspace2(h, sizeof(double) * (static_cast<size_t>(2 * nblk + 1) * BB) + 64));
   if (!base) return TRL_ENOMEM;
   double* C1 = base;
   double* C2 = C1 + static_cast<size_t>(nblk) * BB;
-  double* E = C2 + static_cast<size_t>(nblk) * BB; // [E; Gw0] = [S, W]^T W in one pass
-  double* Gw0 = E + BB;
-  double* Gw1 = Gw0 + BB;
-  double* Gw2 = Gw1 + BB;
-  int* flag1 = reinterpret_cast<int*>(Gw2 + BB);
+  double* Gw0 = C2 + static_cast<size_t>(nblk) * BB;
+  int* flag1 = reinterpret_cast<int*>(Gw0 + BB);
   int* flag2 = flag1 + 1;
   const size_t es = elt_size(dtype);
   int st = TRL_OK;
@@ -1426,40 +1696,28 @@ int trl_cuda_project_out_sketch(trl_cuda_handle h, int dtype, const void* V, int
     T* Wt = static_cast<T*>(W);
     {
       ProfScope prof(h, PROF_DOT, 3.0 * n * bs * es, 4.0 * n * bs * bs);
-      st = launch_block_dot_two<T, BS>(h, St, Wt, Wt, n, E);
+      // [E; G] = [S, W]^T W in one pass over W, the decision, and G = W^T W as it stands
+      st = launch_block_dot_finish<T, BS, 2, 4>(h, St, Wt - St, Wt, n, nullptr, FinishSketch<BS>{G, Gw0, thr * thr, flag1, flag2, pair_state});
     }
     if (st) return st;
-    launch(k_sketch_flag<BS>, 1, 32, 0, h->stream, E, Gw0, thr * thr, flag1, pair_state);
-    if ((st = after_launch(h, "sketch flag"))) return st;
     // both passes only where flagged (decided on the device; their bytes are not credited
     // to the profile because the host does not know whether they ran)
     {
       ProfScope prof(h, PROF_REORTH2, 0.0);
       st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C1, flag1);
-      if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C1, Wt, n, 1, -1.0, Gw1, flag1);
-      if (st) return st;
-      launch(k_dgks_flag_after<BS>, 1, 32, 0, h->stream, flag1, Gw0, Gw1, eta * eta, flag2);
-      if ((st = after_launch(h, "dgks"))) return st;
-      st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C2, flag2);
-      if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C2, Wt, n, 1, -1.0, Gw2, flag2);
+      if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C1, Wt, n, flag1, FinishGram<BS>{G, Gw0, eta * eta, flag2});
+      if (!st) st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C2, flag2);
+      if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C2, Wt, n, flag2, FinishGram<BS>{G, nullptr, 0.0, nullptr});
     }
-    if (st) return st;
-    launch(k_select_block3, 1, 256, 0, h->stream, flag1, flag2, Gw0, Gw1, Gw2, G, BB);
-    st = after_launch(h, "select");
 #ifdef TRL_DEBUG_TRACE
     // debug builds (-DTRL_DEBUG_TRACE) with TRL_PARTIAL_TRACE set: one stderr line per call
     // (synchronises; diagnostics only)
     static const bool trace = std::getenv("TRL_PARTIAL_TRACE") != nullptr;
     if (!st && trace) {
-      double eg[2 * 256];
       int fl[2];
-      cudaMemcpyAsync(eg, E, sizeof(double) * 2 * BB, cudaMemcpyDeviceToHost, h->stream);
       cudaMemcpyAsync(fl, flag1, sizeof(int) * 2, cudaMemcpyDeviceToHost, h->stream);
       cudaStreamSynchronize(h->stream);
-      double e2 = 0.0, tr = 0.0;
-      for (int i = 0; i < BB; ++i) e2 += eg[i] * eg[i];
-      for (int c = 0; c < bs; ++c) tr += eg[BB + c * bs + c];
-      std::fprintf(stderr, "partial nblk %d loss %.3e projected %d forced %d second %d\n", nblk, std::sqrt(e2 / tr), fl[0] & 1, (fl[0] >> 1) & 1, fl[1]);
+      std::fprintf(stderr, "partial nblk %d projected %d forced %d second %d\n", nblk, fl[0] & 1, (fl[0] >> 1) & 1, fl[1]);
     }
 #endif
   }));
@@ -1549,7 +1807,8 @@ static int noalloc_dot(cudaStream_t stream, int sms, double* partial, const T* V
   chunks = (n + rows_per_cta - 1) / rows_per_cta;
   // every (chunk, block) entry of the partials is written before it is read in this call,
   // so nothing left in the array by an earlier call is used and nothing needs clearing
-  launch(k_block_dot<T, BS, JC, G>, dim3(gj, static_cast<unsigned>(chunks)), kThreads, 0, stream, V, n * BS, nblk, W, n, rows_per_cta, partial, nullptr);
+  launch(k_block_dot<T, BS, JC, G, FinishNone>, dim3(gj, static_cast<unsigned>(chunks)), kThreads, 0, stream, V, n * BS, nblk, W, n, rows_per_cta, partial, nullptr, Tickets{},
+         FinishNone{});
   if (cudaGetLastError() != cudaSuccess) return TRL_ECUDA;
   launch_reduce(stream, partial, chunks, len, C, nullptr);
   if (cudaGetLastError() != cudaSuccess) return TRL_ECUDA;

@@ -25,7 +25,7 @@ struct trl_cuda_context {
   void* ws = nullptr;       // growable device workspace (per-call partial sums)
   void* ws2 = nullptr;      // growable device workspace (coefficients kept across calls of one operation)
   size_t ws2_bytes = 0;
-  double* d_small = nullptr; // 1024 doubles of fixed scratch (Gram / factor blocks)
+  double* d_small = nullptr; // fixed scratch (Gram matrix, factors, ticket counters)
   size_t ws_bytes = 0;
   int* pinned_status = nullptr; // pinned host copy of d_status
   void* pinned = nullptr;   // small pinned host staging buffer
@@ -64,7 +64,9 @@ inline bool valid_dtype(int dt) { return dt == TRL_F64 || dt == TRL_F32; }
 // Checks cudaGetLastError after a launch and counts the launch.
 int after_launch(trl_cuda_context* h, const char* what);
 
-// 1024 doubles of per-handle device scratch (Gram / factor blocks); nullptr on failure.
+// Per-handle device scratch of fixed size, in doubles from its start: a Gram matrix, the factors of a
+// CholQR (up to 4), and ticket counters (zero between kernels); nullptr on failure.
+constexpr int kSmallFactors = 256, kSmallTickets = kSmallFactors + 4 * 256, kSmallDoubles = kSmallTickets + 256;
 void* small_scratch(trl_cuda_context* h);
 // Releases the cuSOLVER handle and its workspace.
 void destroy_solver(trl_cuda_context* h);

@@ -165,14 +165,14 @@ namespace trl_detail {
 void* small_scratch(trl_cuda_context* h)
 {
   if (!h->d_small) {
-    if (cudaMalloc(&h->d_small, 1024 * sizeof(double)) != cudaSuccess) {
+    if (cudaMalloc(&h->d_small, kSmallDoubles * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       h->d_small = nullptr;
       set_error(h, TRL_ENOMEM, "scratch allocation failed");
       return nullptr;
     }
-    // zeroed once: the CholQR factor's ticket counter (doubles 768..) must start at zero
-    cudaMemsetAsync(h->d_small, 0, 1024 * sizeof(double), h->stream);
+    // zeroed once: the ticket counters must start at zero
+    cudaMemsetAsync(h->d_small, 0, kSmallDoubles * sizeof(double), h->stream);
   }
   return h->d_small;
 }
