@@ -1,0 +1,78 @@
+"""The prepared SpMM of operators with long rows (16 or more slots per slice), whose warps take their
+slices from a counter: every residue of the row lengths modulo the 8 slots of a group, empty rows,
+fewer slices than warps, rows of one window only, and a last window with missing slices; the counter
+starts at zero again in every call, and two handles may use one operator at the same time.
+Bit for bit the CSR kernel's per-row walk (trl_cuda_spmm_blocks), and the oracle to the
+tolerances of test_sell_gpu.py."""
+import numpy as np
+import pytest
+import torch
+
+from trl_b200 import native
+from trl_b200 import problems as P
+
+from test_kernels_gpu import BS, DT, as_dt, dev
+from test_sell_gpu import _mag
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(deg, seed):
+    rng = np.random.default_rng(seed)
+    n = deg.size
+    cols = np.concatenate([rng.choice(n, size=d, replace=False) for d in deg])
+    return P._from_coo(n, np.repeat(np.arange(n), deg), cols, rng.standard_normal(cols.size))
+
+
+def _patterns():
+    n = 9000  # three windows, the last one incomplete
+    skewed = 17 + np.arange(n) % 9
+    skewed[::501] = 700
+    skewed[5::13] = 0
+    return [("residues", _rows(16 + np.arange(997) % 41, 1)), ("skewed", _rows(skewed, 2)), ("one_slice", _rows(np.full(31, 31), 3))]
+
+
+PATTERNS = _patterns()
+
+
+@pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("case", PATTERNS, ids=lambda c: c[0])
+def test_long_rows(cuda_handle, bs, dtype, case):
+    A = case[1]
+    rng = np.random.default_rng(bs)
+    Ad = native.DeviceCSRTensors.from_host(A, dtype)
+    op = cuda_handle.prepare(Ad, bs)
+    X = as_dt(rng.standard_normal((A.n, bs)), dtype)
+    W = as_dt(rng.standard_normal((A.n, bs)), dtype)
+    Xd, Wd = dev(X, dtype), dev(W, dtype)
+    ref = torch.empty((2, A.n, bs), dtype=dtype, device="cuda")
+    cuda_handle.spmm_blocks(Ad, torch.stack([Xd, Xd]), ref, -0.5, 2.0, 0.25, torch.stack([Wd, Wd]))
+    for _ in range(3):
+        Y = torch.full((A.n, bs), float("nan"), dtype=dtype, device="cuda")
+        op.spmm(Xd, Y, -0.5, 2.0, 0.25, Wd)
+        assert torch.equal(Y, ref[0])
+    vals = A.values.astype(np.float32).astype(np.float64) if dtype == torch.float32 else A.values
+    host = -0.5 * P.CSRMatrix(A.n, A.rowptr, A.colind, vals).matmat(X) + 2.0 * X + 0.25 * W
+    scale = 0.5 * _mag(A, vals, X) + 2.0 * np.abs(X).max() + 0.25 * np.abs(W).max()
+    assert np.abs(Y.double().cpu().numpy() - host).max() <= (1e-12 if dtype == torch.float64 else 2e-6) * scale
+    op.close()
+
+
+def test_one_operator_on_two_handles(cuda_handle):
+    A = PATTERNS[1][1]
+    op = cuda_handle.prepare(native.DeviceCSRTensors.from_host(A), 8)
+    X = torch.randn((A.n, 8), dtype=torch.float64, device="cuda")
+    ref = torch.empty_like(X)
+    op.spmm(X, ref)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    handles = [native.Handle(0, s) for s in streams]
+    out = [[torch.full_like(X, float("nan")) for _ in range(20)] for _ in handles]
+    torch.cuda.synchronize()
+    for k in range(20):
+        for h, o in zip(handles, out):
+            h.check(h.lib.trl_cuda_op_spmm(h.h, op.op, X.data_ptr(), o[k].data_ptr(), 1, 1.0, 0.0, 0.0, None))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, ref) for o in out for y in o)
+    op.close()

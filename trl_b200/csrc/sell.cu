@@ -18,6 +18,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <utility>
 
 namespace {
 
@@ -271,22 +272,19 @@ namespace {
 constexpr int kSpmmThreads = 256;
 constexpr int kSpmmWarps = kSpmmThreads / 32;
 
-// Per instantiation: NBG blocks accumulated per pass over a slice (1 for the single-block
-// SpMM; the multi-block SpMM takes up to kSellBlocksPerPass blocks per pass and re-reads a
-// slice's indices and values, from L2, for each further pass), UG slots per group, and the
-// CTAs per SM the registers must allow.
-template <typename T, int BS, int NBG, bool LONG>
+// Per instantiation of k_spmm_sell: NBG blocks accumulated per pass over a slice (1 for the
+// single-block SpMM of short rows; the multi-block SpMM takes up to kSellBlocksPerPass blocks per
+// pass and re-reads a slice's indices and values, from L2, for each further pass), UG slots per
+// group, and the CTAs per SM the registers must allow. Short rows prefer many warps with few slots
+// each (measured on B200: 96^3 stencil, 7 slots per slice, 0.56 of the copy peak with 2 slots x 4
+// CTAs against 0.53 with 8 x 2). Several blocks per pass keep one slot per lane in flight for
+// each block.
+template <typename T, int BS, int NBG>
 struct SellTune {
   static constexpr int lane_bytes = SellShape<T, BS>::VEC * static_cast<int>(sizeof(T));
   static constexpr int ug = 64 / lane_bytes;
-  // operators with long rows (LONG: 16 or more slots per slice on average) keep 8 slots of
-  // gathers in flight per lane at two CTAs per SM; short rows prefer more warps with fewer
-  // slots each (measured on B200: 96^3 stencil, 7 slots per slice, 0.56 of the copy peak
-  // with 2 slots x 4 CTAs against 0.53 with 8 x 2; elasticity, 81 slots, 0.50 with 8 x 2
-  // against 0.39 with 2 x 4). Several blocks per pass keep one slot per lane in flight for
-  // each block.
-  static constexpr int UG = NBG == 1 ? (LONG ? 8 : (ug > 4 ? 4 : ug)) : (NBG > 2 ? 1 : 2);
-  static constexpr int MINB = NBG == 1 ? (LONG ? 2 : 4) : 2;
+  static constexpr int UG = NBG == 1 ? (ug > 4 ? 4 : ug) : (NBG > 2 ? 1 : 2);
+  static constexpr int MINB = NBG == 1 ? 4 : 2;
 };
 
 // Blocks per pass of the multi-block SpMM (the Chebyshev filter's kept blocks). Measured on
@@ -311,14 +309,14 @@ __device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes)
 // loads the column indices of group g + 1, which may belong to the next slice. The bounds
 // and rows of the next slice are loaded one slice ahead, and lane 0 asks L2 for the slice
 // after it (bulk prefetch), so that the index loads hit L2.
-template <typename T, int BS, int NBG, bool LONG>
-__global__ void __launch_bounds__(kSpmmThreads, SellTune<T, BS, NBG, LONG>::MINB)
+template <typename T, int BS, int NBG>
+__global__ void __launch_bounds__(kSpmmThreads, SellTune<T, BS, NBG>::MINB)
     k_spmm_sell(int nslices, int nwin, int spw, int interleave, const int32_t* __restrict__ perm, const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
                 const T* __restrict__ sval, const T* __restrict__ X, T* Y, T alpha, T beta, T gamma, const T* W, int nb, int64_t bstride)
 {
   ::trl_detail::pdl_enter();
   using S = SellShape<T, BS>;
-  constexpr int VEC = S::VEC, LPR = S::LPR, C = S::RPW, UG = SellTune<T, BS, NBG, LONG>::UG;
+  constexpr int VEC = S::VEC, LPR = S::LPR, C = S::RPW, UG = SellTune<T, BS, NBG>::UG;
   const int lane = threadIdx.x & 31;
   const int grp = lane / LPR, sub = lane % LPR;
   const int wstride = static_cast<int>(gridDim.x) * kSpmmWarps;
@@ -356,7 +354,10 @@ __global__ void __launch_bounds__(kSpmmThreads, SellTune<T, BS, NBG, LONG>::MINB
     for (int u = 0; u < UG; ++u) c[u] = j + u < slen ? ld_stream(scol + e0 + static_cast<int64_t>(j + u) * C + grp) : -1;
   };
 
-  int i = next_valid(static_cast<int>(blockIdx.x) * kSpmmWarps + static_cast<int>(threadIdx.x >> 5));
+  // in the ranked order neighbours are equally long: they go to different SMs
+  const int warp = static_cast<int>(threadIdx.x >> 5);
+  const int first = interleave ? warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kSpmmWarps + warp;
+  int i = next_valid(first);
   if (i >= total) return;
   int in = next_valid(i + wstride);
   Slice cur = load_slice(i), nxt = load_slice(in);
@@ -366,7 +367,7 @@ __global__ void __launch_bounds__(kSpmmThreads, SellTune<T, BS, NBG, LONG>::MINB
     const int nbh = nb - b0 < NBG ? nb - b0 : NBG;
     const T* Xb = X + static_cast<int64_t>(b0) * bstride + sub * VEC;
     if (b0 > 0) { // start the walk again
-      i = next_valid(static_cast<int>(blockIdx.x) * kSpmmWarps + static_cast<int>(threadIdx.x >> 5));
+      i = next_valid(first);
       in = next_valid(i + wstride);
       cur = load_slice(i);
       nxt = load_slice(in);
@@ -446,6 +447,197 @@ __global__ void __launch_bounds__(kSpmmThreads, SellTune<T, BS, NBG, LONG>::MINB
       slen = static_cast<int>((cur.e1 - cur.e0) / C);
       j = 0;
     }
+  }
+}
+
+// One entry of the slice stream at p + OFF elements, not kept in L1 (read once): a constant offset
+// costs no address arithmetic.
+template <int OFF>
+__device__ __forceinline__ int ld_slot(const int32_t* p)
+{
+  int v;
+  asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1 + %2];" : "=r"(v) : "l"(p), "n"(OFF * 4));
+  return v;
+}
+template <int OFF>
+__device__ __forceinline__ double ld_slot(const double* p)
+{
+  double v;
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1 + %2];" : "=d"(v) : "l"(p), "n"(OFF * 8));
+  return v;
+}
+template <int OFF>
+__device__ __forceinline__ float ld_slot(const float* p)
+{
+  float v;
+  asm volatile("ld.global.nc.L1::no_allocate.f32 %0, [%1 + %2];" : "=f"(v) : "l"(p), "n"(OFF * 4));
+  return v;
+}
+
+// out[u] = slot u of a slice (slots C apart) for u < UG, or for u < count
+template <int C, typename V, int... U>
+__device__ __forceinline__ void load_slots(V* out, const V* p, std::integer_sequence<int, U...>)
+{
+  ((out[U] = ld_slot<U * C>(p)), ...);
+}
+template <int C, typename V, int... U>
+__device__ __forceinline__ void load_slots(V* out, const V* p, int count, std::integer_sequence<int, U...>)
+{
+  (((U < count) ? static_cast<void>(out[U] = ld_slot<U * C>(p)) : static_cast<void>(0)), ...);
+}
+
+// One block on an operator with long rows (16 or more slots per slice on average): kSellLongSlots
+// slots of gathers in flight per lane at two CTAs per SM (96^3-node elasticity, 81 slots: 0.50 of the
+// copy peak with 8 x 2 against 0.39 with 2 x 4). Bound by the gathers' L1 wavefronts and, for
+// irregular patterns, by L2-to-SM traffic; the walk of k_spmm_sell spent half of the issue slots on
+// tests and addresses, so here only the last group of a slice tests its slots, and the others'
+// loads are constant offsets from two running pointers.
+// The warps take slices from a counter (at zero between launches) instead of every (number of
+// warps)-th: on the Zipf pattern a slice holds up to 512 slots where a warp's whole share is 480, and
+// a third of the SMs' time was spent waiting for the last warps. For such skewed patterns
+// (`ranked`) the longest slices of all windows come first, and the first ones go to different SMs.
+// Measured on B200, us (before: k_spmm_sell with 8 slots x 2 CTAs, static): elasticity 64^3 bs 8 FP64 223
+// (257), FP32 127 (148); Zipf 524,288 rows FP32 bs 16 115 (170), FP64 bs 8 121 (132-181), FP64 bs 16 181
+// (187-204), FP32 bs 4 114 (180). The counter alone gave 124 and 131 us in place of 115 and 121.
+constexpr int kSellLongSlots = 8;
+
+template <typename T, int BS>
+__global__ void __launch_bounds__(kSpmmThreads, 2)
+    k_spmm_sell_long(int nslices, int nwin, int spw, unsigned* counter, int ranked, const int32_t* __restrict__ perm, const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
+                     const T* __restrict__ sval, const T* __restrict__ X, T* Y, T alpha, T beta, T gamma, const T* W)
+{
+  ::trl_detail::pdl_enter();
+  using S = SellShape<T, BS>;
+  constexpr int VEC = S::VEC, LPR = S::LPR, C = S::RPW, UG = kSellLongSlots;
+  constexpr auto slots = std::make_integer_sequence<int, UG>{};
+  const int lane = threadIdx.x & 31;
+  const int grp = lane / LPR, sub = lane % LPR;
+  const int nwarps = static_cast<int>(gridDim.x) * kSpmmWarps;
+  const int total = ranked ? nwin * spw : nslices;
+  // ranked: window-major within each slice rank
+  auto slice_of = [&](int i) -> int {
+    return ranked ? static_cast<int>(static_cast<unsigned>(i) % static_cast<unsigned>(nwin)) * spw + static_cast<int>(static_cast<unsigned>(i) / static_cast<unsigned>(nwin)) : i;
+  };
+  // the next place: asked for early by lane 0, shared when it is needed
+  int ticket = 0;
+  auto ask = [&]() {
+    if (lane == 0) ticket = static_cast<int>(atomicAdd(counter, 1u)) + nwarps;
+  };
+  auto answer = [&]() {
+    int i = __shfl_sync(0xffffffffu, ticket, 0);
+    while (i < total && slice_of(i) >= nslices) { // the last window's missing slices
+      ask();
+      i = __shfl_sync(0xffffffffu, ticket, 0);
+    }
+    return i;
+  };
+  struct Slice {
+    int64_t e0;
+    int left, row; // slots not taken yet; this lane's row
+  };
+  auto load_slice = [&](int i) {
+    Slice q{0, 0, -1};
+    if (i < total) {
+      const int s = slice_of(i);
+      q.e0 = __ldg(sptr + s);
+      q.left = static_cast<int>(static_cast<unsigned>(__ldg(sptr + s + 1) - q.e0) / C);
+      q.row = __ldg(perm + static_cast<int64_t>(s) * C + grp);
+    }
+    return q;
+  };
+  auto prefetch_slice = [&](const Slice& q) {
+    if (lane == 0 && q.left > 0) {
+      prefetch_l2(scol + q.e0, static_cast<uint32_t>(q.left * C * 4));
+      prefetch_l2(sval + q.e0, static_cast<uint32_t>(q.left * C * sizeof(T)));
+    }
+  };
+  const int warp = static_cast<int>(threadIdx.x >> 5);
+  ticket = ranked ? warp * static_cast<int>(gridDim.x) + static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x) * kSpmmWarps + warp;
+  int i = answer();
+  ask();
+  Slice cur = load_slice(i);
+  int in = answer();
+  ask();
+  Slice nxt = load_slice(in);
+  prefetch_slice(cur);
+  prefetch_slice(nxt);
+  const T* Xb = X + sub * VEC;
+  const int32_t* cp = scol + cur.e0 + grp;
+  const T* vp = sval + cur.e0 + grp;
+  int c[UG];
+#pragma unroll
+  for (int u = 0; u < UG; ++u) c[u] = 0;
+  load_slots<C>(c, cp, cur.left, slots);
+  T acc[VEC];
+#pragma unroll
+  for (int v = 0; v < VEC; ++v) acc[v] = T(0);
+  while (i < total) {
+    T x[UG][VEC];
+    T a[UG];
+    if (cur.left >= UG) { // a whole group
+#pragma unroll
+      for (int u = 0; u < UG; ++u) load_row<T, VEC>(Xb + static_cast<int64_t>(c[u]) * BS, x[u]);
+      cur.left -= UG;
+      cp += UG * C;
+      if (cur.left >= UG) load_slots<C>(c, cp, slots);
+      else if (cur.left > 0) load_slots<C>(c, cp, cur.left, slots);
+      else load_slots<C>(c, scol + nxt.e0 + grp, nxt.left, slots); // the next slice's first group
+      load_slots<C>(a, vp, slots);
+      vp += UG * C;
+#pragma unroll
+      for (int u = 0; u < UG; ++u)
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) acc[v] = fma(a[u], x[u][v], acc[v]);
+      if (cur.left > 0) continue;
+    }
+    else { // the rest of a slice (an empty slice: nothing)
+      load_slots<C>(a, vp, cur.left, slots);
+#pragma unroll
+      for (int u = 0; u < UG; ++u)
+        if (u < cur.left) load_row<T, VEC>(Xb + static_cast<int64_t>(c[u]) * BS, x[u]);
+      load_slots<C>(c, scol + nxt.e0 + grp, nxt.left, slots);
+#pragma unroll
+      for (int u = 0; u < UG; ++u)
+        if (u < cur.left)
+#pragma unroll
+          for (int v = 0; v < VEC; ++v) acc[v] = fma(a[u], x[u][v], acc[v]);
+    }
+    // the slice is complete: write its rows
+    if (cur.row >= 0) {
+      const int64_t off = static_cast<int64_t>(cur.row) * BS + sub * VEC;
+      T y[VEC];
+      if (beta != T(0)) {
+        T xr[VEC];
+        load_row<T, VEC>(X + off, xr);
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) y[v] = fma(alpha, acc[v], beta * xr[v]); // explicit: the same rounding as the CSR kernel
+      }
+      else {
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) y[v] = alpha * acc[v];
+      }
+      if (W) { // W may be Y itself: this lane reads its values before it writes them
+#pragma unroll
+        for (int v = 0; v < VEC; ++v) y[v] = fma(gamma, W[off + v], y[v]);
+      }
+      store_row<T, VEC>(Y + off, y);
+    }
+#pragma unroll
+    for (int v = 0; v < VEC; ++v) acc[v] = T(0);
+    i = in;
+    cur = nxt;
+    cp = scol + cur.e0 + grp;
+    vp = sval + cur.e0 + grp;
+    if (i < total) {
+      in = answer();
+      ask();
+      nxt = load_slice(in);
+      prefetch_slice(nxt);
+    }
+  }
+  if (lane == 0) { // the last warp leaves the counters at zero
+    __threadfence();          // this warp's last ticket is taken before it counts as done
+    if (atomicAdd(counter + 1, 1u) == static_cast<unsigned>(nwarps - 1)) counter[0] = counter[1] = 0u;
   }
 }
 
@@ -595,23 +787,37 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
   ProfScope prof(h, PROF_SPMM, op->nnz * (es + 4.0) + 4.0 * (op->n + 1) + nb * (W ? 3.0 : 2.0) * op->n * bs * es, 2.0 * op->nnz * bs * nb);
   int st = TRL_OK;
   const int dtype = op->dtype;
+  // the slice counter and the count of finished warps belong to the handle: an operator may serve several
+  unsigned* counter = nullptr;
+  if (op->long_rows && nb == 1) {
+    double* small = static_cast<double*>(small_scratch(h));
+    if (!small) return TRL_ENOMEM;
+    counter = reinterpret_cast<unsigned*>(small + kSmallCounters);
+  }
   TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
-    const auto run = [&](auto kernel, int minb) {
+    // one resident wave
+    const auto wave = [&](auto kernel, int minb) {
       static int resident[64]; // per device and instantiation of the kernel
       int& res = resident[h->device & 63];
       if (res == 0) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, kernel, kSpmmThreads, 0) != cudaSuccess || res < 1) res = minb;
         cudaGetLastError();
       }
-      // one resident wave; every warp strides over the slices
-      const unsigned grid = grid_for(h, op->nslices, kSpmmWarps, res);
-      trl_detail::launch(kernel, grid, kSpmmThreads, 0, h->stream, static_cast<int>(op->nslices), static_cast<int>(op->nwin), op->spw, op->interleave, op->perm, op->sptr, op->scol, static_cast<const T*>(op->sval),
-                                                   static_cast<const T*>(X), static_cast<T*>(Y), static_cast<T>(alpha), static_cast<T>(beta), static_cast<T>(gamma),
-                                                   static_cast<const T*>(W), nb, op->n * BS);
+      return grid_for(h, op->nslices, kSpmmWarps, res);
     };
-    if (nb > 1) run(k_spmm_sell<T, BS, kSellBlocksPerPass, false>, SellTune<T, BS, kSellBlocksPerPass, false>::MINB);
-    else if (op->long_rows) run(k_spmm_sell<T, BS, 1, true>, SellTune<T, BS, 1, true>::MINB);
-    else run(k_spmm_sell<T, BS, 1, false>, SellTune<T, BS, 1, false>::MINB);
+    const int ns = static_cast<int>(op->nslices), nwin = static_cast<int>(op->nwin);
+    const T* vals = static_cast<const T*>(op->sval);
+    const T* Wt = static_cast<const T*>(W);
+    const T a = static_cast<T>(alpha), b = static_cast<T>(beta), g = static_cast<T>(gamma);
+    const auto run = [&](auto kernel, int minb) {
+      trl_detail::launch(kernel, wave(kernel, minb), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, op->interleave, op->perm, op->sptr, op->scol, vals, static_cast<const T*>(X),
+                         static_cast<T*>(Y), a, b, g, Wt, nb, op->n * BS);
+    };
+    if (nb > 1) run(k_spmm_sell<T, BS, kSellBlocksPerPass>, SellTune<T, BS, kSellBlocksPerPass>::MINB);
+    else if (op->long_rows)
+      trl_detail::launch(k_spmm_sell_long<T, BS>, wave(k_spmm_sell_long<T, BS>, 2), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, counter, op->interleave, op->perm, op->sptr, op->scol, vals,
+                         static_cast<const T*>(X), static_cast<T*>(Y), a, b, g, Wt);
+    else run(k_spmm_sell<T, BS, 1>, SellTune<T, BS, 1>::MINB);
     st = after_launch(h, "spmm (sliced ELL)");
   }));
   return st;
