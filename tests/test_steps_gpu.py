@@ -74,3 +74,40 @@ def test_cholqr_breakdown_leaves_block_and_factor(cuda_handle, bs, passes):
             cuda_handle.sync()
         close(host(Y).T @ host(Y), np.eye(bs), 1.0, 1e-12)
         close(host(Y) @ host(R), host(X), host(X.abs()).max(), 1e-12)
+
+
+@pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("n,nblk", [(40, 1), (353, 3), (2368, 9), (2369, 5), (8192, 17), (8193, 2), (65536, 2), (65537, 2)])
+def test_projections_at_the_edges_of_one_launch(cuda_handle, bs, dtype, n, nblk):
+    """Rows at the edges of a CTA's share and of the range of the one-launch projection, blocks at those
+    of a warp's: the if-needed projection with one and two passes, and the sketch's with a threshold it
+    misses and one it exceeds, against numpy's Gram-Schmidt. n eps sum|terms| <= 1e-12 of the
+    magnitude in 64 bits, the storage's rounding (2e-6) in 32."""
+    if nblk * bs > n:
+        nblk = n // bs
+    rng = np.random.default_rng(n + bs)
+    Vf = as_dt(np.linalg.qr(rng.standard_normal((n, nblk * bs)))[0], dtype)
+    V = np.ascontiguousarray(Vf.reshape(n, nblk, bs).transpose(1, 0, 2))
+    eps = 1e-12 if dtype == torch.float64 else 2e-6
+    Vd = dev(V, dtype)
+    for size in (100.0, 1e-3):  # components along V: two passes, one pass
+        w = as_dt(Vf @ rng.standard_normal((nblk * bs, bs)) * size + rng.standard_normal((n, bs)), dtype)
+        w1 = w - Vf @ (Vf.T @ w)
+        lost = np.any((w1 * w1).sum(0) < 0.5 * (w * w).sum(0))
+        ref = w1 - Vf @ (Vf.T @ w1) if lost else w1
+        for _ in range(2):
+            Wd = dev(w, dtype)
+            G = torch.full((bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+            cuda_handle.project_out(Vd, Wd, native.TRL_CGS_IFNEEDED, G)
+            close(host(Wd), ref, np.abs(w).max(), eps)
+            close(host(G), host(Wd).T @ host(Wd), max(np.abs(host(G)).max(), 1e-300), 1e-10)
+        S = as_dt(sum(V[j] @ (rng.standard_normal((bs, bs)) / np.sqrt(bs)) for j in range(nblk)), dtype)
+        est = np.linalg.norm(S.T @ w) / np.linalg.norm(w)
+        for thr, out in ((est * 100, w), (est / 100, ref)):
+            Wd = dev(w, dtype)
+            G = torch.full((bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+            cuda_handle.project_out_sketch(Vd, Wd, dev(S, dtype), thr, G)
+            close(host(Wd), out, np.abs(w).max(), eps)
+            close(host(G), host(Wd).T @ host(Wd), max(np.abs(host(G)).max(), 1e-300), 1e-10)
+    cuda_handle.sync()

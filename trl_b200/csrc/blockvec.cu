@@ -1166,6 +1166,261 @@ __global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const doub
   }
 }
 
+// ---------------------------------------------------------------- projection in one launch
+// W -= V (V^T W) against nblk blocks, the Gram matrix of the result, and a second time where a column
+// kept less than eta of its norm, by one cooperative launch of a CTA per SM: CTA r owns a range of
+// rows, and the sums over the CTAs go through global memory between grid-wide barriers. The separate
+// kernels (dot, its reduction, update; each twice, and launched also when the sketch asks for nothing)
+// cost more in launches than in work on small bases, and stream faster on large ones.
+// cond: the sketch's decision. before: the Gram matrix before the pass.
+// Measured on B200, us, separate kernels / this one. Sketch that asks for nothing: 22.8 / 10.5 at
+// every size. Sketch that asks for a projection: 1,024 x 4 x 8 blocks 23 / 20, 16,384 x 4 x 20 28 / 29,
+// 16,384 x 8 x 40 40 / 38 (FP32 36 / 43), 60,000 x 8 x 16 41 / 43, 131,072 x 4 x 14 42 / 51. (project_out
+// always runs and keeps to the separate kernels, so that its modes agree to the last bit.)
+constexpr int kProjThreads = 512;
+constexpr int kProjWarps = kProjThreads / 32;
+constexpr int kProjMaxEntries = 8192; // coefficients, nblk BS^2, in shared memory
+
+// Barrier over the grid of a cooperative launch: bar[0] arrivals (zero between barriers), bar[1]
+// generation. Bounded: false (and TRL_DEV_TIMEOUT) after the limit; the caller then leaves.
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, int* status)
+{
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    volatile unsigned* gen = bar + 1;
+    const unsigned mine = *gen;
+    __threadfence(); // this CTA's writes, and the generation read, come before its arrival
+    ok = 1;
+    if (atomicAdd(bar, 1u) == gridDim.x - 1) {
+      bar[0] = 0u;
+      __threadfence();
+      atomicAdd(bar + 1, 1u);
+    }
+    else {
+      unsigned polls = 0;
+      while (*gen == mine)
+        if (++polls == (1u << 24)) {
+          atomicOr(status, TRL_DEV_TIMEOUT);
+          ok = 0;
+          break;
+        }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+template <typename T, int BS>
+__global__ void __launch_bounds__(kProjThreads, 1) k_project(const T* V, int nblk, T* W, int64_t n, int64_t rows_per_cta, const int* __restrict__ cond,
+                                                             const double* __restrict__ before, double eta2, double* __restrict__ G, double* partial, double* total,
+                                                             double* gpartial, unsigned* bar, int* status)
+{
+  ::trl_detail::pdl_enter();
+  if (*cond == 0) return; // the whole grid
+  constexpr int NT = (BS + 7) / 8, KS = (BS + 3) / 4, BB = BS * BS;
+  constexpr int JC = BS >= 16 ? 2 : 4; // blocks a warp takes at a time in the dots
+  extern __shared__ __align__(16) double sm[];
+  double* coef = sm;                             // [nblk BB]
+  double* stage = coef + nblk * BB;              // [kProjWarps][8 BS]
+  double* red = stage + kProjWarps * 8 * BS;     // [kProjWarps][NT NT 64]
+  __shared__ double Gs[BB], G0[BB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int64_t vstride = n * BS;
+  const int64_t rb = min(n, static_cast<int64_t>(blockIdx.x) * rows_per_cta), re = min(n, rb + rows_per_cta);
+  const int ncta = static_cast<int>(gridDim.x);
+
+  // sum over the CTAs of src[c * stride + e], e = e0 .. e0 + 7, for a warp: lane (q, i) adds every 4th CTA's
+  // entry e0 + i, eight loads in flight; lanes 0 .. 7 return the totals. One order of additions.
+  const auto sum_ctas = [&](const double* src, int stride, int e0, int count) {
+    const int i = lane & 7, q = lane >> 3;
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = 0.0;
+    for (int c = q; c < ncta; c += 32)
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] += (c + 4 * u < ncta && e0 + i < count) ? __ldcg(src + static_cast<int64_t>(c + 4 * u) * stride + e0 + i) : 0.0;
+    double t = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+    t += __shfl_xor_sync(0xffffffffu, t, 8);
+    t += __shfl_xor_sync(0xffffffffu, t, 16);
+    return t;
+  };
+  // total = V^T W. The CTA's warps are split into groups of up to JC blocks each, and what is left of
+  // them over the rows.
+  const auto dots = [&]() {
+    const int len = nblk * BB;
+    const int groups = min(kProjWarps, (nblk + JC - 1) / JC), splits = kProjWarps / groups;
+    const int jg = warp % groups, rs = warp / groups; // warps with rs >= splits only join the barriers
+    constexpr int BUF = NT * NT * 64;
+    for (int j0 = 0; j0 < nblk; j0 += groups * JC) { // block j0 + jg + q * groups, q < JC
+      double acc[JC][NT][NT][2];
+#pragma unroll
+      for (int q = 0; q < JC; ++q)
+#pragma unroll
+        for (int a = 0; a < NT; ++a)
+#pragma unroll
+          for (int b = 0; b < NT; ++b) acc[q][a][b][0] = acc[q][a][b][1] = 0.0;
+      const T* Vb[JC];
+      bool on[JC];
+#pragma unroll
+      for (int q = 0; q < JC; ++q) {
+        const int j = j0 + jg + q * groups;
+        on[q] = j < nblk && rs < splits;
+        Vb[q] = V + static_cast<int64_t>(min(j, nblk - 1)) * vstride;
+      }
+      if (on[0]) {
+#pragma unroll 4
+        for (int64_t r0 = rb + 4 * rs; r0 < re; r0 += 4 * splits) {
+          const int64_t row = r0 + t4;
+          double bf[NT], av[JC][NT];
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const int col = t * 8 + g;
+            const bool ok = row < re && col < BS;
+            bf[t] = ok ? static_cast<double>(W[row * BS + col]) : 0.0;
+#pragma unroll
+            for (int q = 0; q < JC; ++q) av[q][t] = ok && on[q] ? static_cast<double>(Vb[q][row * BS + col]) : 0.0;
+          }
+#pragma unroll
+          for (int q = 0; q < JC; ++q)
+            if (on[q])
+#pragma unroll
+              for (int a = 0; a < NT; ++a)
+#pragma unroll
+                for (int b = 0; b < NT; ++b) dmma_m8n8k4(acc[q][a][b][0], acc[q][a][b][1], av[q][a], bf[b]);
+        }
+      }
+      // over the row splits, one of the JC blocks of every group at a time
+#pragma unroll
+      for (int q = 0; q < JC; ++q) {
+        if (j0 + q * groups >= nblk) break;
+#pragma unroll
+        for (int a = 0; a < NT; ++a)
+#pragma unroll
+          for (int b = 0; b < NT; ++b) {
+            red[warp * BUF + (a * NT + b) * 64 + g * 8 + 2 * t4] = acc[q][a][b][0];
+            red[warp * BUF + (a * NT + b) * 64 + g * 8 + 2 * t4 + 1] = acc[q][a][b][1];
+          }
+        __syncthreads();
+        for (int e = tid; e < groups * BUF; e += kProjThreads) {
+          const int gr = e / BUF, w = e % BUF, j = j0 + gr + q * groups;
+          const int row = (w >> 6) / NT * 8 + ((w & 63) >> 3), col = (w >> 6) % NT * 8 + (w & 7);
+          if (j < nblk && row < BS && col < BS) {
+            double v = 0.0;
+            for (int k = 0; k < splits; ++k) v += red[(k * groups + gr) * BUF + w];
+            partial[static_cast<int64_t>(blockIdx.x) * len + j * BB + row * BS + col] = v;
+          }
+        }
+        __syncthreads();
+      }
+    }
+    if (!grid_barrier(bar, status)) return false;
+    for (int e0 = (static_cast<int>(blockIdx.x) * kProjWarps + warp) * 8; e0 < len; e0 += ncta * kProjWarps * 8) {
+      const double t = sum_ctas(partial, len, e0, len);
+      if (lane < 8 && e0 + lane < len) total[e0 + lane] = t;
+    }
+    return grid_barrier(bar, status);
+  };
+  // W -= sum_j V_j C_j over this CTA's rows, and Gs = the Gram matrix of the result over all rows
+  const auto update = [&]() {
+    for (int e = tid; e < nblk * BB; e += kProjThreads) coef[e] = __ldcg(total + e);
+    __syncthreads();
+    double gacc[NT][NT][2];
+#pragma unroll
+    for (int a = 0; a < NT; ++a)
+#pragma unroll
+      for (int b = 0; b < NT; ++b) gacc[a][b][0] = gacc[a][b][1] = 0.0;
+    double* st = stage + warp * 8 * BS;
+    for (int64_t r0 = rb + warp * 8; r0 < re; r0 += kProjWarps * 8) {
+      const int64_t row = r0 + g;
+      double acc[NT][2];
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int col = t * 8 + 2 * t4 + i;
+          acc[t][i] = (row < re && col < BS) ? static_cast<double>(W[row * BS + col]) : 0.0;
+        }
+#pragma unroll 8
+      for (int j = 0; j < nblk; ++j) {
+        T a[KS];
+        const T* Vj = V + static_cast<int64_t>(j) * vstride;
+        if (row < re && t4 * KS < BS) load_cols<T, KS>(Vj + row * BS + t4 * KS, a);
+        else
+#pragma unroll
+          for (int ks = 0; ks < KS; ++ks) a[ks] = T(0);
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const int krow = t4 * KS + ks, col = t * 8 + g;
+            const double b = (krow < BS && col < BS) ? -coef[j * BB + krow * BS + col] : 0.0;
+            dmma_m8n8k4(acc[t][0], acc[t][1], static_cast<double>(a[ks]), b);
+          }
+      }
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int col = t * 8 + 2 * t4 + i;
+          if (col < BS) {
+            const T v = static_cast<T>(acc[t][i]);
+            if (row < re) W[row * BS + col] = v;
+            st[g * BS + col] = row < re ? static_cast<double>(v) : 0.0;
+          }
+        }
+      __syncwarp();
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int lr = q * 4 + t4;
+        double f[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t) f[t] = (t * 8 + g < BS) ? st[lr * BS + t * 8 + g] : 0.0;
+#pragma unroll
+        for (int a = 0; a < NT; ++a)
+#pragma unroll
+          for (int b = 0; b < NT; ++b) dmma_m8n8k4(gacc[a][b][0], gacc[a][b][1], f[a], f[b]);
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int a = 0; a < NT; ++a)
+#pragma unroll
+      for (int b = 0; b < NT; ++b) {
+        red[warp * (NT * NT * 64) + (a * NT + b) * 64 + g * 8 + 2 * t4] = gacc[a][b][0];
+        red[warp * (NT * NT * 64) + (a * NT + b) * 64 + g * 8 + 2 * t4 + 1] = gacc[a][b][1];
+      }
+    __syncthreads();
+    for (int e = tid; e < NT * NT * 64; e += kProjThreads) {
+      const int row = (e >> 6) / NT * 8 + ((e & 63) >> 3), col = (e >> 6) % NT * 8 + (e & 7);
+      if (row < BS && col < BS) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < kProjWarps; ++w) v += red[w * (NT * NT * 64) + e];
+        gpartial[static_cast<int64_t>(blockIdx.x) * BB + row * BS + col] = v;
+      }
+    }
+    if (!grid_barrier(bar, status)) return false;
+    for (int e0 = warp * 8; e0 < BB; e0 += kProjWarps * 8) { // every CTA for itself: the decision needs no barrier
+      const double t = sum_ctas(gpartial, BB, e0, BB);
+      if (lane < 8 && e0 + lane < BB) Gs[e0 + lane] = t;
+    }
+    __syncthreads();
+    return true;
+  };
+
+  for (int e = tid; e < BB; e += kProjThreads) G0[e] = before[e];
+  for (int pass = 0; pass < 2; ++pass) {
+    if (!dots() || !update()) return;
+    if (blockIdx.x == 0)
+      for (int e = tid; e < BB; e += kProjThreads) G[e] = Gs[e];
+    bool again = false; // the same in every CTA
+    for (int c = 0; c < BS; ++c) again |= Gs[c * BS + c] < eta2 * G0[c * BS + c];
+    if (!again) return;
+  }
+}
+
 } // namespace
 
 using namespace trl_detail;
@@ -1327,6 +1582,59 @@ int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* c
   if (!partial) return TRL_ENOMEM;
   launch(k_update_gram<T, BS, RT, 1, Fin>, grid, kThreads, 0, h->stream, in, n * BS, MB, coef, out, n, 1, -1.0, partial, cond, t, fin);
   return after_launch(h, "update_gram");
+}
+
+// The projection in one launch for small bases: true if it ran (st: its status), false if the separate
+// kernels have to: beyond kProjBytes of basis (about half of L2) or kProjRows rows, where a projection
+// costs more here than the sketches that ask for none save (k_project has the times on both sides).
+constexpr int64_t kProjBytes = int64_t(64) << 20;
+constexpr int64_t kProjRows = 65536;
+
+template <typename T, int BS>
+bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, const int* cond, const double* before, double eta2, double* G, int& st)
+{
+  constexpr int BB = BS * BS, NT = (BS + 7) / 8;
+  if (n > kProjRows || static_cast<int64_t>(nblk) * n * BS * static_cast<int64_t>(sizeof(T)) > kProjBytes || nblk * BB > kProjMaxEntries) return false;
+  const auto kern = k_project<T, BS>;
+  const auto smem = [](int entries) { return sizeof(double) * (entries + static_cast<size_t>(kProjWarps) * (8 * BS + NT * NT * 64)); };
+  static int usable[64]; // per device: 1 the kernel can be launched with the most shared memory, -1 it cannot
+  int& ok = usable[h->device & 63];
+  if (ok == 0) {
+    int resident = 0, coop = 0;
+    const size_t most = smem(kProjMaxEntries);
+    const bool fits = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device) == cudaSuccess && coop &&
+                      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)) == cudaSuccess &&
+                      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, kProjThreads, most) == cudaSuccess && resident > 0;
+    cudaGetLastError();
+    ok = fits ? 1 : -1;
+  }
+  if (ok < 0) return false;
+  // a CTA per SM, each with 16 rows (two tiles) at least
+  int64_t rows = (n + h->num_sms - 1) / h->num_sms;
+  rows = rows < 16 ? 16 : (rows + 7) / 8 * 8;
+  const int64_t ctas = (n + rows - 1) / rows;
+  const size_t len = static_cast<size_t>(nblk) * BB;
+  double* small = static_cast<double*>(small_scratch(h));
+  double* partial = small ? static_cast<double*>(workspace(h, sizeof(double) * ((ctas + 1) * len + ctas * BB))) : nullptr;
+  if (!partial) {
+    st = TRL_ENOMEM;
+    return true;
+  }
+  double* total = partial + ctas * len;
+  cudaLaunchAttribute attr[1] = {};
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+  cfg.blockDim = dim3(kProjThreads);
+  cfg.dynamicSmemBytes = smem(nblk * BB);
+  cfg.stream = h->stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ProfScope prof(h, PROF_UPDATE, (2.0 * nblk + 3.0) * n * BS * sizeof(T), 2.0 * (2.0 * nblk + 2.0) * n * BS * BS);
+  cudaLaunchKernelEx(&cfg, kern, V, nblk, W, n, rows, cond, before, eta2, G, partial, total, total + len, reinterpret_cast<unsigned*>(small + kSmallCounters) + 2, h->d_status);
+  st = after_launch(h, "project");
+  return true;
 }
 
 // One pass of k_cholqr over the block: GRAM factors the Gram matrix of X U_0 ... U_{nf-1}, otherwise
@@ -1704,6 +2012,7 @@ int trl_cuda_project_out_sketch(trl_cuda_handle h, int dtype, const void* V, int
     // to the profile because the host does not know whether they ran)
     {
       ProfScope prof(h, PROF_REORTH2, 0.0);
+      if (launch_project<T, BS>(h, Vt, nblk, Wt, n, flag1, Gw0, eta * eta, G, st)) return st;
       st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C1, flag1);
       if (!st) st = launch_update_gram<T, BS>(h, Vt, nblk, C1, Wt, n, flag1, FinishGram<BS>{G, Gw0, eta * eta, flag2});
       if (!st) st = launch_block_dot<T, BS>(h, Vt, nblk, Wt, n, C2, flag2);

@@ -65,7 +65,7 @@ inline bool valid_dtype(int dt) { return dt == TRL_F64 || dt == TRL_F32; }
 int after_launch(trl_cuda_context* h, const char* what);
 
 // Per-handle device scratch of fixed size, in doubles from its start: a Gram matrix, the factors of a
-// CholQR (up to 4), and ticket and work counters (zero between kernels); nullptr on failure.
+// CholQR (up to 4), and ticket and work counters (zero between kernels) and a grid barrier's state; nullptr on failure.
 constexpr int kSmallFactors = 256, kSmallTickets = kSmallFactors + 4 * 256, kSmallCounters = kSmallTickets + 256,
               kSmallDoubles = kSmallCounters + 8;
 void* small_scratch(trl_cuda_context* h);

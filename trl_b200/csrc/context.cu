@@ -243,6 +243,8 @@ int trl_cuda_synchronize(trl_cuda_handle h)
   const int flags = *st;
   if (flags & TRL_DEV_CHOLESKY) return set_error(h, TRL_ECHOLESKY, "Cholesky factorization failed in orthonormalize");
   if (flags & TRL_DEV_EIGEN) return set_error(h, TRL_EEIGEN, "Eigendecomposition failed");
+  if ((flags & TRL_DEV_TIMEOUT) && h->d_small) // a barrier that gave up may have left counts behind
+    cudaMemsetAsync(h->d_small + kSmallTickets, 0, (kSmallDoubles - kSmallTickets) * sizeof(double), h->stream);
   if (flags & TRL_DEV_TIMEOUT) return set_error(h, TRL_ETIMEOUT, "a bounded device wait timed out");
   return TRL_OK;
 }
