@@ -886,80 +886,84 @@ __global__ void __launch_bounds__(kThreads) k_update_gram(const T* in, int64_t i
 }
 
 // ---------------------------------------------------------------- Cholesky-QR
-// One warp: G = L L^T (reading the lower triangle), Ui = L^{-T}; L is left in shared memory. Lane i
-// owns row i of G, then column i of L^{-1}; chains of one square root or division per column.
+// Shared memory of the factorisation: [G | I] under elimination, L, and the pivots' square roots.
+template <int BS>
+struct FactorSpace {
+  double A[BS][2 * BS + 1];
+  double L[BS][BS + 1];
+  double root[BS];
+};
+
+// By the whole CTA: G = L L^T (reading the lower triangle), Ui = L^{-T}; L is left in f. Gaussian
+// elimination of [G | I] without pivoting (the pivots d are those of Cholesky, L = (unit lower factor)
+// D^{1/2}) gives the factor and its inverse in one chain of a division per column, a matrix entry or
+// two per thread; the square roots come at the end, all at once. Rolled loops: the code runs once
+// per CTA, and by one warp, unrolled, with a chain of its own for the inverse, it took 4,500 / 9,200
+// / 20,500 cycles for 4 / 8 / 16 columns, most of them waiting for instructions; now 2,500
+// / 4,100 / 9,200 (with a division per entry in place of the reciprocal: 2,600 / 4,400 / 10,800, and twice
+// that where the code is cold).
 // false (uniform): a pivot was <= 0 or NaN; Ui is then the identity, which leaves an apply a no-op.
 template <int BS>
-__device__ __forceinline__ bool warp_factor(const double* G, double (*L)[BS + 1], double* Ui)
+__device__ __forceinline__ bool cta_factor(const double* G, FactorSpace<BS>& f, double* Ui)
 {
-  const int lane = threadIdx.x & 31;
-  double row[BS];
+  constexpr int COLS = 2 * BS;
+  constexpr int PER = (BS * COLS + kThreads - 1) / kThreads; // entries per thread
+  for (int e = threadIdx.x; e < BS * BS; e += kThreads) {
+    const int r = e / BS, k = e % BS;
+    f.A[r][k] = k <= r ? G[e] : G[k * BS + r];
+    f.A[r][BS + k] = r == k ? 1.0 : 0.0;
+  }
   bool ok = true;
+  __syncthreads();
+#pragma unroll 1
+  for (int j = 0; j < BS; ++j) { // row j and column j are final: nobody writes them in this round
+    const double d = f.A[j][j];
+    ok = ok && d > 0.0;
+    const double piv = d > 0.0 ? d : 1.0, inv = 1.0 / piv;
 #pragma unroll
-  for (int j = 0; j < BS; ++j) row[j] = lane < BS ? G[lane * BS + j] : 0.0;
-#pragma unroll
-  for (int j = 0; j < BS; ++j) {
-    const double piv = __shfl_sync(0xffffffffu, row[j], j);
-    ok = ok && piv > 0.0;
-    const double l = piv > 0.0 ? sqrt(piv) : 1.0;
-    row[j] = lane == j ? l : (lane > j ? row[j] / l : 0.0);
-#pragma unroll
-    for (int k = j + 1; k < BS; ++k) {
-      const double lk = __shfl_sync(0xffffffffu, row[j], k);
-      row[k] = fma(-row[j], lk, row[k]);
+    for (int q = 0; q < PER; ++q) {
+      const int e = threadIdx.x + q * kThreads, i = e / COLS, k = e % COLS;
+      if (i > j && i < BS && k != j) {
+        const double a = f.A[i][j];
+        double m = a * inv;
+        m = fma(fma(-m, piv, a), inv, m); // a / piv with its remainder added back
+        f.A[i][k] = fma(-m, f.A[j][k], f.A[i][k]);
+      }
+      if (k == j && i < BS) f.L[i][j] = i < j ? 0.0 : (i == j ? piv : f.A[i][j]);
     }
+    __syncthreads();
   }
-  if (lane < BS) {
-#pragma unroll
-    for (int j = 0; j < BS; ++j) L[lane][j] = row[j];
+  if (threadIdx.x < BS) f.root[threadIdx.x] = sqrt(f.L[threadIdx.x][threadIdx.x]); // the pivots
+  __syncthreads();
+  for (int e = threadIdx.x; e < BS * BS; e += kThreads) {
+    const int r = e / BS, k = e % BS; // row r, column k of L, and of L^{-1}
+    f.L[r][k] = r == k ? f.root[k] : f.L[r][k] / f.root[k];
+    Ui[k * BS + r] = ok ? (k <= r ? f.A[r][BS + k] / f.root[r] : 0.0) : (r == k ? 1.0 : 0.0);
   }
-  __syncwarp();
-  if (lane < BS) {
-    double x[BS]; // column `lane` of the identity, then of L^{-1}
-#pragma unroll
-    for (int i = 0; i < BS; ++i) x[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-    for (int i = 0; i < BS; ++i) {
-      x[i] = x[i] / L[i][i];
-#pragma unroll
-      for (int m = i + 1; m < BS; ++m) x[m] = fma(-L[m][i], x[i], x[m]);
-    }
-#pragma unroll
-    for (int c = 0; c < BS; ++c) Ui[lane * BS + c] = ok ? x[c] : (c == lane ? 1.0 : 0.0);
-  }
-  __syncwarp();
+  __syncthreads();
   return ok;
 }
 
-// The factor's outputs, by the same warp: Ui to global memory, and R <- L^T (first pass) or
+// The factor's outputs, by the same CTA: Ui to global memory, and R <- L^T (first pass) or
 // R <- L^T R (X_in = X_out R across passes). A breakdown leaves R and records TRL_DEV_CHOLESKY.
 template <int BS>
-__device__ __forceinline__ void warp_factor_store(bool ok, const double (*L)[BS + 1], const double* Ui, double* Uout, double* R, bool first, int* status)
+__device__ __forceinline__ void cta_factor_store(bool ok, FactorSpace<BS>& f, const double* Ui, double* Uout, double* R, bool first, int* status)
 {
-  const int lane = threadIdx.x & 31;
-  for (int e = lane; e < BS * BS; e += 32) Uout[e] = Ui[e];
+  for (int e = threadIdx.x; e < BS * BS; e += kThreads) {
+    Uout[e] = Ui[e];
+    f.A[e / BS][e % BS] = first ? 0.0 : __ldcg(R + e); // R before (L2: another CTA may have written it)
+  }
   if (!ok) {
-    if (lane == 0) atomicOr(status, TRL_DEV_CHOLESKY);
+    if (threadIdx.x == 0) atomicOr(status, TRL_DEV_CHOLESKY);
     return;
   }
-  double r[BS]; // column `lane` of R before
-  if (lane < BS && !first) {
-#pragma unroll
-    for (int k = 0; k < BS; ++k) r[k] = __ldcg(R + k * BS + lane); // L2: another CTA may have written it
-  }
-  __syncwarp();
-  if (lane < BS) {
-#pragma unroll
-    for (int i = 0; i < BS; ++i) { // entry (i, lane)
-      double v = 0.0;
-      if (first) v = L[lane][i]; // zero above the diagonal of L: R is upper triangular
-      else {
-#pragma unroll
-        for (int k = i; k < BS; ++k)
-          if (k <= lane) v = fma(L[k][i], r[k], v);
-      }
-      R[i * BS + lane] = i <= lane ? v : 0.0;
-    }
+  __syncthreads();
+  for (int e = threadIdx.x; e < BS * BS; e += kThreads) {
+    const int i = e / BS, c = e % BS;
+    double v = first && i <= c ? f.L[c][i] : 0.0;
+    if (!first)
+      for (int k = i; k <= c; ++k) v = fma(f.L[k][i], f.A[k][c], v);
+    R[e] = v;
   }
 }
 
@@ -1033,7 +1037,7 @@ constexpr int kCholMaxPasses = 4;
 // place of a launch); CTA 0 keeps the outputs.
 // GRAM: forms the Gram matrix of the result, and the last CTA factors it into U_nf. Otherwise the
 // result is stored in place, and CholQR2 has read the block twice and written it once.
-// Measured on B200, CholQR2 of 884,736 x 8 FP64 / 100,003 x 16 FP32: 40 / 45 us (before, with a
+// Measured on B200, CholQR2 of 884,736 x 8 FP64 / 100,003 x 16 FP32: 34 / 33 us (before, with a
 // launch per factor and the block stored between the passes: 57 / 61 us).
 template <typename T, int BS, int RT, bool GRAM>
 __global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const double* __restrict__ G0, int nf, double* U, double* R, int* status, double* __restrict__ partial,
@@ -1044,7 +1048,7 @@ __global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const doub
   constexpr int NT = Tile::NT;
   constexpr int BB = BS * BS;
   __shared__ double Us[kCholMaxPasses][BB];
-  __shared__ double Ls[BS][BS + 1];
+  __shared__ FactorSpace<BS> fs;
   __shared__ double stage[GRAM ? kWarps : 1][GRAM ? RT * 8 * BS : 1];
   __shared__ double red[GRAM ? kWarps : 1][GRAM ? NT * NT * 64 : BB];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1053,10 +1057,8 @@ __global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const doub
     double* Gs = &red[0][0];
     for (int e = threadIdx.x; e < BB; e += kThreads) Gs[e] = G0[e];
     __syncthreads();
-    if (warp == 0) {
-      const bool ok = warp_factor<BS>(Gs, Ls, Us[0]);
-      if (blockIdx.x == 0) warp_factor_store<BS>(ok, Ls, Us[0], U, R, true, status);
-    }
+    const bool ok = cta_factor<BS>(Gs, fs, Us[0]);
+    if (blockIdx.x == 0) cta_factor_store<BS>(ok, fs, Us[0], U, R, true, status);
   }
   else
     for (int e = threadIdx.x; e < nf * BB; e += kThreads) Us[e / BB][e % BB] = U[e];
@@ -1159,9 +1161,9 @@ __global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const doub
     }
     __syncthreads();
     double* sum = &red[0][0];
-    if (last_cta_sum<BB>(partial, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), tickets, sum, sum + BB) && warp == 0) {
-      const bool ok = warp_factor<BS>(sum, Ls, Us[0]);
-      warp_factor_store<BS>(ok, Ls, Us[0], U + nf * BB, R, false, status);
+    if (last_cta_sum<BB>(partial, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), tickets, sum, sum + BB)) {
+      const bool ok = cta_factor<BS>(sum, fs, Us[0]);
+      cta_factor_store<BS>(ok, fs, Us[0], U + nf * BB, R, false, status);
     }
   }
 }
