@@ -111,3 +111,29 @@ def test_projections_at_the_edges_of_one_launch(cuda_handle, bs, dtype, n, nblk)
             close(host(Wd), out, np.abs(w).max(), eps)
             close(host(G), host(Wd).T @ host(Wd), max(np.abs(host(G)).max(), 1e-300), 1e-10)
     cuda_handle.sync()
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("n", [1, 15, 17, 48, 63, 65, 113, 127, 129, 3584, 3585, 3601, 20011])
+@pytest.mark.parametrize("nblk", [1, 2, 4, 5, 9])
+def test_wide_blocks_at_tile_edges(cuda_handle, dtype, n, nblk):
+    # 16 columns: tiles of 64 (FP64) and 128 (FP32) rows in pieces of 16, updates of 8 and 24 rows per warp
+    bs = 16
+    rng = np.random.default_rng(n + nblk)
+    V, W = (as_dt(rng.standard_normal(s) / np.sqrt(n), dtype) for s in ((nblk, n, bs), (n, bs)))
+    # n rows of a larger block, NaN behind them
+    Vd, Wd = (torch.full((m, bs), float("nan"), dtype=dtype, device="cuda") for m in (nblk * n + 8, n + 8))
+    Vd[: nblk * n].copy_(dev(V, dtype).view(-1, bs))
+    Wd[:n].copy_(dev(W, dtype))
+    Vd, Wd = Vd[: nblk * n].view(nblk, n, bs), Wd[:n]
+    C = torch.full((nblk, bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+    cuda_handle.block_dot(Vd, Wd, C)
+    ref = np.einsum("jnb,nc->jbc", V, W)
+    close(host(C), ref, np.einsum("jnb,nc->jbc", np.abs(V), np.abs(W)).max())
+    G = torch.full((bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+    cuda_handle.project_out(Vd, Wd, native.TRL_CGS_ONE, G)
+    out = W - np.einsum("jnb,jbc->nc", V, ref)
+    size = np.abs(W).max() + np.einsum("jnb,jbc->nc", np.abs(V), np.abs(ref)).max()
+    got = host(Wd)
+    assert np.abs(got - out).max() <= (1e-12 if dtype == torch.float64 else 1.2e-7) * size
+    close(host(G), got.T @ got, (np.abs(got).T @ np.abs(got)).max())

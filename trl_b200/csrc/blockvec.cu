@@ -335,17 +335,24 @@ __global__ void __launch_bounds__(kThreads) k_block_dot(const T* __restrict__ V,
 
 // ---------------------------------------------------------------- block dot, bulk-copy pipeline
 // Same result as k_block_dot, for BS*sizeof(T) a multiple of 16 bytes. The CTA walks its
-// row range in tiles of R rows (4 KB per block tile). Thread 0 streams the W tile and the
+// row range in tiles of R rows (2 to 8 KB per block tile). Thread 0 streams the W tile and the
 // tiles of the JC blocks of V into an S-stage shared-memory ring with 1-D bulk copies that
 // complete on a per-stage "full" mbarrier; the 8 warps read DMMA fragments from shared
 // memory and release the stage on its "empty" mbarrier. HBM traffic is a continuous stream
-// of 4 KB copies, independent of register pressure and of the element width.
+// of copies, independent of register pressure and of the element width.
 // Waits are bounded (mbar_wait): on a timeout the status word records TRL_DEV_TIMEOUT, the
 // threads leave the tile loop, and thread 0 waits (bounded) for the copies it issued.
 template <typename T, int BS, int TB>
 struct BulkTile {
   static constexpr int R = TB / (BS * static_cast<int>(sizeof(T))); // rows per tile (TB bytes per block tile)
-  static constexpr int ELEMS = R * BS;
+  // Rows of 128 bytes: the four rows of a fragment load would share their shared-memory banks (4-way
+  // conflicts, a wavefront per cycle at the DMMA's full rate). They are taken from SUB pieces of the tile
+  // instead, which lie 32 bytes apart modulo 128 (B200, 300,001 x 16 FP64, 12 blocks: 110 -> 90 us; the
+  // bytes take 76).
+  static constexpr int SUB = BS * sizeof(T) >= 128 ? 4 : 1;
+  static constexpr int SROWS = R / SUB; // rows per piece
+  static constexpr int PIECE = SROWS * BS + (SUB > 1 ? 32 / static_cast<int>(sizeof(T)) : 0);
+  static constexpr int ELEMS = SUB * PIECE;
 };
 
 template <typename T, int BS, int JC, int S, int TB>
@@ -358,6 +365,7 @@ __global__ void __launch_bounds__(kThreads) k_block_dot_bulk(const T* __restrict
   constexpr int BB = BS * BS;
   constexpr int R = BulkTile<T, BS, TB>::R;
   constexpr int TILE = BulkTile<T, BS, TB>::ELEMS;
+  constexpr int SUB = BulkTile<T, BS, TB>::SUB, SROWS = BulkTile<T, BS, TB>::SROWS, PIECE = BulkTile<T, BS, TB>::PIECE;
   constexpr int GPW = R / (kWarps * 4); // 4-row groups per warp per tile
   static_assert(GPW >= 1 && R % (kWarps * 4) == 0, "tile rows must cover the CTA's warps");
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -383,18 +391,32 @@ __global__ void __launch_bounds__(kThreads) k_block_dot_bulk(const T* __restrict
   }
   __syncthreads();
 
-  int issued = 0; // thread 0: tiles whose copies were started
+  // one thread starts a tile's copies; with SUB pieces per block it is a warp (100,003 x 16 FP64, 20 blocks:
+  // 53 us, by one thread 61)
+  const bool issuer = SUB > 1 ? warp == 0 : threadIdx.x == 0;
+  int issued = 0; // by the issuer: tiles whose copies were started
   auto issue = [&](int t) {
     const int s = t % S;
     const int64_t r0 = rb + static_cast<int64_t>(t) * R;
-    const uint32_t bytes = static_cast<uint32_t>(min(static_cast<int64_t>(R), re - r0) * BS * sizeof(T));
+    const int rows = static_cast<int>(min(static_cast<int64_t>(R), re - r0));
+    const uint32_t bytes = static_cast<uint32_t>(rows * BS * sizeof(T));
     T* st = tiles + static_cast<size_t>(s) * (JC + 1) * TILE;
-    mbar_arrive_expect_tx(&full[s], bytes * static_cast<uint32_t>(jn + 1));
-    bulk_g2s(st, W + r0 * BS, bytes, &full[s]);
-    for (int jj = 0; jj < jn; ++jj) bulk_g2s(st + (jj + 1) * TILE, V + static_cast<int64_t>(j0 + jj) * vstride + r0 * BS, bytes, &full[s]);
+    if (threadIdx.x == 0) mbar_arrive_expect_tx(&full[s], bytes * static_cast<uint32_t>(jn + 1));
+    if constexpr (SUB == 1) {
+      bulk_g2s(st, W + r0 * BS, bytes, &full[s]);
+      for (int jj = 0; jj < jn; ++jj) bulk_g2s(st + (jj + 1) * TILE, V + static_cast<int64_t>(j0 + jj) * vstride + r0 * BS, bytes, &full[s]);
+    }
+    else {
+      __syncwarp();
+      for (int e = lane; e < (jn + 1) * SUB; e += 32) {
+        const int jj = e / SUB - 1, first = e % SUB * SROWS;
+        const T* from = jj < 0 ? W : V + static_cast<int64_t>(j0 + jj) * vstride;
+        if (first < rows) bulk_g2s(st + (jj + 1) * TILE + e % SUB * PIECE, from + (r0 + first) * BS, static_cast<uint32_t>(min(SROWS, rows - first) * BS * sizeof(T)), &full[s]);
+      }
+    }
     issued = t + 1;
   };
-  if (threadIdx.x == 0)
+  if (issuer)
     for (int t = 0; t < min(S - 1, ntiles); ++t) issue(t);
 
   double acc[JC][NT][NT][2];
@@ -407,9 +429,11 @@ __global__ void __launch_bounds__(kThreads) k_block_dot_bulk(const T* __restrict
 
   int consumed = 0;
   for (int t = 0; t < ntiles; ++t) {
-    if (threadIdx.x == 0 && t + S - 1 < ntiles) {
+    if (issuer && t + S - 1 < ntiles) {
       const int tn = t + S - 1; // refill the slot that tile t-1 used
-      if (tn < S || mbar_wait(&empty[tn % S], static_cast<uint32_t>((tn - S) / S) & 1u, status)) issue(tn);
+      bool vacant = tn < S || mbar_wait(&empty[tn % S], static_cast<uint32_t>((tn - S) / S) & 1u, status);
+      if constexpr (SUB > 1) vacant = __all_sync(0xffffffffu, vacant);
+      if (vacant) issue(tn);
     }
     const int s = t % S;
     if (!mbar_wait(&full[s], static_cast<uint32_t>(t / S) & 1u, status)) break;
@@ -417,13 +441,14 @@ __global__ void __launch_bounds__(kThreads) k_block_dot_bulk(const T* __restrict
     const int rows = static_cast<int>(min(static_cast<int64_t>(R), re - (rb + static_cast<int64_t>(t) * R)));
 #pragma unroll
     for (int q = 0; q < GPW; ++q) {
-      const int lr = (warp * GPW + q) * 4 + t4;
+      const int lr = SUB > 1 ? t4 * SROWS + warp * GPW + q : (warp * GPW + q) * 4 + t4;
+      const int at = SUB > 1 ? t4 * PIECE + (warp * GPW + q) * BS : lr * BS;
       const bool rok = lr < rows;
       double bf[NT];
 #pragma unroll
       for (int tk = 0; tk < NT; ++tk) {
         const int col = tk * 8 + g;
-        bf[tk] = (rok && col < BS) ? static_cast<double>(st[lr * BS + col]) : 0.0;
+        bf[tk] = (rok && col < BS) ? static_cast<double>(st[at + col]) : 0.0;
       }
 #pragma unroll
       for (int jj = 0; jj < JC; ++jj) {
@@ -431,7 +456,7 @@ __global__ void __launch_bounds__(kThreads) k_block_dot_bulk(const T* __restrict
 #pragma unroll
           for (int ti = 0; ti < NT; ++ti) {
             const int col = ti * 8 + g;
-            const double a = (rok && col < BS) ? static_cast<double>(st[(jj + 1) * TILE + lr * BS + col]) : 0.0;
+            const double a = (rok && col < BS) ? static_cast<double>(st[(jj + 1) * TILE + at + col]) : 0.0;
 #pragma unroll
             for (int tk = 0; tk < NT; ++tk) dmma_m8n8k4(acc[jj][ti][tk][0], acc[jj][ti][tk][1], a, bf[tk]);
           }
@@ -758,7 +783,7 @@ __device__ __forceinline__ void load_cols(const T* p, T (&v)[KS])
 // gram_partial[blockIdx.x][BS*BS], added up by the last CTA. When cond is given and *cond == 0
 // the kernel does nothing (a device-side decision: no host round trip).
 template <typename T, int BS, int RT, int U, class Fin>
-__global__ void __launch_bounds__(kThreads) k_update_gram(const T* in, int64_t istride, int MB, const double* __restrict__ coef, T* out, int64_t n,
+__global__ void __launch_bounds__(kThreads, BS == 16 ? 2 : 0) k_update_gram(const T* in, int64_t istride, int MB, const double* __restrict__ coef, T* out, int64_t n,
                                                           int accumulate, double sign, double* __restrict__ gram_partial, const int* __restrict__ cond, Tickets tickets, Fin fin)
 {
   ::trl_detail::pdl_enter();
@@ -1506,7 +1531,8 @@ int launch_block_dot_bulk(trl_cuda_context* h, const T* V, int nblk, const T* W,
   const int gj = (nblk + JC - 1) / JC;
   int64_t chunks = static_cast<int64_t>(h->num_sms) * resident / gj;
   if (chunks < 1) chunks = 1;
-  const int64_t max_chunks = (n + 2 * R - 1) / (2 * R); // at least two tiles per CTA
+  constexpr int kLeast = TB > 4096 ? 1 : 2; // tiles per CTA at least
+  const int64_t max_chunks = (n + kLeast * R - 1) / (kLeast * R);
   if (chunks > max_chunks) chunks = max_chunks;
   int64_t rows_per_cta = (n + chunks - 1) / chunks;
   rows_per_cta = (rows_per_cta + R - 1) / R * R;
@@ -1548,31 +1574,37 @@ int launch_block_dot(trl_cuda_context* h, const T* V, int nblk, const T* W, int6
     return launch_block_dot_jc<T, BS, 1, G1>(h, V, nblk, W, n, C, cond);
   }
   if constexpr ((BS * sizeof(T)) % 16 == 0) {
-    constexpr int TBS = (BS * sizeof(T) <= 64) ? 2048 : 4096; // small tiles where 32 rows fit
-    constexpr int JCL = BS >= 16 ? 4 : 8;
-    if (nblk == 1) return launch_block_dot_bulk<T, BS, 1, 8, 4096>(h, V, nblk, W, n, C, cond);
-    if (nblk == 2) return launch_block_dot_bulk<T, BS, 2, 6, 4096>(h, V, nblk, W, n, C, cond);
-    if (nblk <= 4) return launch_block_dot_bulk<T, BS, 4, 4, 4096>(h, V, nblk, W, n, C, cond);
-    if constexpr (sizeof(T) == 8) return launch_block_dot_bulk<T, BS, JCL, 3, TBS>(h, V, nblk, W, n, C, cond);
-    if (nblk <= 8) return launch_block_dot_bulk<T, BS, JCL, 3, 4096>(h, V, nblk, W, n, C, cond);
-    return launch_block_dot_bulk<T, BS, 4, 3, TBS>(h, V, nblk, W, n, C, cond);
+    if constexpr (BS == 16) {
+      // 8 KB tiles, stages for the same shared memory: a copy's start costs its thread as much as 4 KB
+      // of data (B200, 300,001 rows, 4 KB -> 8 KB tiles: 1 block FP64 22 -> 17 us, FP32 14 -> 13; 4 blocks 54 -> 40,
+      // 45 -> 29; 8 blocks FP32 53 -> 48; 24 blocks FP32, from 2 KB, 162 -> 127)
+      if (nblk == 1) return launch_block_dot_bulk<T, BS, 1, 4, 8192>(h, V, nblk, W, n, C, cond);
+      if (nblk == 2) return launch_block_dot_bulk<T, BS, 2, 3, 8192>(h, V, nblk, W, n, C, cond);
+      return launch_block_dot_bulk<T, BS, 4, 2, 8192>(h, V, nblk, W, n, C, cond);
+    }
+    else {
+      if (nblk == 1) return launch_block_dot_bulk<T, BS, 1, 8, 4096>(h, V, nblk, W, n, C, cond);
+      if (nblk == 2) return launch_block_dot_bulk<T, BS, 2, 6, 4096>(h, V, nblk, W, n, C, cond);
+      if (nblk <= 4) return launch_block_dot_bulk<T, BS, 4, 4, 4096>(h, V, nblk, W, n, C, cond);
+      if constexpr (sizeof(T) == 8) return launch_block_dot_bulk<T, BS, 8, 3, 2048>(h, V, nblk, W, n, C, cond);
+      if (nblk <= 8) return launch_block_dot_bulk<T, BS, 8, 3, 4096>(h, V, nblk, W, n, C, cond);
+      return launch_block_dot_bulk<T, BS, 4, 3, 4096>(h, V, nblk, W, n, C, cond);
+    }
   }
   if (nblk == 1) return launch_block_dot_jc<T, BS, 1, 8>(h, V, nblk, W, n, C, cond);
   if (nblk == 2) return launch_block_dot_jc<T, BS, 2, 4>(h, V, nblk, W, n, C, cond);
-  if (nblk <= 4) return launch_block_dot_jc<T, BS, 4, (BS >= 16 ? 2 : 4)>(h, V, nblk, W, n, C, cond);
-  return launch_block_dot_jc<T, BS, (BS >= 16 ? 4 : 8), 2>(h, V, nblk, W, n, C, cond);
+  if (nblk <= 4) return launch_block_dot_jc<T, BS, 4, 4>(h, V, nblk, W, n, C, cond);
+  return launch_block_dot_jc<T, BS, 8, 2>(h, V, nblk, W, n, C, cond);
 }
 
 // out -= V C over MB blocks and the Gram matrix of the result, which fin gets
-template <typename T, int BS, class Fin>
-int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* coef, T* out, int64_t n, const int* cond, const Fin& fin)
+template <typename T, int BS, int RT, class Fin>
+int launch_update_gram_rt(trl_cuda_context* h, const T* in, int MB, const double* coef, T* out, int64_t n, const int* cond, const Fin& fin)
 {
-  constexpr int NT = (BS + 7) / 8;
   // Measured on B200 (24 blocks of 884,736 x 8, GB/s of algorithmic bytes; copy peak
   // 6,539): one input block per loop iteration (U = 1) beats explicit multi-block register
   // prefetch (U = 4: FP64 6,075, FP32 3,860), and 8-row tiles per warp RT = 4 (FP64, 6,784)
   // and RT = 2 (FP32, 5,439) with two resident waves of CTAs do best.
-  constexpr int RT = NT >= 2 ? 1 : (sizeof(T) == 8 ? 4 : 2);
   static int resident = 0;
   if (resident == 0) {
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_update_gram<T, BS, RT, 1, Fin>, kThreads, 0) != cudaSuccess || resident < 1) resident = 4;
@@ -1584,6 +1616,26 @@ int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* c
   if (!partial) return TRL_ENOMEM;
   launch(k_update_gram<T, BS, RT, 1, Fin>, grid, kThreads, 0, h->stream, in, n * BS, MB, coef, out, n, 1, -1.0, partial, cond, t, fin);
   return after_launch(h, "update_gram");
+}
+
+// 16 columns: two tiles of columns take each coefficient load to 2 RT products, and with RT = 1 the loads
+// bound the kernel. With 24 rows per warp and registers for two CTAs per SM (RT = 1 -> 3, one projection less
+// its dot): 300,001 rows, 24 blocks FP32 285 -> 166 us (the products take 103), 12 blocks FP64 196 -> 156 (the
+// bytes 82); 20,000 rows, 30 blocks 44 -> 37 and 51 -> 41. Up to kFewRows rows single tiles give
+// more warps (RT = 1 / 3, FP32 and FP64: 1,500 rows 13.9 / 16.5 and 20.2 / 23.5 us, 3,500 22.3 / 25.9 and
+// 23.8 / 27.0; 4,096 33.7 / 30.8 and 36.7 / 31.8).
+constexpr int64_t kFewRows = 3584;
+
+template <typename T, int BS, class Fin>
+int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* coef, T* out, int64_t n, const int* cond, const Fin& fin)
+{
+  if constexpr (BS == 16) {
+    if (n <= kFewRows) return launch_update_gram_rt<T, BS, 1>(h, in, MB, coef, out, n, cond, fin);
+    return launch_update_gram_rt<T, BS, 3>(h, in, MB, coef, out, n, cond, fin);
+  }
+  else {
+    return launch_update_gram_rt<T, BS, (sizeof(T) == 8 ? 4 : 2)>(h, in, MB, coef, out, n, cond, fin);
+  }
 }
 
 // The projection in one launch for small bases: true if it ran (st: its status), false if the separate
