@@ -87,3 +87,13 @@ def test_counts_at_exact_zeros(cuda_handle, N):
                  (10.0 ** -(i % 20), 10.0 ** -(i[:-1] % 17)), (np.zeros(N), 1e-25 * np.ones(N - 1) + (i[:-1] == 0))):
         D = np.diag(d) + np.diag(e, 1) + np.diag(e, -1)
         _check(cuda_handle, D, 0 if N > 100 else 1)
+
+
+@pytest.mark.parametrize("N", [33, 34, 35, 49, 67, 130])
+@pytest.mark.parametrize("coupling", [1e-6, 1e-14, 1e-16, 1e-40])
+def test_products_that_shrink_between_looks(cuda_handle, N, coupling):
+    """Runs of equal diagonal entries and minute couplings: near them every row shrinks the products;
+    each half ends in a different number of rows after the last group of eight."""
+    d = np.where(np.arange(N) < N // 3, 1.0, 0.25 * (np.arange(N) % 2))
+    D = np.diag(d) + np.diag(np.full(N - 1, coupling), 1) + np.diag(np.full(N - 1, coupling), -1)
+    _check(cuda_handle, D, 0)
