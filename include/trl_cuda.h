@@ -214,7 +214,8 @@ int trl_cuda_project_out_sketch(trl_cuda_handle h, int dtype, const void* V, int
 
 /* trl_cuda_cholqr with the Gram matrix of the first pass supplied (G0 = X^T X on the device,
  * e.g. from trl_cuda_project_out); each further pass forms its Gram matrix while it applies
- * U^{-1}, so CholQR2 reads and writes X twice. G0 == NULL is trl_cuda_cholqr. */
+ * U^{-1}, and only the last stores, so CholQR2 reads X twice and writes it once. G0 == NULL is
+ * trl_cuda_cholqr. */
 int trl_cuda_cholqr_gram(trl_cuda_handle h, int dtype, void* X, int64_t n, int bs, int passes, double* R, const double* G0);
 
 /* Thick-restart rotation W_j = sum_{i<m} V_i Y(i,j) for j < k, in one pass over V.
@@ -314,7 +315,7 @@ int trl_cuda_mb_set_diagonal(trl_cuda_handle h, double* dst, const double* host_
  * columns kvec.. of evecs are zero; evals, host_evals and *host_nconv (over the first
  * min(nev, kvec) pairs) as above. The driver reads only the kept kr = nev/bs + 1 blocks of
  * eigenvectors (lanczos.hh:105-131), so EVPBase::solve_small_dense asks for kr*bs. For
- * 3 <= N <= 448 and kvec <= 128 it runs on hand-written kernels: Householder
+ * 3 <= N <= 1024 and kvec <= 256 it runs on hand-written kernels: Householder
  * tridiagonalisation in one thread-block cluster, bisection, inverse iteration, and the
  * back-transform; otherwise it uses trl_cuda_small_eigen. Synchronises the stream. */
 int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, int nblk, int bs, const double* beta, int nev, double tol, int kvec, double* evals,

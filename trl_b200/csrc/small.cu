@@ -953,8 +953,8 @@ __device__ __forceinline__ int sturm_count(const double2* up, const double2* dow
 // latency of the recurrence: N / 2 rows x 9 rounds.
 // Measured on B200: N = 384 94 us, N = 512 123 us (before, on pivots from one end, one warp and 32
 // points per eigenvalue, and the Gershgorin bounds summed by one thread: 427 and 568 us); with signs
-// shifted into a word and the range looked at every eight rows instead of four, the whole call
-// 844 -> 818 and 1,359 -> 1,324 us.
+// shifted into a word and the range looked at every eight rows instead of four N = 384 72 us, and the
+// whole call 844 -> 818 and, N = 512, 1,359 -> 1,324 us.
 constexpr int kBisectPoints = 64;
 
 __global__ void __launch_bounds__(kBisectPoints) k_bisect(const double* __restrict__ dg, const double* __restrict__ eg, int N, double* __restrict__ w)
