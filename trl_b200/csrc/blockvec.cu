@@ -436,7 +436,9 @@ __global__ void __launch_bounds__(kThreads) k_block_dot_bulk(const T* __restrict
       if (vacant) issue(tn);
     }
     const int s = t % S;
-    if (!mbar_wait(&full[s], static_cast<uint32_t>(t / S) & 1u, status)) break;
+    bool there = mbar_wait(&full[s], static_cast<uint32_t>(t / S) & 1u, status);
+    if constexpr (SUB > 1) there = __all_sync(0xffffffffu, there); // the whole warp leaves or none of it: it issues together
+    if (!there) break;
     const T* st = tiles + static_cast<size_t>(s) * (JC + 1) * TILE;
     const int rows = static_cast<int>(min(static_cast<int64_t>(R), re - (rb + static_cast<int64_t>(t) * R)));
 #pragma unroll
