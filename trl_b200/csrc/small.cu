@@ -7,6 +7,7 @@
 // and the Ritz estimates ||beta * y_last|| / max(|theta|, eps) (evp_base.hh:124-151) are
 // counted on the device. Only the eigenvalues and the converged count come back to the host.
 #include "common.cuh"
+#include "tridiag_schedule.h"
 
 #include <cooperative_groups.h>
 #include <cusolverDn.h>
@@ -444,7 +445,8 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // barrier over the CTA or the cluster:
 //  - step s starts with each warp sending {t_g, a_gs} of its rows g >= s to every CTA, t = A u_{s-1}
 //    and a_gs the row's entry in column s before the update of step s - 1, as one 16-byte
-//    asynchronous store that counts on the receiver's mbarrier;
+//    asynchronous store that counts on the receiver's mbarrier (every CTA that still has a row
+//    beyond s and so waits for the step: tri_sends);
 //  - with all pairs there, every warp of every CTA forms w = tau t - K u, column s after the
 //    rank-2 update (x = a - u w_s - w u_s), and u_s from x. They compute from the same operands in
 //    the same order, so all hold the same bits, and the column's norm needs no second exchange;
@@ -461,7 +463,6 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // sums over all CTAs' partials): 1,719, 2,604, 480. At N = 384 a step is about 2,300 cycles:
 // sending and waiting 660, reading the pairs and the first sum 440, rows and columns 750, the
 // second sum and the norm 410.
-constexpr int kTriC = 16;
 constexpr int kTriW = 8;
 constexpr int kTriStride = kTriC * kTriW; // rows of one warp are this far apart
 
@@ -495,7 +496,7 @@ __device__ __forceinline__ bool tri_steps(TriState<RPW>& st, const TriArgs& k)
 #pragma unroll
       for (int i = F; i < RPW; ++i) {
         const int g = k.g0 + i * kTriStride;
-        if (g >= s && g < N && lane < kTriC)
+        if (tri_sends(N, g, lane, s))
           st_async_pair(k.to_pairs + static_cast<uint32_t>((cur * N + g) * 16), st.t[i], st.col[i], k.to_bar + static_cast<uint32_t>(cur * 8));
       }
     }
@@ -647,8 +648,7 @@ __global__ void __launch_bounds__(kTriW * 32, 1)
   k.ld = ld;
   k.g0 = r + kTriC * warp;
   k.glast = k.g0 < N ? k.g0 + (N - 1 - k.g0) / kTriStride * kTriStride : -1;
-  const int cta_rows = r < N ? (N - 1 - r) / kTriC + 1 : 0;
-  k.keeper = cta_rows > 0 && warp == (cta_rows - 1) % kTriW;
+  k.keeper = k.glast >= 0 && k.glast == tri_last_row(N, r);
   // lane q < 16 sends to CTA q
   k.to_pairs = cluster_addr(smem_addr(sm), lane < kTriC ? lane : 0);
   k.to_bar = cluster_addr(smem_addr(&bars[0]), lane < kTriC ? lane : 0);
@@ -674,7 +674,9 @@ __global__ void __launch_bounds__(kTriW * 32, 1)
   st.s = 0;
   cluster.sync(); // every CTA's barriers exist before any store counts on them
   if (k.glast >= 0) tri_phases<RPW, 0>(st, k);
-  cluster.sync(); // no CTA leaves while another may still store into its shared memory
+  // Every store sent to a CTA is one its keeper waits for, so none is under way when the keepers are
+  // here; the barrier keeps the shared memory of the CTAs in place until then.
+  cluster.sync();
 }
 
 // The same reduction for matrices whose rows do not fit the cluster's registers, or where a
@@ -846,7 +848,7 @@ __global__ void __launch_bounds__(kTriThreads, 1)
     }
     __syncthreads();
   }
-  cluster.sync(); // no CTA leaves while another may still store into its shared memory
+  cluster.sync(); // every CTA waited for every step's stores; its shared memory stays until all have sent
 }
 
 // ---- eigenvalues of the tridiagonal by bisection on Sturm counts
