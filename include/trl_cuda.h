@@ -214,8 +214,8 @@ int trl_cuda_project_out_sketch(trl_cuda_handle h, int dtype, const void* V, int
 
 /* trl_cuda_cholqr with the Gram matrix of the first pass supplied (G0 = X^T X on the device,
  * e.g. from trl_cuda_project_out); each further pass forms its Gram matrix while it applies
- * U^{-1}, and only the last stores, so CholQR2 reads X twice and writes it once. G0 == NULL is
- * trl_cuda_cholqr. */
+ * U^{-1}, and only the last stores, so CholQR2 reads X twice and writes it once. R may be G0
+ * (the factor takes the Gram matrix's place). G0 == NULL is trl_cuda_cholqr. */
 int trl_cuda_cholqr_gram(trl_cuda_handle h, int dtype, void* X, int64_t n, int bs, int passes, double* R, const double* G0);
 
 /* Thick-restart rotation W_j = sum_{i<m} V_i Y(i,j) for j < k, in one pass over V.

@@ -56,6 +56,27 @@ def test_cholqr_passes(cuda_handle, bs, dtype, passes, n, offset):
 
 
 @pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("passes", [1, 2, 3, 4])
+def test_cholqr_factor_in_place_of_its_gram_matrix(cuda_handle, bs, dtype, passes):
+    n = 300001  # more CTAs than are resident at once
+    X = as_dt(np.random.default_rng(bs).standard_normal((n, bs)), dtype)
+    Xd, Yd = dev(X, dtype), dev(X, dtype)
+    G0 = torch.empty((1, bs, bs), dtype=torch.float64, device="cuda")
+    cuda_handle.block_dot(Xd[None], Xd, G0)
+    R = torch.empty_like(G0)
+    cuda_handle.cholqr_gram(Xd, passes, R, G0)
+    for shift in {0, bs * bs - 1}:  # R over all of G0, and over its last entry alone
+        Z = Yd.clone()
+        both = torch.zeros(2 * bs * bs, dtype=torch.float64, device="cuda")
+        both[: bs * bs] = G0.view(-1)
+        cuda_handle.cholqr_gram(Z, passes, both[shift:], both)
+        cuda_handle.sync()
+        assert torch.equal(Z, Xd)
+        assert torch.equal(both[shift : shift + bs * bs].view_as(R), R)
+
+
+@pytest.mark.parametrize("bs", BS)
 @pytest.mark.parametrize("passes", [1, 2])
 def test_cholqr_breakdown_leaves_block_and_factor(cuda_handle, bs, passes):
     X = torch.randn((1000, bs), dtype=torch.float64, device="cuda")

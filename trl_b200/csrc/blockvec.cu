@@ -1978,6 +1978,14 @@ int trl_cuda_cholqr_gram(trl_cuda_handle h, int dtype, void* X, int64_t n, int b
   double* small = static_cast<double*>(small_scratch(h));
   if (!small) return TRL_ENOMEM;
   double* U = small + kSmallFactors;
+  // R over G0 (the factor in place of its Gram matrix): every CTA of the first launch reads G0 while CTA 0
+  // writes R, so they read a copy
+  const size_t block = sizeof(double) * bs * bs;
+  const auto at = [](const double* p) { return reinterpret_cast<uintptr_t>(p); };
+  if (at(R) < at(G0) + block && at(G0) < at(R) + block) {
+    if (int st = trl_cuda_memcpy(h, small, G0, block, TRL_D2D)) return st;
+    G0 = small;
+  }
   ProfScope prof(h, PROF_CHOLQR, 2.0 * passes * n * bs * elt_size(dtype), 4.0 * passes * n * bs * bs);
   int st = TRL_OK;
   TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
