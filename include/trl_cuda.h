@@ -79,8 +79,8 @@ uint64_t trl_cuda_launch_count(trl_cuda_handle handle);
 /* ---- failure injection (tests of the error paths; no counterpart in the reference) -------
  * trl_cuda_inject_alloc_failures: the handle's next `count` calls of trl_cuda_malloc fail with
  * TRL_ENOMEM (the device is not touched); 0 clears. trl_cuda_test_bounded_wait: enqueues a
- * kernel whose wait on a shared-memory barrier can never complete; the wait gives up after
- * `polls` polls (at most 2^24), the kernel returns, and the next
+ * kernel whose waits, on a shared-memory barrier and on the handle's barrier over a grid, can
+ * never complete; each gives up after `polls` polls (at most 2^24), the kernel returns, and the next
  * trl_cuda_synchronize reports TRL_ETIMEOUT, as every bounded device wait of this library
  * does. The handle stays usable. */
 int trl_cuda_inject_alloc_failures(trl_cuda_handle handle, int count);

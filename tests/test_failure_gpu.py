@@ -44,6 +44,34 @@ def test_bounded_wait_times_out_and_the_handle_stays_usable():
         h.close()
 
 
+@pytest.mark.parametrize("breakdown", [False, True])
+def test_projection_after_a_grid_barrier_gave_up(breakdown):
+    """The barrier's arrivals are cleared with the status word, whichever error is reported."""
+    n, nblk, bs = 8193, 4, 4
+    rng = np.random.default_rng(7)
+    Vf = np.linalg.qr(rng.standard_normal((n, nblk * bs)))[0]
+    W = Vf @ rng.standard_normal((nblk * bs, bs)) + rng.standard_normal((n, bs))
+    ref = W - Vf @ (Vf.T @ W)
+    Vd = torch.from_numpy(np.ascontiguousarray(Vf.reshape(n, nblk, bs).transpose(1, 0, 2))).cuda()
+    Sd = Vd.sum(0) / np.sqrt(nblk)
+    G = torch.zeros((bs, bs), dtype=torch.float64, device="cuda")
+    h = native.Handle(0)
+    try:
+        for _ in range(3):
+            assert h.lib.trl_cuda_test_bounded_wait(h.h, 1000) == native.TRL_OK
+            if breakdown:
+                h.cholqr_gram(Sd.clone(), 1, G, -torch.eye(bs, dtype=torch.float64, device="cuda"))
+            assert h.lib.trl_cuda_synchronize(h.h) == (native.TRL_ECHOLESKY if breakdown else native.TRL_ETIMEOUT)
+            for _ in range(2):
+                Wd = torch.from_numpy(W).cuda()
+                h.project_out_sketch(Vd, Wd, Sd, 1e-6, G)
+                h.sync()
+                assert np.abs(Wd.cpu().numpy() - ref).max() < 1e-12 * np.abs(W).max()
+                assert np.allclose(G.cpu().numpy(), ref.T @ ref, rtol=0, atol=1e-12 * np.abs(ref.T @ ref).max())
+    finally:
+        h.close()
+
+
 def test_refused_allocation_makes_a_solve_return_enomem():
     A = P.laplace2d(32)
     X0 = torch.from_numpy(P.initial_block(A.n, 4, seed=42)).cuda()

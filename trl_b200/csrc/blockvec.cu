@@ -1210,37 +1210,6 @@ constexpr int kProjThreads = 512;
 constexpr int kProjWarps = kProjThreads / 32;
 constexpr int kProjMaxEntries = 8192; // coefficients, nblk BS^2, in shared memory
 
-// Barrier over the grid of a cooperative launch: bar[0] arrivals (zero between barriers), bar[1]
-// generation. Bounded: false (and TRL_DEV_TIMEOUT) after the limit; the caller then leaves.
-__device__ __forceinline__ bool grid_barrier(unsigned* bar, int* status)
-{
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned* gen = bar + 1;
-    const unsigned mine = *gen;
-    __threadfence(); // this CTA's writes, and the generation read, come before its arrival
-    ok = 1;
-    if (atomicAdd(bar, 1u) == gridDim.x - 1) {
-      bar[0] = 0u;
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    }
-    else {
-      unsigned polls = 0;
-      while (*gen == mine)
-        if (++polls == (1u << 24)) {
-          atomicOr(status, TRL_DEV_TIMEOUT);
-          ok = 0;
-          break;
-        }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
 template <typename T, int BS>
 __global__ void __launch_bounds__(kProjThreads, 1) k_project(const T* V, int nblk, T* W, int64_t n, int64_t rows_per_cta, const int* __restrict__ cond,
                                                              const double* __restrict__ before, double eta2, double* __restrict__ G, double* partial, double* total,
@@ -1344,12 +1313,12 @@ __global__ void __launch_bounds__(kProjThreads, 1) k_project(const T* V, int nbl
         __syncthreads();
       }
     }
-    if (!grid_barrier(bar, status)) return false;
+    if (!grid_barrier(bar, gridDim.x, status)) return false;
     for (int e0 = (static_cast<int>(blockIdx.x) * kProjWarps + warp) * 8; e0 < len; e0 += ncta * kProjWarps * 8) {
       const double t = sum_ctas(partial, len, e0, len);
       if (lane < 8 && e0 + lane < len) total[e0 + lane] = t;
     }
-    return grid_barrier(bar, status);
+    return grid_barrier(bar, gridDim.x, status);
   };
   // W -= sum_j V_j C_j over this CTA's rows, and Gs = the Gram matrix of the result over all rows
   const auto update = [&]() {
@@ -1430,7 +1399,7 @@ __global__ void __launch_bounds__(kProjThreads, 1) k_project(const T* V, int nbl
         gpartial[static_cast<int64_t>(blockIdx.x) * BB + row * BS + col] = v;
       }
     }
-    if (!grid_barrier(bar, status)) return false;
+    if (!grid_barrier(bar, gridDim.x, status)) return false;
     for (int e0 = warp * 8; e0 < BB; e0 += kProjWarps * 8) { // every CTA for itself: the decision needs no barrier
       const double t = sum_ctas(gpartial, BB, e0, BB);
       if (lane < 8 && e0 + lane < BB) Gs[e0 + lane] = t;

@@ -213,6 +213,38 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
+// Barrier over the `ctas` CTAs of a cooperative launch: bar[0] arrivals (zero between barriers), bar[1]
+// generation. Bounded: false (and TRL_DEV_TIMEOUT) after `limit` polls; the caller then leaves, and
+// the arrivals stay until trl_cuda_synchronize reads the status word.
+__device__ __forceinline__ bool grid_barrier(unsigned* bar, unsigned ctas, int* status, unsigned limit = (1u << 24))
+{
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    volatile unsigned* gen = bar + 1;
+    const unsigned mine = *gen;
+    __threadfence(); // this CTA's writes, and the generation read, come before its arrival
+    ok = 1;
+    if (atomicAdd(bar, 1u) == ctas - 1) {
+      bar[0] = 0u;
+      __threadfence();
+      atomicAdd(bar + 1, 1u);
+    }
+    else {
+      unsigned polls = 0;
+      while (*gen == mine)
+        if (++polls == limit) {
+          atomicOr(status, TRL_DEV_TIMEOUT);
+          ok = 0;
+          break;
+        }
+    }
+    __threadfence();
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
 // 1-D bulk copy global -> shared, completing `bytes` transactions on `bar`. Both addresses
 // 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar)

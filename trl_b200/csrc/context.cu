@@ -241,10 +241,10 @@ int trl_cuda_synchronize(trl_cuda_handle h)
   if (e != cudaSuccess) return set_error(h, TRL_ECUDA, "stream synchronize: %s", cudaGetErrorString(e));
   if (!h->prof_pending.empty()) prof_resolve(h);
   const int flags = *st;
+  // whatever else happened, a barrier that gave up has left counts behind
+  if ((flags & TRL_DEV_TIMEOUT) && h->d_small) cudaMemsetAsync(h->d_small + kSmallTickets, 0, (kSmallDoubles - kSmallTickets) * sizeof(double), h->stream);
   if (flags & TRL_DEV_CHOLESKY) return set_error(h, TRL_ECHOLESKY, "Cholesky factorization failed in orthonormalize");
   if (flags & TRL_DEV_EIGEN) return set_error(h, TRL_EEIGEN, "Eigendecomposition failed");
-  if ((flags & TRL_DEV_TIMEOUT) && h->d_small) // a barrier that gave up may have left counts behind
-    cudaMemsetAsync(h->d_small + kSmallTickets, 0, (kSmallDoubles - kSmallTickets) * sizeof(double), h->stream);
   if (flags & TRL_DEV_TIMEOUT) return set_error(h, TRL_ETIMEOUT, "a bounded device wait timed out");
   return TRL_OK;
 }
@@ -351,16 +351,19 @@ int trl_cuda_memset_zero(trl_cuda_handle h, void* ptr, size_t bytes)
 
 namespace {
 
-// One thread waits on a shared-memory mbarrier that expects two arrivals and gets one: the
-// phase never completes, the wait gives up after `polls` polls and records TRL_DEV_TIMEOUT.
-__global__ void k_wait_never_completes(int* status, unsigned polls)
+// One thread waits on a shared-memory mbarrier that expects two arrivals and gets one, then the CTA
+// waits at the handle's grid barrier for a second one that does not exist: neither phase ever
+// completes, each wait gives up after `polls` polls and records TRL_DEV_TIMEOUT.
+__global__ void k_wait_never_completes(unsigned* grid_bar, int* status, unsigned polls)
 {
   ::trl_detail::pdl_enter();
   __shared__ uint64_t bar;
-  if (threadIdx.x != 0) return;
-  mbar_init(&bar, 2);
-  mbar_arrive(&bar);
-  mbar_wait(&bar, 0, status, polls);
+  if (threadIdx.x == 0) {
+    mbar_init(&bar, 2);
+    mbar_arrive(&bar);
+    mbar_wait(&bar, 0, status, polls);
+  }
+  grid_barrier(grid_bar, 2, status, polls);
 }
 
 } // namespace
@@ -377,6 +380,8 @@ extern "C" int trl_cuda_test_bounded_wait(trl_cuda_handle h, unsigned polls)
 {
   TRL_CHECK_HANDLE(h);
   if (polls == 0 || polls > (1u << 24)) return set_error(h, TRL_EINVAL, "polls must be in [1, 2^24]");
-  launch(k_wait_never_completes, 1, 32, 0, h->stream, h->d_status, polls);
+  double* small = static_cast<double*>(small_scratch(h));
+  if (!small) return TRL_ENOMEM;
+  launch(k_wait_never_completes, 1, 32, 0, h->stream, reinterpret_cast<unsigned*>(small + kSmallCounters) + 2, h->d_status, polls);
   return after_launch(h, "bounded wait");
 }
