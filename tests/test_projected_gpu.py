@@ -97,3 +97,14 @@ def test_products_that_shrink_between_looks(cuda_handle, N, coupling):
     d = np.where(np.arange(N) < N // 3, 1.0, 0.25 * (np.arange(N) % 2))
     D = np.diag(d) + np.diag(np.full(N - 1, coupling), 1) + np.diag(np.full(N - 1, coupling), -1)
     _check(cuda_handle, D, 0)
+
+
+@pytest.mark.parametrize("N", [8, 140])
+@pytest.mark.parametrize("g", [2.0 ** -70, 2.0 ** -85, 2.0 ** -98])
+def test_reflectors_of_minute_norm(cuda_handle, N, g):
+    """Couplings that multiply up to g^3, down to 3e-89: a column of that norm is reduced by a reflector
+    whose scale, squared, is out of range."""
+    D = np.diag(np.where(np.arange(N) < 6, 0.0, 0.25 * np.arange(N) / (N - 1)))
+    for i, j, v in ((0, 1, 1.0), (0, 2, g), (1, 3, 1.0), (2, 3, g), (2, 4, g), (4, 5, g)):
+        D[i, j] = D[j, i] = v
+    _check(cuda_handle, D, 4)

@@ -543,7 +543,8 @@ __device__ __forceinline__ bool tri_steps(TriState<RPW>& st, const TriArgs& k)
       k4[q & 3] = fma(p.x, st.u[q], k4[q & 3]);
     }
     const double2 ps = pc[s];
-    const double K = 0.5 * tau * tau * warp_sum((k4[0] + k4[1]) + (k4[2] + k4[3]));
+    // tau times the sum first: tau is up to 1e290, and tau^2 alone may be out of range
+    const double K = 0.5 * tau * (tau * warp_sum((k4[0] + k4[1]) + (k4[2] + k4[3])));
     const double ws = fma(-K, us, tau * ps.x);
     st.dprev = fma(-2.0 * ws, us, ps.y);
     if constexpr (kReload) asm volatile("" ::: "memory");
