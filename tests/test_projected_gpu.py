@@ -108,3 +108,23 @@ def test_reflectors_of_minute_norm(cuda_handle, N, g):
     for i, j, v in ((0, 1, 1.0), (0, 2, g), (1, 3, 1.0), (2, 3, g), (2, 4, g), (4, 5, g)):
         D[i, j] = D[j, i] = v
     _check(cuda_handle, D, 4)
+
+
+@pytest.mark.parametrize("N,kvec", [(8, 8), (9, 9), (140, 139)])
+@pytest.mark.parametrize("g", [2.0 ** -40, 2.0 ** -60, 2.0 ** -98])
+def test_vectors_of_repeated_eigenvalues_with_minute_couplings(cuda_handle, N, kvec, g):
+    """Zero diagonals behind couplings that stand for zero: no pivot of the inverse iteration, whichever
+    row it comes from, is below the floor."""
+    D = np.diag(np.where(np.arange(N) < 6, 0.0, 0.25 * np.arange(N) / (N - 1)))
+    for i, j, v in ((0, 1, 1.0), (0, 2, g), (1, 3, 1.0), (2, 3, g), (2, 4, g), (4, 5, g)):
+        D[i, j] = D[j, i] = v
+    _check(cuda_handle, D, kvec)
+
+
+@pytest.mark.parametrize("N", [24, 97])
+@pytest.mark.parametrize("g", [1e-18, 1e-22, 1e-29])
+def test_vectors_of_chains_with_minute_couplings(cuda_handle, N, g):
+    """Tridiagonal already: pairs of rows with a strong coupling, minute ones between the pairs, all eigenvalues
+    +1 and -1 but for the odd last row."""
+    off = np.where(np.arange(N - 1) % 2 == 0, 1.0, g)
+    _check(cuda_handle, np.diag(off, 1) + np.diag(off, -1), N)

@@ -1032,7 +1032,8 @@ __device__ __forceinline__ double hash_unit(unsigned a, unsigned b)
 // and lane 1 from row N - 1 (a side sees the matrix in its own order, so both run the same
 // code), and leaves two equations in the two middle unknowns; substitution runs outwards. The
 // recurrences are chains of one reciprocal (factorisation) or one FMA (substitution) per row;
-// everything else is prepared by all lanes. Pivots below eps * ||T|| are replaced by +-eps * ||T||.
+// everything else is prepared by all lanes. Pivots below eps * ||T|| are replaced by +-eps * ||T||,
+// and the vector is brought to the middle of the range after each solve.
 // Position i of side s is stored at 2 i + s.
 // Measured on B200 (K = 40, N = 384 / K = 112, N = 512): 51 / 63 us (before,
 // one lane from one end, a kernel for the factors and one per solve: 177 / 227 us).
@@ -1068,6 +1069,9 @@ __global__ void __launch_bounds__(32) k_tri_vectors(const double* __restrict__ d
   if (!(nrm > 0.0)) nrm = 1.0;
   const double tiny = DBL_EPSILON * nrm;
   const auto floored = [tiny](double p) { return fabs(p) < tiny ? (p < 0.0 ? -tiny : tiny) : p; };
+  // whether the row below is the pivot row: not for an entry below the floor, which stands for zero (taken as
+  // a pivot it would multiply what is behind it by 1e25 and more, a vector out of range after a few)
+  const auto below = [tiny](double own, double other) { return fabs(own) < fabs(other) && fabs(other) >= tiny; };
   __syncwarp();
   const int side = lane & 1, len = side ? h1 : h0;
   double D = 0.0, U = 0.0, c = 0.0; // the equation carried along: D x_i + U x_{i+1} = c
@@ -1081,7 +1085,7 @@ __global__ void __launch_bounds__(32) k_tri_vectors(const double* __restrict__ d
       const int at = 2 * i + side;
       const int nx = i + 2 < len ? at + 4 : at + 2;
       const double d2 = U1[nx], e2 = U2[nx], b2 = X[nx]; // the next round's row
-      const bool sw = fabs(D) < fabs(L);
+      const bool sw = below(D, L);
       const double piv = sw ? L : floored(D);
       const double rp = 1.0 / piv;
       const double f = (sw ? D : L) * rp;
@@ -1104,7 +1108,7 @@ __global__ void __launch_bounds__(32) k_tri_vectors(const double* __restrict__ d
   // the two middle equations D x_own + U x_other = c, eliminated with pivoting on x of side 0
   const double D0 = __shfl_sync(0xffffffffu, D, 0), U0 = __shfl_sync(0xffffffffu, U, 0);
   const double D1 = __shfl_sync(0xffffffffu, D, 1), V1 = __shfl_sync(0xffffffffu, U, 1);
-  const bool mid = fabs(D0) < fabs(V1); // the equation of side 1 is the pivot row
+  const bool mid = below(D0, V1); // the equation of side 1 is the pivot row
   const double mr = 1.0 / (mid ? V1 : floored(D0));
   const double mf = (mid ? D0 : V1) * mr;
   const double mu = mid ? D1 : U0; // the pivot row's entry of x of side 1
@@ -1179,6 +1183,13 @@ __global__ void __launch_bounds__(32) k_tri_vectors(const double* __restrict__ d
         x1 = v;
       }
     }
+    __syncwarp();
+    double mx = 0.0;
+    for (int at = lane; at < N + 1; at += 32)
+      if (at / 2 < ((at & 1) ? h1 : h0)) mx = fmax(mx, fabs(X[at]));
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const double by = scalbn(1.0, -scale_exponent(mx));
+    for (int at = lane; at < N + 1; at += 32) X[at] *= by;
     __syncwarp();
   }
   for (int i = lane; i < N; i += 32) Z[static_cast<size_t>(t) * N + i] = X[i < h0 ? 2 * i : 2 * (N - 1 - i) + 1];
