@@ -293,7 +293,7 @@ int trl_cuda_sddmm(trl_cuda_handle h, const trl_csr* pattern, const double* X, i
  * cluster is well defined; its individual eigenvectors are not).
  *   kind = 0: grad[p] = df/dA_ij  = sum_c wbar[c] x_c[i] x_c[j]            (A, or K)
  *   kind = 1: grad[p] = df/dM_ij  = -sum_c wbar[c] lambda[c] x_c[i] x_c[j] (mass M)
- * for every stored entry p = (i, j) of `pattern` (values unused). */
+ * for every stored entry p = (i, j) of `pattern` (values unused). Synchronises the stream. */
 int trl_cuda_eigen_adjoint(trl_cuda_handle h, const trl_csr* pattern, const double* X, int k, const double* host_evals, const double* host_weights, double cluster_rtol,
                            int kind, double* grad);
 

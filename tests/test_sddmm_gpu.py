@@ -38,3 +38,26 @@ def test_sddmm_forms(cuda_handle, k, offset):
         out.fill_(float("nan"))
         cuda_handle.eigen_adjoint(Ad, Xd, np.arange(1.0, k + 1.0), w, out)
         assert np.all(np.abs(host(out) - terms.sum(1)) <= bound)
+
+
+@pytest.mark.parametrize("k", [1, 16, 256, 300])
+def test_adjoint_is_complete_on_return(k):
+    """Behind work that keeps the stream busy for milliseconds, the gradient is there for any stream when
+    the call returns."""
+    A = P.laplace2d(9)
+    X = torch.randn((A.n, k), dtype=torch.float64, device="cuda")
+    Ad = native.DeviceCSRTensors.from_host(A)
+    out = torch.empty(A.nnz, dtype=torch.float64, device="cuda")
+    a = torch.randn((4096, 4096), dtype=torch.float32, device="cuda")
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    h = native.Handle(0, stream=s)
+    try:
+        with torch.cuda.stream(s):
+            for _ in range(20):
+                a @ a
+        h.eigen_adjoint(Ad, X, np.arange(1.0, k + 1.0), np.ones(k), out)
+        assert s.query()
+    finally:
+        torch.cuda.synchronize()
+        h.close()

@@ -231,8 +231,9 @@ __global__ void __launch_bounds__(kThreads, SpmmShape<T, BS>::MINB) k_spmm(int64
 // q: L - 1 shuffles instead of L log L, and a coalesced store).
 // Bound by the L1/L2 traffic of the rows of X, 2 nnz * k * 8 bytes.
 // Measured on B200, 512^2 five-point pattern (nnz = 1.31 M) and its diagonal, k = 16, together:
-// 41 us (a lane per entry of one row per warp, X uncoalesced: 255 us with its copies and waits; a row
-// per group of 8 lanes and 16-byte pieces: 63 us; entries 32 at a time, 16-byte pieces: 57 us).
+// 41 us (a row per group of 8 lanes and 16-byte pieces: 63 us; entries 32 at a time, 16-byte pieces: 57
+// us). The two calls of trl_cuda_eigen_adjoint, each of which waits for its result: 67 us (a lane per
+// entry of one row per warp, X uncoalesced, coefficients copied: 256 us).
 constexpr int kSddmmMaxCoef = 256; // coefficients passed by value (2 KB of kernel parameters)
 
 struct SddmmCoef {
@@ -453,18 +454,23 @@ int trl_cuda_eigen_adjoint(trl_cuda_handle h, const trl_csr* P, const double* X,
     }
     s = e;
   }
-  if (k <= kSddmmMaxCoef) { // the coefficients travel with the launch: no copy, no wait
-    if (P->n == 0 || P->nnz == 0) return TRL_OK;
-    ProfScope prof(h, PROF_SDDMM, 12.0 * P->nnz + 4.0 * (P->n + 1) + 8.0 * P->n * k, 3.0 * P->nnz * k);
-    SddmmCoef cf;
-    std::copy(c.begin(), c.end(), cf.v);
-    return launch_sddmm(h, P, X, k, nullptr, cf, grad);
+  int st = TRL_OK;
+  if (k <= kSddmmMaxCoef) { // the coefficients travel with the launch
+    if (P->n > 0 && P->nnz > 0) {
+      ProfScope prof(h, PROF_SDDMM, 12.0 * P->nnz + 4.0 * (P->n + 1) + 8.0 * P->n * k, 3.0 * P->nnz * k);
+      SddmmCoef cf;
+      std::copy(c.begin(), c.end(), cf.v);
+      st = launch_sddmm(h, P, X, k, nullptr, cf, grad);
+    }
   }
-  double* dc = static_cast<double*>(workspace2(h, sizeof(double) * k));
-  if (!dc) return TRL_ENOMEM;
-  if (int st = trl_cuda_memcpy(h, dc, c.data(), sizeof(double) * k, TRL_H2D)) return st;
-  if (int st = trl_cuda_sddmm(h, P, X, k, dc, grad)) return st;
-  // the host coefficient array goes out of scope: make sure the copy has been consumed
+  else {
+    double* dc = static_cast<double*>(workspace2(h, sizeof(double) * k));
+    if (!dc) return TRL_ENOMEM;
+    st = trl_cuda_memcpy(h, dc, c.data(), sizeof(double) * k, TRL_H2D);
+    if (!st) st = trl_cuda_sddmm(h, P, X, k, dc, grad);
+  }
+  if (st) return st;
+  // the gradient is complete on return (and the host's coefficients have been consumed)
   cudaError_t e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) return set_error(h, TRL_ECUDA, "eigen_adjoint: %s", cudaGetErrorString(e));
   return TRL_OK;
