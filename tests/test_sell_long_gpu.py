@@ -76,3 +76,34 @@ def test_one_operator_on_two_handles(cuda_handle):
     torch.cuda.synchronize()
     assert all(torch.equal(y, ref) for o in out for y in o)
     op.close()
+
+
+@pytest.mark.parametrize("dtype", DT)
+def test_first_call_of_a_handle_inside_a_capture(cuda_handle, dtype):
+    """A prepared product allocates nothing, so it may be the first thing a handle does inside a stream
+    capture; the graph may be replayed."""
+    A = PATTERNS[1][1]
+    Ad = native.DeviceCSRTensors.from_host(A, dtype)
+    op = cuda_handle.prepare(Ad, 4)
+    X = dev(np.random.default_rng(0).standard_normal((A.n, 4)).astype(np.float32), dtype)
+    ref, Y = torch.empty_like(X), torch.empty_like(X)
+    op.spmm(X, ref)
+    cuda_handle.sync()
+    s = torch.cuda.Stream()
+    h = native.Handle(0, stream=s)
+    try:
+        h.sync()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            h.check(h.lib.trl_cuda_op_spmm(h.h, op.op, X.data_ptr(), Y.data_ptr(), 1, 1.0, 0.0, 0.0, None))
+        for _ in range(3):
+            Y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(Y, ref)
+        del g
+    finally:
+        torch.cuda.synchronize()
+        h.close()
+        op.close()

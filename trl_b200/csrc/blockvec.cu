@@ -1430,10 +1430,9 @@ namespace trl_detail {
 inline double* ticket_workspace(trl_cuda_context* h, int64_t chunks, int64_t len, Tickets& t)
 {
   const int64_t groups = (chunks + kTicketGroup - 1) / kTicketGroup;
-  double* small = static_cast<double*>(small_scratch(h));
-  if (!small || groups + 1 > kTickets) return nullptr;
+  if (groups + 1 > kTickets) return nullptr;
   double* partial = static_cast<double*>(workspace(h, static_cast<size_t>(chunks + groups) * len * sizeof(double)));
-  t.count = reinterpret_cast<unsigned*>(small + kSmallTickets);
+  t.count = reinterpret_cast<unsigned*>(h->d_small + kSmallTickets);
   t.groups = partial ? partial + chunks * len : nullptr;
   return partial;
 }
@@ -1639,8 +1638,7 @@ bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, 
   rows = rows < 16 ? 16 : (rows + 7) / 8 * 8;
   const int64_t ctas = (n + rows - 1) / rows;
   const size_t len = static_cast<size_t>(nblk) * BB;
-  double* small = static_cast<double*>(small_scratch(h));
-  double* partial = small ? static_cast<double*>(workspace(h, sizeof(double) * ((ctas + 1) * len + ctas * BB))) : nullptr;
+  double* partial = static_cast<double*>(workspace(h, sizeof(double) * ((ctas + 1) * len + ctas * BB)));
   if (!partial) {
     st = TRL_ENOMEM;
     return true;
@@ -1657,7 +1655,7 @@ bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, 
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   ProfScope prof(h, PROF_UPDATE, (2.0 * nblk + 3.0) * n * BS * sizeof(T), 2.0 * (2.0 * nblk + 2.0) * n * BS * BS);
-  cudaLaunchKernelEx(&cfg, kern, V, nblk, W, n, rows, cond, before, eta2, G, partial, total, total + len, reinterpret_cast<unsigned*>(small + kSmallCounters) + 2, h->d_status);
+  cudaLaunchKernelEx(&cfg, kern, V, nblk, W, n, rows, cond, before, eta2, G, partial, total, total + len, reinterpret_cast<unsigned*>(h->d_small + kSmallCounters) + 2, h->d_status);
   st = after_launch(h, "project");
   return true;
 }
@@ -1926,9 +1924,7 @@ int trl_cuda_cholqr(trl_cuda_handle h, int dtype, void* X, int64_t n, int bs, in
   if (int st = check_common(h, dtype, n, bs)) return st;
   if (passes < 1 || passes > 4) return set_error(h, TRL_EINVAL, "passes must be in [1, 4]");
   if (!X || !R) return set_error(h, TRL_EINVAL, "null pointer");
-  double* small = static_cast<double*>(small_scratch(h));
-  if (!small) return TRL_ENOMEM;
-  double* G = small;
+  double* G = h->d_small;
   ProfScope prof(h, PROF_CHOLQR, 3.0 * passes * n * bs * elt_size(dtype), 4.0 * passes * n * bs * bs);
   int st = trl_cuda_block_dot(h, dtype, X, 1, X, n, bs, G);
   if (st) return st;
@@ -1944,16 +1940,14 @@ int trl_cuda_cholqr_gram(trl_cuda_handle h, int dtype, void* X, int64_t n, int b
   if (int st = check_common(h, dtype, n, bs)) return st;
   if (passes < 1 || passes > kCholMaxPasses) return set_error(h, TRL_EINVAL, "passes must be in [1, 4]");
   if (!X || !R) return set_error(h, TRL_EINVAL, "null pointer");
-  double* small = static_cast<double*>(small_scratch(h));
-  if (!small) return TRL_ENOMEM;
-  double* U = small + kSmallFactors;
+  double* U = h->d_small + kSmallFactors;
   // R over G0 (the factor in place of its Gram matrix): every CTA of the first launch reads G0 while CTA 0
   // writes R, so they read a copy
   const size_t block = sizeof(double) * bs * bs;
   const auto at = [](const double* p) { return reinterpret_cast<uintptr_t>(p); };
   if (at(R) < at(G0) + block && at(G0) < at(R) + block) {
-    if (int st = trl_cuda_memcpy(h, small, G0, block, TRL_D2D)) return st;
-    G0 = small;
+    if (int st = trl_cuda_memcpy(h, h->d_small, G0, block, TRL_D2D)) return st;
+    G0 = h->d_small;
   }
   ProfScope prof(h, PROF_CHOLQR, 2.0 * passes * n * bs * elt_size(dtype), 4.0 * passes * n * bs * bs);
   int st = TRL_OK;
@@ -2216,8 +2210,7 @@ extern "C" int trl_cuda_measure_dmma_rate(trl_cuda_handle h, double* host_tflops
 {
   TRL_CHECK_HANDLE(h);
   if (!host_tflops) return set_error(h, TRL_EINVAL, "null output");
-  double* out = static_cast<double*>(small_scratch(h));
-  if (!out) return TRL_ENOMEM;
+  double* out = h->d_small;
   const int iters = 4096;
   const unsigned grid = static_cast<unsigned>(h->num_sms) * 8;
   cudaEvent_t a, b;

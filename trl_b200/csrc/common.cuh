@@ -64,11 +64,11 @@ inline bool valid_dtype(int dt) { return dt == TRL_F64 || dt == TRL_F32; }
 // Checks cudaGetLastError after a launch and counts the launch.
 int after_launch(trl_cuda_context* h, const char* what);
 
-// Per-handle device scratch of fixed size, in doubles from its start: a Gram matrix, the factors of a
-// CholQR (up to 4), and ticket and work counters (zero between kernels) and a grid barrier's state; nullptr on failure.
+// d_small, in doubles from its start: a Gram matrix, the factors of a CholQR (up to 4), and ticket and
+// work counters (zero between kernels) and a grid barrier's state. Allocated with the handle, so that
+// no call allocates it inside a stream capture.
 constexpr int kSmallFactors = 256, kSmallTickets = kSmallFactors + 4 * 256, kSmallCounters = kSmallTickets + 256,
               kSmallDoubles = kSmallCounters + 8;
-void* small_scratch(trl_cuda_context* h);
 // Releases the cuSOLVER handle and its workspace.
 void destroy_solver(trl_cuda_context* h);
 

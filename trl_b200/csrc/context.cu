@@ -191,8 +191,9 @@ int trl_cuda_create(trl_cuda_handle* out, int device, void* stream)
     }
     h->owns_stream = true;
   }
-  if (cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&h->d_status, sizeof(int)) != cudaSuccess || cudaMalloc(&h->d_small, kSmallDoubles * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
+    if (h->d_status) cudaFree(h->d_status);
     if (h->owns_stream) cudaStreamDestroy(h->stream);
     delete h;
     return TRL_ENOMEM;
@@ -200,11 +201,13 @@ int trl_cuda_create(trl_cuda_handle* out, int device, void* stream)
   if (cudaMallocHost(&h->pinned_status, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(h->d_status);
+    cudaFree(h->d_small);
     if (h->owns_stream) cudaStreamDestroy(h->stream);
     delete h;
     return TRL_ENOMEM;
   }
   cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream);
+  cudaMemsetAsync(h->d_small, 0, kSmallDoubles * sizeof(double), h->stream); // the counters start at zero
   *out = h;
   return TRL_OK;
 }
@@ -242,7 +245,7 @@ int trl_cuda_synchronize(trl_cuda_handle h)
   if (!h->prof_pending.empty()) prof_resolve(h);
   const int flags = *st;
   // whatever else happened, a barrier that gave up has left counts behind
-  if ((flags & TRL_DEV_TIMEOUT) && h->d_small) cudaMemsetAsync(h->d_small + kSmallTickets, 0, (kSmallDoubles - kSmallTickets) * sizeof(double), h->stream);
+  if (flags & TRL_DEV_TIMEOUT) cudaMemsetAsync(h->d_small + kSmallTickets, 0, (kSmallDoubles - kSmallTickets) * sizeof(double), h->stream);
   if (flags & TRL_DEV_CHOLESKY) return set_error(h, TRL_ECHOLESKY, "Cholesky factorization failed in orthonormalize");
   if (flags & TRL_DEV_EIGEN) return set_error(h, TRL_EEIGEN, "Eigendecomposition failed");
   if (flags & TRL_DEV_TIMEOUT) return set_error(h, TRL_ETIMEOUT, "a bounded device wait timed out");
@@ -380,8 +383,6 @@ extern "C" int trl_cuda_test_bounded_wait(trl_cuda_handle h, unsigned polls)
 {
   TRL_CHECK_HANDLE(h);
   if (polls == 0 || polls > (1u << 24)) return set_error(h, TRL_EINVAL, "polls must be in [1, 2^24]");
-  double* small = static_cast<double*>(small_scratch(h));
-  if (!small) return TRL_ENOMEM;
-  launch(k_wait_never_completes, 1, 32, 0, h->stream, reinterpret_cast<unsigned*>(small + kSmallCounters) + 2, h->d_status, polls);
+  launch(k_wait_never_completes, 1, 32, 0, h->stream, reinterpret_cast<unsigned*>(h->d_small + kSmallCounters) + 2, h->d_status, polls);
   return after_launch(h, "bounded wait");
 }

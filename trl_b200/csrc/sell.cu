@@ -788,12 +788,7 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
   int st = TRL_OK;
   const int dtype = op->dtype;
   // the slice counter and the count of finished warps belong to the handle: an operator may serve several
-  unsigned* counter = nullptr;
-  if (op->long_rows && nb == 1) {
-    double* small = static_cast<double*>(small_scratch(h));
-    if (!small) return TRL_ENOMEM;
-    counter = reinterpret_cast<unsigned*>(small + kSmallCounters);
-  }
+  unsigned* counter = reinterpret_cast<unsigned*>(h->d_small + kSmallCounters);
   TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
     // one resident wave
     const auto wave = [&](auto kernel, int minb) {

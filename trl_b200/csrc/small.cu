@@ -163,21 +163,6 @@ using namespace trl_detail;
 
 namespace trl_detail {
 
-void* small_scratch(trl_cuda_context* h)
-{
-  if (!h->d_small) {
-    if (cudaMalloc(&h->d_small, kSmallDoubles * sizeof(double)) != cudaSuccess) {
-      cudaGetLastError();
-      h->d_small = nullptr;
-      set_error(h, TRL_ENOMEM, "scratch allocation failed");
-      return nullptr;
-    }
-    // zeroed once: the ticket counters must start at zero
-    cudaMemsetAsync(h->d_small, 0, kSmallDoubles * sizeof(double), h->stream);
-  }
-  return h->d_small;
-}
-
 void destroy_solver(trl_cuda_context* h)
 {
   if (h->solver) cusolverDnDestroy(static_cast<cusolverDnHandle_t>(h->solver));
