@@ -77,6 +77,25 @@ def test_cholqr_factor_in_place_of_its_gram_matrix(cuda_handle, bs, dtype, passe
 
 
 @pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("columns", ["all", "first", "last"])
+@pytest.mark.parametrize("exponent", [-520, -500, 480])
+def test_cholqr_of_columns_at_the_ends_of_the_range(cuda_handle, bs, columns, exponent):
+    """2^-520: norms whose squares are subnormal, with 42 bits left of the Gram matrix; the second pass makes up
+    for them. Held to 1e-12: eps times the columns' condition (below 10) and the rows' sums."""
+    n = 300
+    scale = np.ones(bs)
+    scale[{"all": slice(None), "first": slice(0, 1), "last": slice(bs - 1, bs)}[columns]] = 2.0 ** exponent
+    X = np.random.default_rng(bs).standard_normal((n, bs))
+    Xd = dev(X * scale, torch.float64)
+    R = torch.full((bs, bs), float("nan"), dtype=torch.float64, device="cuda")
+    cuda_handle.cholqr(Xd, 2, R)
+    cuda_handle.sync()
+    Q, Rh = host(Xd), host(R) / scale  # R of X itself
+    assert np.abs(Q.T @ Q - np.eye(bs)).max() < 1e-12
+    assert np.abs(Q @ Rh - X).max() < 1e-12 * np.abs(X).max()
+
+
+@pytest.mark.parametrize("bs", BS)
 @pytest.mark.parametrize("passes", [1, 2])
 def test_cholqr_breakdown_leaves_block_and_factor(cuda_handle, bs, passes):
     X = torch.randn((1000, bs), dtype=torch.float64, device="cuda")

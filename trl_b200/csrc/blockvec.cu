@@ -929,15 +929,18 @@ struct FactorSpace {
 // / 20,500 cycles for 4 / 8 / 16 columns, most of them waiting for instructions; now 2,500
 // / 4,100 / 9,200 (with a division per entry in place of the reciprocal: 2,600 / 4,400 / 10,800, and twice
 // that where the code is cold).
+// A row and column whose diagonal entry is below 2^-800 are scaled by 2^400 and the factor scaled back:
+// a pivot's reciprocal would be out of range (columns of norm below 7e-155).
 // false (uniform): a pivot was <= 0 or NaN; Ui is then the identity, which leaves an apply a no-op.
 template <int BS>
 __device__ __forceinline__ bool cta_factor(const double* G, FactorSpace<BS>& f, double* Ui)
 {
   constexpr int COLS = 2 * BS;
   constexpr int PER = (BS * COLS + kThreads - 1) / kThreads; // entries per thread
+  const auto minute = [&](int k) { return G[k * (BS + 1)] < 0x1p-800; };
   for (int e = threadIdx.x; e < BS * BS; e += kThreads) {
     const int r = e / BS, k = e % BS;
-    f.A[r][k] = k <= r ? G[e] : G[k * BS + r];
+    f.A[r][k] = (k <= r ? G[e] : G[k * BS + r]) * (minute(r) ? 0x1p400 : 1.0) * (minute(k) ? 0x1p400 : 1.0);
     f.A[r][BS + k] = r == k ? 1.0 : 0.0;
   }
   bool ok = true;
@@ -964,8 +967,8 @@ __device__ __forceinline__ bool cta_factor(const double* G, FactorSpace<BS>& f, 
   __syncthreads();
   for (int e = threadIdx.x; e < BS * BS; e += kThreads) {
     const int r = e / BS, k = e % BS; // row r, column k of L, and of L^{-1}
-    f.L[r][k] = r == k ? f.root[k] : f.L[r][k] / f.root[k];
-    Ui[k * BS + r] = ok ? (k <= r ? f.A[r][BS + k] / f.root[r] : 0.0) : (r == k ? 1.0 : 0.0);
+    f.L[r][k] = (r == k ? f.root[k] : f.L[r][k] / f.root[k]) * (minute(r) ? 0x1p-400 : 1.0);
+    Ui[k * BS + r] = ok ? (k <= r ? f.A[r][BS + k] / f.root[r] * (minute(k) ? 0x1p400 : 1.0) : 0.0) : (r == k ? 1.0 : 0.0);
   }
   __syncthreads();
   return ok;
