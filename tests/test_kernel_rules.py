@@ -5,6 +5,9 @@ import os
 import re
 import subprocess
 
+import numpy as np
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "trl_b200", "csrc")
 
@@ -36,3 +39,32 @@ def test_every_pair_of_the_tridiagonalisation_is_waited_for(tmp_path):
     assert steps.count("st_async_pair(") == 1
     assert re.search(r"if \(tri_sends\(N, g, lane, s\)\)\s*st_async_pair\(", steps)
     assert "static_cast<uint32_t>(N - s) * 16u" in steps
+
+
+@pytest.fixture(scope="module")
+def largest_overlaps(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("host") / "orthonormal_limit")
+    src = os.path.join(ROOT, "tests", "host", "orthonormal_limit.cc")
+    subprocess.run(["/usr/bin/g++", "-std=c++17", "-O1", f"-I{CSRC}", src, "-o", exe], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
+    return [(int(k), float(e)) for k, e in (ln.split() for ln in out.splitlines())]
+
+
+@pytest.mark.parametrize("signs", ["equal", "random"])
+def test_second_orthonormalisation_step_ends_at_rounding(largest_overlaps, signs):
+    """The step z_j - E_jj / 2 z_j - sum_{i<j} E_ij z_i in extended precision on a Gram matrix I + E with every
+    overlap at the largest that is let through. It leaves (S^T (I + E) S) - I with S = I - D / 2 - U: -E_ij E_ik
+    summed over K vectors, and E^2 once for the diagonal's share: (K + 1) E^2 <= 2 eps."""
+    for K, e in largest_overlaps:
+        E = np.full((K, K), e, dtype=np.longdouble)
+        if signs == "random":
+            E *= np.sign(np.random.default_rng(K).standard_normal((K, K)))
+            E = np.triu(E) + np.triu(E, 1).T
+        S = np.eye(K, dtype=np.longdouble) - np.triu(E, 1) - np.diag(np.diag(E)) / 2
+        left = S.T @ (np.eye(K, dtype=np.longdouble) + E) @ S - np.eye(K, dtype=np.longdouble)
+        assert np.abs(left).max() <= 2 * np.finfo(np.float64).eps, K
+
+
+def test_orthonormalisation_decides_by_the_checked_limit():
+    launches = re.findall(r"launch\((?:k_gs_apply|k_tri_gs),[^;]*;", source("small.cu"))
+    assert len(launches) == 2 and all("gs_limit(K)" in ln for ln in launches)

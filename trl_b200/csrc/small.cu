@@ -7,6 +7,7 @@
 // and the Ritz estimates ||beta * y_last|| / max(|theta|, eps) (evp_base.hh:124-151) are
 // counted on the device. Only the eigenvalues and the converged count come back to the host.
 #include "common.cuh"
+#include "orthonormal_limit.h"
 #include "tridiag_schedule.h"
 
 #include <cooperative_groups.h>
@@ -1191,10 +1192,9 @@ __global__ void __launch_bounds__(32) k_tri_vectors(const double* __restrict__ d
 //  1. k_tri_cluster: Gram-Schmidt twice within each group of closer eigenvalues, a CTA per group;
 //     it also scales every vector to unit length;
 //  2. k_gs_gram, k_gs_apply twice;
-//  3. k_tri_gs, where the first step left more than kGsLimit (never seen): Gram-Schmidt twice
-//     over all vectors.
+//  3. k_tri_gs, where the first step left more than the second may be given (gs_limit; never
+//     seen): Gram-Schmidt twice over all vectors.
 constexpr double kClusterGap = 1e-10;
-constexpr double kGsLimit = 1e-8;
 
 // Gram-Schmidt twice of z_j against z_first .. z_{j-1}, then unit length, by one CTA; coef: K
 // doubles of shared memory
@@ -1286,14 +1286,14 @@ __global__ void __launch_bounds__(256) k_gs_gram(int N, int K, const double* __r
 }
 
 // out_j = z_j - (E_jj / 2) z_j - sum_{i<j} E_ij z_i: a warp per 8 vectors x 32 entries (DMMA).
-// With emax above kGsLimit: out = z.
-__global__ void __launch_bounds__(128) k_gs_apply(int N, int K, const double* __restrict__ Z, const double* __restrict__ E, const unsigned long long* emax, double* __restrict__ out)
+// With emax above the limit: out = z.
+__global__ void __launch_bounds__(128) k_gs_apply(int N, int K, const double* __restrict__ Z, const double* __restrict__ E, const unsigned long long* emax, double limit, double* __restrict__ out)
 {
   ::trl_detail::pdl_enter();
   const int lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
   const int j0 = blockIdx.x * 8, n0 = (blockIdx.y * 4 + (threadIdx.x >> 5)) * 32;
   if (n0 >= N) return;
-  const int iend = (emax && __longlong_as_double(static_cast<long long>(*emax)) > kGsLimit) ? 0 : min(j0 + 8, K);
+  const int iend = (emax && __longlong_as_double(static_cast<long long>(*emax)) > limit) ? 0 : min(j0 + 8, K);
   double d0[4] = {0.0, 0.0, 0.0, 0.0}, d1[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 4
   for (int i0 = 0; i0 < iend; i0 += 4) {
@@ -1317,11 +1317,11 @@ __global__ void __launch_bounds__(128) k_gs_apply(int N, int K, const double* __
   }
 }
 
-// Gram-Schmidt twice over all vectors, one CTA, if *emax is above kGsLimit
-__global__ void __launch_bounds__(kTriThreads) k_tri_gs(int N, int K, double* __restrict__ Z, const unsigned long long* emax)
+// Gram-Schmidt twice over all vectors, one CTA, if *emax is above the limit
+__global__ void __launch_bounds__(kTriThreads) k_tri_gs(int N, int K, double* __restrict__ Z, const unsigned long long* emax, double limit)
 {
   ::trl_detail::pdl_enter();
-  if (!(__longlong_as_double(static_cast<long long>(*emax)) > kGsLimit)) return;
+  if (!(__longlong_as_double(static_cast<long long>(*emax)) > limit)) return;
   __shared__ double coef[kTriMaxVec];
   __shared__ double red[32];
   for (int j = 0; j < K; ++j) gs_column(N, 0, j, Z, coef, red);
@@ -1690,10 +1690,10 @@ extern "C" int trl_cuda_small_eigen_partial(trl_cuda_handle h, const double* T, 
     unsigned long long* check = round == 0 ? nullptr : emax;
     launch(k_gs_gram, kt * (kt + 1) / 2, 256, 0, h->stream, N, K, from, E, check);
     if (int st = after_launch(h, "overlaps")) return st;
-    launch(k_gs_apply, apply_grid, 128, 0, h->stream, N, K, from, E, check, to);
+    launch(k_gs_apply, apply_grid, 128, 0, h->stream, N, K, from, E, check, gs_limit(K), to);
     if (int st = after_launch(h, "orthogonalise")) return st;
   }
-  launch(k_tri_gs, 1, kTriThreads, 0, h->stream, N, K, Z, emax);
+  launch(k_tri_gs, 1, kTriThreads, 0, h->stream, N, K, Z, emax, gs_limit(K));
   if (int st = after_launch(h, "gram-schmidt")) return st;
   const int nch = (N - 2 + kWyRows - 1) / kWyRows;
   launch(k_wy_factor, nch, kWyThreads, 0, h->stream, refl, tau, N, ld, Tw);
