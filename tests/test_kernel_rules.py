@@ -68,3 +68,16 @@ def test_second_orthonormalisation_step_ends_at_rounding(largest_overlaps, signs
 def test_orthonormalisation_decides_by_the_checked_limit():
     launches = re.findall(r"launch\((?:k_gs_apply|k_tri_gs),[^;]*;", source("small.cu"))
     assert len(launches) == 2 and all("gs_limit(K)" in ln for ln in launches)
+
+
+def test_kernels_of_one_type_have_their_own_ctas_per_sm(tmp_path):
+    from trl_b200 import build
+
+    exe = str(tmp_path / "resident_ctas")
+    src = os.path.join(ROOT, "tests", "host", "resident_ctas.cu")
+    subprocess.run([build.NVCC, *build.ARCH, "-std=c++17", f"-I{CSRC}", f"-I{ROOT}/include", src, "-o", exe], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True, env=dict(os.environ, CUDA_VISIBLE_DEVICES="")).stdout
+    assert out.split() == ["4", "2", "4", "2", "3"]
+    # no cache beside it that is shared between kernels of one type
+    for name in ("sell.cu", "spmm.cu"):
+        assert "cudaOccupancyMaxActiveBlocksPerMultiprocessor" not in source(name)

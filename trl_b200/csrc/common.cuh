@@ -5,6 +5,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <string>
@@ -124,6 +125,29 @@ inline unsigned grid_for(const trl_cuda_context* h, int64_t work_items, int item
   if (need < 1) need = 1;
   return static_cast<unsigned>(need < cap ? need : cap);
 }
+
+// CTAs of `Kernel` that fit an SM, at least 1; `fallback` where the runtime cannot say. Asked for once
+// per kernel and device: kernels of one type (other template arguments) have an answer each, and
+// host threads may ask at once.
+template <auto Kernel>
+int resident_ctas(int device, int threads, size_t smem, int fallback)
+{
+  static std::atomic<int> known[64];
+  std::atomic<int>& slot = known[device & 63];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, Kernel, threads, smem) != cudaSuccess || n < 1) n = fallback;
+    cudaGetLastError();
+    slot.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// A kernel as a type, for functions that are generic over kernels
+template <auto Kernel>
+struct KernelOf {
+  static constexpr auto fn = Kernel;
+};
 
 // Programmatic dependent launch. Every kernel of the library starts with pdl_enter(). A
 // kernel launched by launch() below (programmatic stream serialization) may have its CTAs

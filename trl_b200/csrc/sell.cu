@@ -791,28 +791,20 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
   unsigned* counter = reinterpret_cast<unsigned*>(h->d_small + kSmallCounters);
   TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
     // one resident wave
-    const auto wave = [&](auto kernel, int minb) {
-      static int resident[64]; // per device and instantiation of the kernel
-      int& res = resident[h->device & 63];
-      if (res == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&res, kernel, kSpmmThreads, 0) != cudaSuccess || res < 1) res = minb;
-        cudaGetLastError();
-      }
-      return grid_for(h, op->nslices, kSpmmWarps, res);
-    };
+    const auto wave = [&](auto kernel, int minb) { return grid_for(h, op->nslices, kSpmmWarps, resident_ctas<decltype(kernel)::fn>(h->device, kSpmmThreads, 0, minb)); };
     const int ns = static_cast<int>(op->nslices), nwin = static_cast<int>(op->nwin);
     const T* vals = static_cast<const T*>(op->sval);
     const T* Wt = static_cast<const T*>(W);
     const T a = static_cast<T>(alpha), b = static_cast<T>(beta), g = static_cast<T>(gamma);
     const auto run = [&](auto kernel, int minb) {
-      trl_detail::launch(kernel, wave(kernel, minb), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, op->interleave, op->perm, op->sptr, op->scol, vals, static_cast<const T*>(X),
+      trl_detail::launch(kernel.fn, wave(kernel, minb), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, op->interleave, op->perm, op->sptr, op->scol, vals, static_cast<const T*>(X),
                          static_cast<T*>(Y), a, b, g, Wt, nb, op->n * BS);
     };
-    if (nb > 1) run(k_spmm_sell<T, BS, kSellBlocksPerPass>, SellTune<T, BS, kSellBlocksPerPass>::MINB);
+    if (nb > 1) run(KernelOf<k_spmm_sell<T, BS, kSellBlocksPerPass>>{}, SellTune<T, BS, kSellBlocksPerPass>::MINB);
     else if (op->long_rows)
-      trl_detail::launch(k_spmm_sell_long<T, BS>, wave(k_spmm_sell_long<T, BS>, 2), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, counter, op->interleave, op->perm, op->sptr, op->scol, vals,
+      trl_detail::launch(k_spmm_sell_long<T, BS>, wave(KernelOf<k_spmm_sell_long<T, BS>>{}, 2), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, counter, op->interleave, op->perm, op->sptr, op->scol, vals,
                          static_cast<const T*>(X), static_cast<T*>(Y), a, b, g, Wt);
-    else run(k_spmm_sell<T, BS, 1>, SellTune<T, BS, 1>::MINB);
+    else run(KernelOf<k_spmm_sell<T, BS, 1>>{}, SellTune<T, BS, 1>::MINB);
     st = after_launch(h, "spmm (sliced ELL)");
   }));
   return st;

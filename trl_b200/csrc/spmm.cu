@@ -379,17 +379,12 @@ static int spmm_impl(trl_cuda_context* h, const trl_csr* A, int dtype, const voi
     using S = SpmmShape<T, BS>;
     // one resident wave: every warp strides over the rows (its rowptr prefetch pays off)
     const auto run = [&](auto kernel) {
-      static int resident = 0; // one per instantiation of the kernel
-      if (resident == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThreads, 0) != cudaSuccess || resident < 1) resident = S::MINB;
-        cudaGetLastError();
-      }
-      const unsigned grid = grid_for(h, (A->n + S::RPW - 1) / S::RPW, kThreads / 32, resident);
-      trl_detail::launch(kernel, grid, kThreads, 0, h->stream, A->n, A->rowptr, A->colind, static_cast<const T*>(A->values), static_cast<const T*>(X), static_cast<T*>(Y),
+      const unsigned grid = grid_for(h, (A->n + S::RPW - 1) / S::RPW, kThreads / 32, resident_ctas<decltype(kernel)::fn>(h->device, kThreads, 0, S::MINB));
+      trl_detail::launch(kernel.fn, grid, kThreads, 0, h->stream, A->n, A->rowptr, A->colind, static_cast<const T*>(A->values), static_cast<const T*>(X), static_cast<T*>(Y),
                                                static_cast<T>(alpha), static_cast<T>(beta), static_cast<T>(gamma), static_cast<const T*>(W), nb, A->n * BS);
     };
-    if (nb > 1) run(k_spmm<T, BS, true>);
-    else run(k_spmm<T, BS, false>);
+    if (nb > 1) run(KernelOf<k_spmm<T, BS, true>>{});
+    else run(KernelOf<k_spmm<T, BS, false>>{});
     st = after_launch(h, "spmm");
   }));
   return st;
