@@ -81,3 +81,17 @@ def test_kernels_of_one_type_have_their_own_ctas_per_sm(tmp_path):
     # no cache beside it that is shared between kernels of one type
     for name in ("sell.cu", "spmm.cu"):
         assert "cudaOccupancyMaxActiveBlocksPerMultiprocessor" not in source(name)
+
+
+def test_no_unguarded_static_state():
+    """What a function keeps for the process is atomic or behind a lock: host threads with a handle each call the
+    library at the same time."""
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh")):
+            continue
+        src = source(name)
+        kept = [ln.strip() for ln in src.splitlines() if re.match(r"\s+static (?!constexpr|const |std::atomic|std::mutex|__device__|_?assert)(?!.*\()", ln)]
+        if name == "small.cu":  # tri_variant's, behind its lock
+            assert "static std::mutex lock;" in body(src, "const TriVariant* tri_variant(")
+            kept = [ln for ln in kept if ln not in ("static int ok[64][kNumTriVariants];", "static bool checked[64];")]
+        assert kept == [], name

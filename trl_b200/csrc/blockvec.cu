@@ -1495,11 +1495,7 @@ int launch_block_dot_bulk(trl_cuda_context* h, const T* V, int nblk, const T* W,
     cudaGetLastError();
     return set_error(h, TRL_ECUDA, "block dot: %zu bytes of shared memory refused", smem);
   }
-  static int resident = 0; // CTAs per SM at this shared-memory size (queried once; same on every B200)
-  if (resident == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_block_dot_bulk<T, BS, JC, S, TB>, kThreads, smem) != cudaSuccess || resident < 1) resident = 1;
-    cudaGetLastError();
-  }
+  const int resident = resident_ctas<k_block_dot_bulk<T, BS, JC, S, TB>>(h->device, kThreads, smem, 1);
   const int64_t len = static_cast<int64_t>(nblk) * BS * BS;
   const int gj = (nblk + JC - 1) / JC;
   int64_t chunks = static_cast<int64_t>(h->num_sms) * resident / gj;
@@ -1578,11 +1574,7 @@ int launch_update_gram_rt(trl_cuda_context* h, const T* in, int MB, const double
   // 6,539): one input block per loop iteration (U = 1) beats explicit multi-block register
   // prefetch (U = 4: FP64 6,075, FP32 3,860), and 8-row tiles per warp RT = 4 (FP64, 6,784)
   // and RT = 2 (FP32, 5,439) with two resident waves of CTAs do best.
-  static int resident = 0;
-  if (resident == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_update_gram<T, BS, RT, 1, Fin>, kThreads, 0) != cudaSuccess || resident < 1) resident = 4;
-    cudaGetLastError();
-  }
+  const int resident = resident_ctas<k_update_gram<T, BS, RT, 1, Fin>>(h->device, kThreads, 0, 4);
   const unsigned grid = grid_for(h, (n + 8 * RT - 1) / (8 * RT), kWarps, 2 * resident);
   Tickets t{};
   double* partial = ticket_workspace(h, grid, BS * BS, t);
@@ -1624,8 +1616,8 @@ bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, 
   if (n > kProjRows || static_cast<int64_t>(nblk) * n * BS * static_cast<int64_t>(sizeof(T)) > kProjBytes || nblk * BB > kProjMaxEntries) return false;
   const auto kern = k_project<T, BS>;
   const auto smem = [](int entries) { return sizeof(double) * (entries + static_cast<size_t>(kProjWarps) * (8 * BS + NT * NT * 64)); };
-  static int usable[64]; // per device: 1 the kernel can be launched with the most shared memory, -1 it cannot
-  int& ok = usable[h->device & 63];
+  static std::atomic<int> usable[64]; // per device: 1 the kernel can be launched with the most shared memory, -1 it cannot
+  int ok = usable[h->device & 63];
   if (ok == 0) {
     int resident = 0, coop = 0;
     const size_t most = smem(kProjMaxEntries);
@@ -1633,7 +1625,7 @@ bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, 
                       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)) == cudaSuccess &&
                       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, kProjThreads, most) == cudaSuccess && resident > 0;
     cudaGetLastError();
-    ok = fits ? 1 : -1;
+    usable[h->device & 63] = ok = fits ? 1 : -1;
   }
   if (ok < 0) return false;
   // a CTA per SM, each with 16 rows (two tiles) at least
@@ -1670,11 +1662,7 @@ int launch_cholqr(trl_cuda_context* h, T* X, int64_t n, const double* G0, int nf
 {
   constexpr int NT = (BS + 7) / 8;
   constexpr int RT = NT >= 2 ? 2 : 4;
-  static int resident = 0;
-  if (resident == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_cholqr<T, BS, RT, GRAM>, kThreads, 0) != cudaSuccess || resident < 1) resident = 4;
-    cudaGetLastError();
-  }
+  const int resident = resident_ctas<k_cholqr<T, BS, RT, GRAM>>(h->device, kThreads, 0, 4);
   // one resident wave: every CTA prepares its factors once
   const unsigned grid = grid_for(h, (n + 8 * RT - 1) / (8 * RT), kWarps, resident);
   Tickets t{};
