@@ -61,3 +61,28 @@ def test_adjoint_is_complete_on_return(k):
     finally:
         torch.cuda.synchronize()
         h.close()
+
+
+def _band(n, width):
+    cols = np.sort((np.arange(n)[:, None] + np.arange(width)) % n, axis=1)
+    return P._from_coo(n, np.repeat(np.arange(n), width), cols.ravel(), np.ones(n * width))
+
+
+@pytest.mark.parametrize("n,width", [(4096, 11), (4097, 11), (4097, 12), (8192, 7), (8193, 7), (8193, 8), (8193, 15), (8193, 16), (9001, 1), (500, 300)])
+@pytest.mark.parametrize("k,offset", [(1, 0), (3, 0), (6, 0), (8, 1), (8, 2), (34, 0), (62, 0), (66, 0), (5, 0), (20, 0)])
+def test_sddmm_either_side_of_the_choice_of_kernel(cuda_handle, n, width, k, offset):
+    rng = np.random.default_rng(n + k)
+    A = _band(n, width)
+    X = rng.standard_normal((n, k))
+    w = rng.uniform(0.5, 2.0, k)
+    Xd = torch.zeros(n * k + offset, dtype=torch.float64, device="cuda")[offset:].view(n, k)
+    Xd.copy_(torch.from_numpy(X))
+    terms = w * X[A.row_indices()] * X[A.colind]
+    bound = 2 * (k + 2) * EPS * np.abs(terms).sum(1)
+    Ad = native.DeviceCSRTensors.from_host(A)
+    out = torch.full((A.nnz,), float("nan"), dtype=torch.float64, device="cuda")
+    cuda_handle.sddmm(Ad, Xd, dev(w), out)
+    assert np.all(np.abs(host(out) - terms.sum(1)) <= bound)
+    out.fill_(float("nan"))
+    cuda_handle.eigen_adjoint(Ad, Xd, np.arange(1.0, k + 1.0), w, out)
+    assert np.all(np.abs(host(out) - terms.sum(1)) <= bound)

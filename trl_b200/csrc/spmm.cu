@@ -238,6 +238,11 @@ constexpr int kSddmmMaxCoef = 256; // coefficients passed by value (2 KB of kern
 
 struct SddmmCoef {
   double v[kSddmmMaxCoef];
+  __device__ __forceinline__ double operator()(int c) const { return v[c]; }
+};
+struct SddmmCoefPtr { // in device memory
+  const double* w;
+  __device__ __forceinline__ double operator()(int c) const { return __ldg(w + c); }
 };
 
 template <int VEC>
@@ -249,17 +254,16 @@ __device__ __forceinline__ void load_cols(const double* p, double (&out)[VEC])
     load_vec<double, VEC>(p, out);
 }
 
-// w in device memory, or (null) by value in cf; the CTA keeps them in shared memory either way
-// as far as they fit kSddmmMaxCoef
-template <int L, int VEC>
+// the CTA keeps the coefficients in shared memory as far as they fit kSddmmMaxCoef
+template <int L, int VEC, class Coef>
 __global__ void __launch_bounds__(kThreads) k_sddmm(int64_t n, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, const double* __restrict__ X, int k,
-                                                    const double* __restrict__ w, const __grid_constant__ SddmmCoef cf, int rpw, double* __restrict__ out)
+                                                    const __grid_constant__ Coef cf, int rpw, double* __restrict__ out)
 {
   ::trl_detail::pdl_enter();
   __shared__ double ws[kSddmmMaxCoef];
-  for (int c = threadIdx.x; c < k && c < kSddmmMaxCoef; c += kThreads) ws[c] = w ? w[c] : cf.v[c];
+  for (int c = threadIdx.x; c < k && c < kSddmmMaxCoef; c += kThreads) ws[c] = cf(c);
   __syncthreads();
-  const auto coef = [&](int c) { return c < kSddmmMaxCoef ? ws[c] : __ldg(w + c); };
+  const auto coef = [&](int c) { return c < kSddmmMaxCoef ? ws[c] : cf(c); };
   const int lane = threadIdx.x & 31, sub = lane % L;
   const int64_t step = static_cast<int64_t>(gridDim.x) * (kThreads / 32) * rpw;
   for (int64_t r0 = (static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5)) * rpw; r0 < n; r0 += step) {
@@ -322,24 +326,65 @@ __global__ void __launch_bounds__(kThreads) k_sddmm(int64_t n, const int32_t* __
   }
 }
 
-// lanes per entry by k: a lane's VEC columns at a time cover k in one round up to k = 8 VEC
-int launch_sddmm(trl_cuda_context* h, const trl_csr* P, const double* X, int k, const double* w, const SddmmCoef& cf, double* out)
+// One warp per row, a lane per entry: a lane reads the k values of its entry's row of X one after the
+// other, the warp its own row's as broadcasts.
+template <class Coef>
+__global__ void __launch_bounds__(kThreads) k_sddmm_rows(int64_t n, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colind, const double* __restrict__ X, int k,
+                                                         const __grid_constant__ Coef cf, double* __restrict__ out)
+{
+  ::trl_detail::pdl_enter();
+  const int lane = threadIdx.x & 31;
+  const int64_t warp_global = static_cast<int64_t>(blockIdx.x) * (kThreads / 32) + (threadIdx.x >> 5);
+  const int64_t warp_stride = static_cast<int64_t>(gridDim.x) * (kThreads / 32);
+  for (int64_t row = warp_global; row < n; row += warp_stride) {
+    const int kbeg = __ldg(rowptr + row), kend = __ldg(rowptr + row + 1);
+    const double* xr = X + row * k;
+    for (int p = kbeg + lane; p < kend; p += 32) {
+      const double* xc = X + static_cast<int64_t>(__ldg(colind + p)) * k;
+      double s = 0.0;
+      for (int c = 0; c < k; ++c) s = fma(cf(c) * __ldg(xr + c), __ldg(xc + c), s);
+      out[p] = s;
+    }
+  }
+}
+
+// Which kernel. Where X comes in single columns (odd k, or X so aligned), a lane of k_sddmm gathers 8 bytes
+// at a time and pays two shuffles for it, where a lane of k_sddmm_rows walks down one row of X; but of a
+// short row that leaves most lanes idle. us, rows / entries: 74 entries per row, k = 1 13 / 18, 5 26 / 40, 17
+// 97 / 112; 35 per row, k = 5 45 / 70, 17 124 / 185, 255 1,773 / 3,494; 15 per row, k = 5 11 / 24; 7 per
+// row, k = 5 23 / 13; 5 per row, 262,144 rows, k = 5 49 / 18, 17 117 / 53, 8,100 rows, k = 17 6.5 / 8.0; 10
+// per row, k = 1 7.6 / 5.0, 5 11 / 16. With 16-byte pieces (k even, not a multiple of 4) the same up to a few
+// rounds: 35 per row, k = 10 72 / 99, 18 129 / 170, 66 432 / 402; 12 per row, k = 10 9.3 / 16, 66 45 / 61;
+// 10 per row, k = 10 16 / 14. (k = 8, 32: a walk's lanes, strides of a power of two apart, collide: 10 per
+// row, k = 32 74 / 23.)
+template <class Coef>
+int launch_sddmm(trl_cuda_context* h, const trl_csr* P, const double* X, int k, const Coef& cf, double* out)
 {
   const auto aligned = [&](int v) { return k % v == 0 && reinterpret_cast<uintptr_t>(X) % (v * sizeof(double)) == 0; }; // every row of X
   const int vec = aligned(4) ? 4 : (aligned(2) ? 2 : 1);
-  const int need = k / vec;
-  // rows per warp: 32, fewer where that would leave SMs without two warps per scheduler
+  const auto mean = [&](int entries) { return P->nnz >= entries * P->n; }; // rows of `entries` or more on average
+  const bool rows = vec == 1 ? mean(k == 1 ? 16 : 8) || P->n <= 8192 : vec == 2 && k % 4 != 0 && k < 64 && (mean(12) || P->n <= 4096);
+  if (rows) {
+    launch(k_sddmm_rows<Coef>, grid_for(h, P->n, kThreads / 32, 16), kThreads, 0, h->stream, P->n, P->rowptr, P->colind, X, k, cf, out);
+    return after_launch(h, "sddmm");
+  }
+  // rows per warp: 32, fewer where a warp would get more than 256 entries, or where that would leave an SM
+  // fewer than 20 warps (8 for short rows in 16- or 32-byte pieces, which a warp is soon done with). us at 32 /
+  // this many, rows of 74 on average, 41,472 of them: k = 4 45 / 23, 16 110 / 50, 300 2,355 / 785.
+  const int64_t warps = static_cast<int64_t>(h->num_sms) * (vec > 1 && !mean(vec == 4 ? 16 : 8) ? 8 : 20);
   int rpw = 32;
-  while (rpw > 4 && P->n < static_cast<int64_t>(rpw) * h->num_sms * 8) rpw /= 2;
+  while (rpw > 1 && (P->n < rpw * warps || rpw * P->nnz > 256 * P->n)) rpw /= 2;
+  // lanes per entry by k: a lane's VEC columns at a time cover k in one round up to k = 8 VEC
+  const int need = k / vec;
   const auto run = [&](auto kernel) {
-    launch(kernel, grid_for(h, (P->n + rpw - 1) / rpw, kThreads / 32, 8), kThreads, 0, h->stream, P->n, P->rowptr, P->colind, X, k, w, cf, rpw, out);
+    launch(kernel, grid_for(h, (P->n + rpw - 1) / rpw, kThreads / 32, 8), kThreads, 0, h->stream, P->n, P->rowptr, P->colind, X, k, cf, rpw, out);
   };
   const auto lanes = [&](auto v) {
     constexpr int VEC = decltype(v)::value;
-    if (need <= 1) run(k_sddmm<1, VEC>);
-    else if (need <= 2) run(k_sddmm<2, VEC>);
-    else if (need <= 4) run(k_sddmm<4, VEC>);
-    else run(k_sddmm<8, VEC>);
+    if (need <= 1) run(k_sddmm<1, VEC, Coef>);
+    else if (need <= 2) run(k_sddmm<2, VEC, Coef>);
+    else if (need <= 4) run(k_sddmm<4, VEC, Coef>);
+    else run(k_sddmm<8, VEC, Coef>);
   };
   if (vec == 4) lanes(std::integral_constant<int, 4>{});
   else if (vec == 2) lanes(std::integral_constant<int, 2>{});
@@ -415,7 +460,7 @@ int trl_cuda_sddmm(trl_cuda_handle h, const trl_csr* P, const double* X, int k, 
   if (k <= 0) return set_error(h, TRL_EINVAL, "k must be positive");
   if (P->n == 0 || P->nnz == 0) return TRL_OK;
   ProfScope prof(h, PROF_SDDMM, 12.0 * P->nnz + 4.0 * (P->n + 1) + 8.0 * P->n * k, 3.0 * P->nnz * k);
-  return launch_sddmm(h, P, X, k, w, SddmmCoef{}, out);
+  return launch_sddmm(h, P, X, k, SddmmCoefPtr{w}, out);
 }
 
 int trl_cuda_eigen_adjoint(trl_cuda_handle h, const trl_csr* P, const double* X, int k, const double* host_evals, const double* host_weights, double cluster_rtol, int kind,
@@ -455,7 +500,7 @@ int trl_cuda_eigen_adjoint(trl_cuda_handle h, const trl_csr* P, const double* X,
       ProfScope prof(h, PROF_SDDMM, 12.0 * P->nnz + 4.0 * (P->n + 1) + 8.0 * P->n * k, 3.0 * P->nnz * k);
       SddmmCoef cf;
       std::copy(c.begin(), c.end(), cf.v);
-      st = launch_sddmm(h, P, X, k, nullptr, cf, grad);
+      st = launch_sddmm(h, P, X, k, cf, grad);
     }
   }
   else {
