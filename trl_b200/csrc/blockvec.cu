@@ -997,6 +997,20 @@ __device__ __forceinline__ void cta_factor_store(bool ok, FactorSpace<BS>& f, co
   }
 }
 
+// KS adjacent columns of a row in as few stores as possible (the counterpart of load_cols)
+template <typename T, int KS>
+__device__ __forceinline__ void store_cols(T* p, const T (&v)[KS])
+{
+  constexpr int VEC = KS * sizeof(T) > 16 ? 16 / static_cast<int>(sizeof(T)) : KS;
+#pragma unroll
+  for (int c = 0; c < KS; c += VEC) {
+    T part[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) part[i] = v[c + i];
+    ::trl_detail::store_vec<T, VEC>(p + c, part);
+  }
+}
+
 // X's rows as a warp holds them: lane (g, t4) columns 8 t + 2 t4 and the next one of row g of an
 // 8-row tile, which is at once the accumulator layout of a DMMA and, with the k dimension
 // permuted, its A operand: the product with a factor feeds the next one without a move.
@@ -1194,6 +1208,108 @@ __global__ void __launch_bounds__(kThreads) k_cholqr(T* X, int64_t n, const doub
     if (last_cta_sum<BB>(partial, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), tickets, sum, sum + BB)) {
       const bool ok = cta_factor<BS>(sum, fs, Us[0]);
       cta_factor_store<BS>(ok, fs, Us[0], U + nf * BB, R, false, status);
+    }
+  }
+}
+
+// The same for rows of up to 16 bytes: a thread per row, since of the 32 lanes that hold 8 rows above
+// half or more would have nothing to load. Only the lower triangle of the Gram matrix is formed.
+// Measured on B200, us, k_cholqr / this, two passes: 100,003 x 1 FP64 11.1 / 8.5, x 2 FP32 13.7 / 10.9, x 4 FP32
+// 14.7 / 12.8; 884,736 x 2 FP32 32.9 / 13.9, x 4 FP32 34.9 / 24.5. (Rows of 32 bytes: 884,736 x 4 FP64
+// 27.8 / 29.5, 5,000 x 4 9.1 / 10.0; a factor per launch and the block stored between the passes: 100,003 x 1
+// 11.4, x 2 FP32 12.7, 884,736 x 2 FP32 31.3.)
+template <typename T, int BS, int R, bool GRAM>
+__global__ void __launch_bounds__(kThreads) k_cholqr_narrow(T* X, int64_t n, const double* __restrict__ G0, int nf, double* U, double* R_out, int* status,
+                                                            double* __restrict__ partial, Tickets tickets)
+{
+  ::trl_detail::pdl_enter();
+  constexpr int BB = BS * BS, TRI = BS * (BS + 1) / 2;
+  __shared__ double Us[kCholMaxPasses][BB];
+  __shared__ FactorSpace<BS> fs;
+  __shared__ double Gs[BB];
+  __shared__ double red[TRI + kThreads]; // totals, scratch
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (G0) {
+    for (int e = tid; e < BB; e += kThreads) Gs[e] = G0[e];
+    __syncthreads();
+    const bool ok = cta_factor<BS>(Gs, fs, Us[0]);
+    if (blockIdx.x == 0) cta_factor_store<BS>(ok, fs, Us[0], U, R_out, true, status);
+  }
+  else
+    for (int e = tid; e < nf * BB; e += kThreads) Us[e / BB][e % BB] = U[e];
+  __syncthreads();
+  const bool whole = reinterpret_cast<uintptr_t>(X) % (BS * sizeof(T) < 16 ? BS * sizeof(T) : 16) == 0; // rows in as few loads as possible
+  double gram[TRI];
+#pragma unroll
+  for (int e = 0; e < TRI; ++e) gram[e] = 0.0;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kThreads * R;
+  for (int64_t r0 = static_cast<int64_t>(blockIdx.x) * kThreads * R + tid; r0 < n; r0 += step) {
+    T v[R][BS];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int64_t row = r0 + q * kThreads;
+#pragma unroll
+      for (int c = 0; c < BS; ++c) v[q][c] = T(0);
+      if (row < n) {
+        if (whole) load_cols<T, BS>(X + row * BS, v[q]);
+        else
+#pragma unroll
+          for (int c = 0; c < BS; ++c) v[q][c] = X[row * BS + c];
+      }
+    }
+    for (int f = 0; f < nf; ++f) {
+#pragma unroll
+      for (int c = BS - 1; c >= 0; --c) { // the factor is upper triangular: column c needs the first c + 1
+        double u[BS];
+#pragma unroll
+        for (int k = 0; k <= c; ++k) u[k] = Us[f][k * BS + c];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          double s = 0.0;
+#pragma unroll
+          for (int k = 0; k <= c; ++k) s = fma(static_cast<double>(v[q][k]), u[k], s);
+          v[q][c] = static_cast<T>(s); // rounded to T as a stored block would be
+        }
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int64_t row = r0 + q * kThreads;
+      if constexpr (GRAM) { // rows past n are zero
+#pragma unroll
+        for (int i = 0; i < BS; ++i)
+#pragma unroll
+          for (int k = 0; k <= i; ++k) gram[i * (i + 1) / 2 + k] = fma(static_cast<double>(v[q][i]), static_cast<double>(v[q][k]), gram[i * (i + 1) / 2 + k]);
+      }
+      else if (row < n) {
+        if (whole) store_cols<T, BS>(X + row * BS, v[q]);
+        else
+#pragma unroll
+          for (int c = 0; c < BS; ++c) X[row * BS + c] = v[q][c];
+      }
+    }
+  }
+  if constexpr (GRAM) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int e = 0; e < TRI; ++e) gram[e] += __shfl_xor_sync(0xffffffffu, gram[e], o);
+    if (lane == 0)
+#pragma unroll
+      for (int e = 0; e < TRI; ++e) red[warp * TRI + e] = gram[e];
+    __syncthreads();
+    if (tid < TRI) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) v += red[w * TRI + tid];
+      partial[static_cast<int64_t>(blockIdx.x) * TRI + tid] = v;
+    }
+    __syncthreads();
+    if (last_cta_sum<TRI>(partial, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), tickets, red, red + TRI)) {
+      if (tid < BB) Gs[tid] = tid / BS >= tid % BS ? red[tid / BS * (tid / BS + 1) / 2 + tid % BS] : 0.0; // the factorisation reads the lower triangle
+      __syncthreads();
+      const bool ok = cta_factor<BS>(Gs, fs, Us[0]);
+      cta_factor_store<BS>(ok, fs, Us[0], U + nf * BB, R_out, false, status);
     }
   }
 }
@@ -1655,21 +1771,38 @@ bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, 
   return true;
 }
 
+constexpr int64_t kCholStream = int64_t(64) << 20; // bytes of a block that comes from memory (about half of L2)
+
 // One pass of k_cholqr over the block: GRAM factors the Gram matrix of X U_0 ... U_{nf-1}, otherwise
 // X <- X U_0 ... U_{nf-1}.
 template <typename T, int BS, bool GRAM>
 int launch_cholqr(trl_cuda_context* h, T* X, int64_t n, const double* G0, int nf, double* U, double* R)
 {
-  constexpr int NT = (BS + 7) / 8;
-  constexpr int RT = NT >= 2 ? 2 : 4;
-  const int resident = resident_ctas<k_cholqr<T, BS, RT, GRAM>>(h->device, kThreads, 0, 4);
-  // one resident wave: every CTA prepares its factors once
-  const unsigned grid = grid_for(h, (n + 8 * RT - 1) / (8 * RT), kWarps, resident);
-  Tickets t{};
-  double* partial = nullptr;
-  if (GRAM && !(partial = ticket_workspace(h, grid, BS * BS, t))) return TRL_ENOMEM;
-  launch(k_cholqr<T, BS, RT, GRAM>, grid, kThreads, 0, h->stream, X, n, G0, nf, U, R, h->d_status, partial, t);
-  return after_launch(h, "cholqr");
+  const auto run = [&](auto kernel, unsigned grid) {
+    Tickets t{};
+    double* partial = nullptr;
+    if (GRAM && !(partial = ticket_workspace(h, grid, BS * BS, t))) return static_cast<int>(TRL_ENOMEM);
+    launch(kernel.fn, grid, kThreads, 0, h->stream, X, n, G0, nf, U, R, h->d_status, partial, t);
+    return after_launch(h, "cholqr");
+  };
+  if constexpr (BS * sizeof(T) <= 16) {
+    constexpr int ROWS = 4;
+    unsigned grid = grid_for(h, n, kThreads * ROWS, 2);
+    if (GRAM && grid > kTicketGroup && grid <= 2 * kTicketGroup) grid = kTicketGroup; // one round of sums
+    return run(KernelOf<k_cholqr_narrow<T, BS, ROWS, GRAM>>{}, grid);
+  }
+  else {
+    // one resident wave: every CTA prepares its factors once
+    const auto tiles = [&](auto rt) {
+      constexpr int RT = decltype(rt)::value;
+      return run(KernelOf<k_cholqr<T, BS, RT, GRAM>>{}, grid_for(h, n, kWarps * 8 * RT, resident_ctas<k_cholqr<T, BS, RT, GRAM>>(h->device, kThreads, 0, 4)));
+    };
+    // 16 columns in FP32 from memory: more warps with a tile each (us, 4,194,304 rows, two tiles / one: 1 pass 218
+    // / 174, 2 passes 494 / 405, 4 passes 1,231 / 1,134; from L2 two are better, 300,001 rows, 4 passes 126 / 137)
+    if constexpr (BS == 16 && sizeof(T) == 4)
+      if (n * BS * static_cast<int64_t>(sizeof(T)) > kCholStream) return tiles(std::integral_constant<int, 1>{});
+    return tiles(std::integral_constant<int, (BS > 8 ? 2 : 4)>{});
+  }
 }
 
 template <typename T, int BS, int NBMAX>
