@@ -4,6 +4,8 @@ fewer slices than warps, rows of one window only, and a last window with missing
 starts at zero again in every call, and two handles may use one operator at the same time.
 Bit for bit the CSR kernel's per-row walk (trl_cuda_spmm_blocks), and the oracle to the
 tolerances of test_sell_gpu.py."""
+import functools
+
 import numpy as np
 import pytest
 import torch
@@ -107,3 +109,40 @@ def test_first_call_of_a_handle_inside_a_capture(cuda_handle, dtype):
         torch.cuda.synchronize()
         h.close()
         op.close()
+
+
+@functools.lru_cache(None)
+def _with_counter(kind):
+    """Slices enough and long enough that their warps take them from the counter: rows of one length nearly, and
+    a skewed pattern whose longest slices come first."""
+    n, base = (20000, 420) if kind == "even" else (40000, 152)
+    deg = base + np.arange(n) % 9
+    if kind == "skewed":
+        deg[::1501] = 1500
+        deg[7::1013] = 0
+    row = np.repeat(np.arange(n), deg)
+    col = (row + 7 * (np.arange(row.size) - np.repeat(np.cumsum(deg) - deg, deg))) % n
+    return P._from_coo(n, row, col, np.random.default_rng(n).standard_normal(row.size))
+
+
+@pytest.mark.parametrize("bs", BS)
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("kind", ["even", "skewed"])
+def test_slices_from_the_counter(cuda_handle, bs, dtype, kind):
+    A = _with_counter(kind)
+    Ad = native.DeviceCSRTensors.from_host(A, dtype)
+    op = cuda_handle.prepare(Ad, bs)
+    X, W = (dev(as_dt(np.random.default_rng(s).standard_normal((A.n, bs)), dtype), dtype) for s in (1, 2))
+    ref = torch.empty((2, A.n, bs), dtype=dtype, device="cuda")
+    cuda_handle.spmm_blocks(Ad, torch.stack([X, X]), ref, -0.5, 2.0, 0.25, torch.stack([W, W]))
+    for _ in range(3):
+        Y = torch.full((A.n, bs), float("nan"), dtype=dtype, device="cuda")
+        op.spmm(X, Y, -0.5, 2.0, 0.25, W)
+        assert torch.equal(Y, ref[0])
+    op.close()
+
+
+def test_counters_of_two_handles_and_of_replays(cuda_handle, monkeypatch):
+    monkeypatch.setitem(globals(), "PATTERNS", [None, ("skewed", _with_counter("skewed"))])
+    test_one_operator_on_two_handles(cuda_handle)
+    test_first_call_of_a_handle_inside_a_capture(cuda_handle, torch.float64)

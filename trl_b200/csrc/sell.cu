@@ -492,19 +492,20 @@ __device__ __forceinline__ void load_slots(V* out, const V* p, int count, std::i
 // irregular patterns, by L2-to-SM traffic; the walk of k_spmm_sell spent half of the issue slots on
 // tests and addresses, so here only the last group of a slice tests its slots, and the others'
 // loads are constant offsets from two running pointers.
-// The warps take slices from a counter (at zero between launches) instead of every (number of
+// With a counter (at zero between launches) the warps take slices from it instead of every (number of
 // warps)-th: on the Zipf pattern a slice holds up to 512 slots where a warp's whole share is 480, and
 // a third of the SMs' time was spent waiting for the last warps. For such skewed patterns
 // (`ranked`) the longest slices of all windows come first, and the first ones go to different SMs.
-// Measured on B200, us (before: k_spmm_sell with 8 slots x 2 CTAs, static): elasticity 64^3 bs 8 FP64 223
-// (257), FP32 127 (148); Zipf 524,288 rows FP32 bs 16 115 (170), FP64 bs 8 121 (132-181), FP64 bs 16 181
-// (187-204), FP32 bs 4 114 (180). The counter alone gave 124 and 131 us in place of 115 and 121.
+// trl_cuda_op_spmm says when a counter pays.
+// Measured on B200, us (before: k_spmm_sell with 8 slots x 2 CTAs): elasticity 64^3 bs 8 FP64 223
+// (257), FP32 127 (147); Zipf 524,288 rows FP32 bs 16 115 (169), FP64 bs 8 121 (181), FP64 bs 16 181
+// (204), FP32 bs 4 109 (178). The counter without the order gave 124 and 131 us in place of 115 and 121.
 constexpr int kSellLongSlots = 8;
 
 template <typename T, int BS>
 __global__ void __launch_bounds__(kSpmmThreads, 2)
     k_spmm_sell_long(int nslices, int nwin, int spw, unsigned* counter, int ranked, const int32_t* __restrict__ perm, const int64_t* __restrict__ sptr, const int32_t* __restrict__ scol,
-                     const T* __restrict__ sval, const T* __restrict__ X, T* Y, T alpha, T beta, T gamma, const T* W)
+                     const T* __restrict__ sval, const T* __restrict__ X, T* Y, T alpha, T beta, T gamma, const T* W, int prefetch)
 {
   ::trl_detail::pdl_enter();
   using S = SellShape<T, BS>;
@@ -518,10 +519,12 @@ __global__ void __launch_bounds__(kSpmmThreads, 2)
   auto slice_of = [&](int i) -> int {
     return ranked ? static_cast<int>(static_cast<unsigned>(i) % static_cast<unsigned>(nwin)) * spw + static_cast<int>(static_cast<unsigned>(i) / static_cast<unsigned>(nwin)) : i;
   };
-  // the next place: asked for early by lane 0, shared when it is needed
+  // the next place: asked for early by lane 0, shared when it is needed; without a counter every
+  // nwarps-th
   int ticket = 0;
   auto ask = [&]() {
-    if (lane == 0) ticket = static_cast<int>(atomicAdd(counter, 1u)) + nwarps;
+    if (!counter) ticket += nwarps;
+    else if (lane == 0) ticket = static_cast<int>(atomicAdd(counter, 1u)) + nwarps;
   };
   auto answer = [&]() {
     int i = __shfl_sync(0xffffffffu, ticket, 0);
@@ -546,7 +549,7 @@ __global__ void __launch_bounds__(kSpmmThreads, 2)
     return q;
   };
   auto prefetch_slice = [&](const Slice& q) {
-    if (lane == 0 && q.left > 0) {
+    if (prefetch && lane == 0 && q.left > 0) {
       prefetch_l2(scol + q.e0, static_cast<uint32_t>(q.left * C * 4));
       prefetch_l2(sval + q.e0, static_cast<uint32_t>(q.left * C * sizeof(T)));
     }
@@ -635,7 +638,7 @@ __global__ void __launch_bounds__(kSpmmThreads, 2)
       prefetch_slice(nxt);
     }
   }
-  if (lane == 0) { // the last warp leaves the counters at zero
+  if (counter && lane == 0) { // the last warp leaves the counters at zero
     __threadfence();          // this warp's last ticket is taken before it counts as done
     if (atomicAdd(counter + 1, 1u) == static_cast<unsigned>(nwarps - 1)) counter[0] = counter[1] = 0u;
   }
@@ -787,8 +790,6 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
   ProfScope prof(h, PROF_SPMM, op->nnz * (es + 4.0) + 4.0 * (op->n + 1) + nb * (W ? 3.0 : 2.0) * op->n * bs * es, 2.0 * op->nnz * bs * nb);
   int st = TRL_OK;
   const int dtype = op->dtype;
-  // the slice counter and the count of finished warps belong to the handle: an operator may serve several
-  unsigned* counter = reinterpret_cast<unsigned*>(h->d_small + kSmallCounters);
   TRL_DISPATCH_DT(dtype, TRL_DISPATCH_BS(bs, {
     // one resident wave
     const auto wave = [&](auto kernel, int minb) { return grid_for(h, op->nslices, kSpmmWarps, resident_ctas<decltype(kernel)::fn>(h->device, kSpmmThreads, 0, minb)); };
@@ -801,9 +802,24 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
                          static_cast<T*>(Y), a, b, g, Wt, nb, op->n * BS);
     };
     if (nb > 1) run(KernelOf<k_spmm_sell<T, BS, kSellBlocksPerPass>>{}, SellTune<T, BS, kSellBlocksPerPass>::MINB);
-    else if (op->long_rows)
-      trl_detail::launch(k_spmm_sell_long<T, BS>, wave(KernelOf<k_spmm_sell_long<T, BS>>{}, 2), kSpmmThreads, 0, h->stream, ns, nwin, op->spw, counter, op->interleave, op->perm, op->sptr, op->scol, vals,
-                         static_cast<const T*>(X), static_cast<T*>(Y), a, b, g, Wt);
+    else if (op->long_rows) {
+      const unsigned grid = wave(KernelOf<k_spmm_sell_long<T, BS>>{}, 2);
+      // A counter costs its first round of tickets, and short slices wait for theirs. us, every n-th slice /
+      // counter: 24^3 elasticity bs 8 FP64 21 / 24; 44^3 bs 4 FP64 (273 slots a warp) 64 / 63, bs 8 (545) 88 / 85;
+      // 64^3 bs 8 (1,700) 235 / 223; 300,000 rows of 20, bs 16 FP64 (316) 58 / 66. Skewed: Zipf 60,000 rows bs 16
+      // FP64 (114) 40 / 41, 200,000 rows bs 8 (190) 73 / 68, bs 16 (380) 89 / 71; 524,288 rows, bs 1 FP64
+      // (250) 128 / 129, FP32 111 / 117, bs 2 FP64 129 / 121.
+      const int64_t per_warp = op->stored / op->C / (static_cast<int64_t>(grid) * kSpmmWarps); // slots
+      const bool wide = bs * es >= 16;
+      const bool tickets = wide && (op->interleave ? per_warp >= 150 : per_warp >= 400 && op->stored >= 48 * op->nslices * op->C);
+      // the counter and the count of finished warps belong to the handle: an operator may serve several
+      unsigned* counter = tickets ? reinterpret_cast<unsigned*>(h->d_small + kSmallCounters) : nullptr;
+      // narrow rows leave so many slices under way that, beyond L2, what is prefetched is gone before it is
+      // read (64^3 elasticity, bs 1 FP64, with / without: 181 / 110 us; 32^3, 95 MB: 13 / 16)
+      const int prefetch = wide || op->stored * static_cast<int64_t>(es + 4) <= int64_t(128) << 20;
+      trl_detail::launch(k_spmm_sell_long<T, BS>, grid, kSpmmThreads, 0, h->stream, ns, nwin, op->spw, counter, op->interleave, op->perm, op->sptr, op->scol, vals,
+                         static_cast<const T*>(X), static_cast<T*>(Y), a, b, g, Wt, prefetch);
+    }
     else run(KernelOf<k_spmm_sell<T, BS, 1>>{}, SellTune<T, BS, 1>::MINB);
     st = after_launch(h, "spmm (sliced ELL)");
   }));
