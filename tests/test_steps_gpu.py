@@ -177,3 +177,10 @@ def test_wide_blocks_at_tile_edges(cuda_handle, dtype, n, nblk):
     got = host(Wd)
     assert np.abs(got - out).max() <= (1e-12 if dtype == torch.float64 else 1.2e-7) * size
     close(host(G), got.T @ got, (np.abs(got).T @ np.abs(got)).max())
+
+
+@pytest.mark.parametrize("dtype", DT)
+@pytest.mark.parametrize("n,nblk,bs", [(17500, 20, 4), (17501, 20, 4), (32768, 3, 1), (32769, 3, 1), (32768, 2, 8), (32769, 2, 8),
+                                       (4096, 2, 16), (4097, 2, 16), (24576, 3, 16), (24577, 3, 16)])
+def test_projections_where_the_launches_split(cuda_handle, dtype, n, nblk, bs):
+    test_projections_at_the_edges_of_one_launch(cuda_handle, bs, dtype, n, nblk)

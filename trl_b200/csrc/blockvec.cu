@@ -1321,10 +1321,8 @@ __global__ void __launch_bounds__(kThreads) k_cholqr_narrow(T* X, int64_t n, con
 // kernels (dot, its reduction, update; each twice, and launched also when the sketch asks for nothing)
 // cost more in launches than in work on small bases, and stream faster on large ones.
 // cond: the sketch's decision. before: the Gram matrix before the pass.
-// Measured on B200, us, separate kernels / this one. Sketch that asks for nothing: 22.8 / 10.5 at
-// every size. Sketch that asks for a projection: 1,024 x 4 x 8 blocks 23 / 20, 16,384 x 4 x 20 28 / 29,
-// 16,384 x 8 x 40 40 / 38 (FP32 36 / 43), 60,000 x 8 x 16 41 / 43, 131,072 x 4 x 14 42 / 51. (project_out
-// always runs and keeps to the separate kernels, so that its modes agree to the last bit.)
+// one_launch_projects has the times on both sides. (project_out always runs and keeps to the separate
+// kernels, so that its modes agree to the last bit.)
 constexpr int kProjThreads = 512;
 constexpr int kProjWarps = kProjThreads / 32;
 constexpr int kProjMaxEntries = 8192; // coefficients, nblk BS^2, in shared memory
@@ -1719,17 +1717,28 @@ int launch_update_gram(trl_cuda_context* h, const T* in, int MB, const double* c
   }
 }
 
-// The projection in one launch for small bases: true if it ran (st: its status), false if the separate
-// kernels have to: beyond kProjBytes of basis (about half of L2) or kProjRows rows, where a projection
-// costs more here than the sketches that ask for none save (k_project has the times on both sides).
-constexpr int64_t kProjBytes = int64_t(64) << 20;
-constexpr int64_t kProjRows = 65536;
+// Where the projection is one launch. A sketch that asks for nothing is 8 - 10 us there and 18 - 19 us in
+// separate kernels, at every size; one that asks for a projection is faster in separate kernels by an
+// amount that grows with the rows and, in narrow or FP32 blocks, with their number. The line lies where
+// that amount would make the call slower than it was with a kernel for each test, flag and sum (29 - 34 us
+// at least). us, that / one launch / separate kernels: FP32 16,384 x 4, 20 blocks 34 / 31 / 25, 40 blocks 35 / 38 /
+// 28; 24,576 x 4, 16 blocks 32 / 33 / 26; FP64 16,384 x 4, 40 blocks 35 / 34 / 32; 32,768 x 8, 24 blocks 42 / 41 / 38;
+// 49,152 x 8, 4 blocks 31 / 33 / 27; 24,576 x 1, 40 blocks 38 / 39 / 18; 16 columns FP32, 24,576 rows, 2 blocks 38 / 42 /
+// 34, 16 blocks 63 / 59 / 53; 32,768 rows, 8 blocks 49 / 52 / 45; 4,096 rows, 2 blocks 34 / 29 / 23.
+template <typename T, int BS>
+bool one_launch_projects(int64_t n, int nblk)
+{
+  if (nblk * BS * BS > kProjMaxEntries || nblk * n * BS * static_cast<int64_t>(sizeof(T)) > (int64_t(64) << 20)) return false; // (half of L2)
+  if (BS == 16) return n <= 4096 || (n <= 24576 && nblk > 2);
+  return n <= 32768 && ((BS > 1 && sizeof(T) == 8) || nblk * n <= 350000);
+}
 
+// True if the projection ran in one launch (st: its status), false if the separate kernels have to.
 template <typename T, int BS>
 bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, const int* cond, const double* before, double eta2, double* G, int& st)
 {
   constexpr int BB = BS * BS, NT = (BS + 7) / 8;
-  if (n > kProjRows || static_cast<int64_t>(nblk) * n * BS * static_cast<int64_t>(sizeof(T)) > kProjBytes || nblk * BB > kProjMaxEntries) return false;
+  if (!one_launch_projects<T, BS>(n, nblk)) return false;
   const auto kern = k_project<T, BS>;
   const auto smem = [](int entries) { return sizeof(double) * (entries + static_cast<size_t>(kProjWarps) * (8 * BS + NT * NT * 64)); };
   static std::atomic<int> usable[64]; // per device: 1 the kernel can be launched with the most shared memory, -1 it cannot
