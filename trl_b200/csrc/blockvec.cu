@@ -791,9 +791,11 @@ __global__ void __launch_bounds__(kThreads, BS == 16 ? 2 : 0) k_update_gram(cons
   ::trl_detail::pdl_enter();
   if (cond && *cond == 0) return;
   // input blocks per loop body, without which ptxas picks worse ones from kernel to kernel.
-  // Measured on B200 (one projection, 884,736 rows, 2 / 3 blocks): FP64 bs 1 250 / 214 us, 2 175 / 183,
-  // 4 285 / 319, 8 462 / 511; FP32 bs 1 195 / 182, 2 415 / 393, 4 265 / 220, 8 286 / 295.
-  constexpr int kUnroll = (sizeof(T) == 4 ? BS <= 4 : BS == 1) ? 3 : 2;
+  // Measured on B200 (one projection, 884,736 rows, 2 / 3 blocks): FP64 bs 2 175 / 183 us, 4 285 / 319, 8
+  // 462 / 511; FP32 bs 1 195 / 182, 2 415 / 393, 4 265 / 220, 8 286 / 295; FP64 bs 1, 24 blocks (3 / 4) 258 / 225.
+  // ptxas's schedule hangs on the form of this loop: with `accumulate`, `sign` and U, which have one value each,
+  // taken out, FP64 bs 2 and 24 blocks took 377 us in place of 218, bs 4 322 in place of 259.
+  constexpr int kUnroll = sizeof(T) == 4 ? (BS <= 4 ? 3 : 2) : (BS == 1 ? 4 : 2);
   constexpr int NT = (BS + 7) / 8;
   constexpr int KS = (BS + 3) / 4;
   __shared__ double stage[kWarps][RT * 8 * BS];
