@@ -1776,7 +1776,6 @@ bool launch_project(trl_cuda_context* h, const T* V, int nblk, T* W, int64_t n, 
   cfg.stream = h->stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ProfScope prof(h, PROF_UPDATE, (2.0 * nblk + 3.0) * n * BS * sizeof(T), 2.0 * (2.0 * nblk + 2.0) * n * BS * BS);
   cudaLaunchKernelEx(&cfg, kern, V, nblk, W, n, rows, cond, before, eta2, G, partial, total, total + len, reinterpret_cast<unsigned*>(h->d_small + kSmallCounters) + 2, h->d_status);
   st = after_launch(h, "project");
   return true;
