@@ -146,3 +146,40 @@ def test_counters_of_two_handles_and_of_replays(cuda_handle, monkeypatch):
     monkeypatch.setitem(globals(), "PATTERNS", [None, ("skewed", _with_counter("skewed"))])
     test_one_operator_on_two_handles(cuda_handle)
     test_first_call_of_a_handle_inside_a_capture(cuda_handle, torch.float64)
+
+
+def test_captured_products_of_one_handle_beside_one_another():
+    """Two graphs captured from one handle, replayed on two streams at once, and the handle's own calls."""
+    A = _with_counter("skewed")
+    s = torch.cuda.Stream()
+    h = native.Handle(0, stream=s)
+    try:
+        Ad = native.DeviceCSRTensors.from_host(A)  # on torch's stream; read on the handle's until the next synchronisation
+        torch.cuda.synchronize()
+        op = h.prepare(Ad, 16)
+        h.sync()
+        X = torch.randn((3, A.n, 16), dtype=torch.float64, device="cuda")
+        Y, ref = torch.empty_like(X), torch.empty_like(X)
+        torch.cuda.synchronize()
+        for x, y in zip(X, ref):
+            op.spmm(x, y)
+        torch.cuda.synchronize()
+        graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+        for g, x, y in zip(graphs, X, Y):
+            with torch.cuda.graph(g, stream=s):
+                op.spmm(x, y)
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        for _ in range(20):
+            Y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            for g, t in zip(graphs, streams):
+                with torch.cuda.stream(t):
+                    g.replay()
+            op.spmm(X[2], Y[2])
+            torch.cuda.synchronize()
+            assert torch.equal(Y, ref)
+        del graphs
+        op.close()
+    finally:
+        torch.cuda.synchronize()
+        h.close()

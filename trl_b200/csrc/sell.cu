@@ -811,7 +811,11 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
       // (250) 128 / 129, FP32 111 / 117, bs 2 FP64 129 / 121.
       const int64_t per_warp = op->stored / op->C / (static_cast<int64_t>(grid) * kSpmmWarps); // slots
       const bool wide = bs * es >= 16;
-      const bool tickets = wide && (op->interleave ? per_warp >= 150 : per_warp >= 400 && op->stored >= 48 * op->nslices * op->C);
+      bool tickets = wide && (op->interleave ? per_warp >= 150 : per_warp >= 400 && op->stored >= 48 * op->nslices * op->C);
+      // replays of a captured product may run beside one another: they share no counter
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      if (tickets && cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
+      tickets = tickets && capture == cudaStreamCaptureStatusNone;
       // the counter and the count of finished warps belong to the handle: an operator may serve several
       unsigned* counter = tickets ? reinterpret_cast<unsigned*>(h->d_small + kSmallCounters) : nullptr;
       // narrow rows leave so many slices under way that, beyond L2, what is prefetched is gone before it is
