@@ -808,10 +808,11 @@ int trl_cuda_op_spmm(trl_cuda_handle h, trl_cuda_op op, const void* X, void* Y, 
       // counter: 24^3 elasticity bs 8 FP64 21 / 24; 44^3 bs 4 FP64 (273 slots a warp) 64 / 63, bs 8 (545) 88 / 85;
       // 64^3 bs 8 (1,700) 235 / 223; 300,000 rows of 20, bs 16 FP64 (316) 58 / 66. Skewed: Zipf 60,000 rows bs 16
       // FP64 (114) 40 / 41, 200,000 rows bs 8 (190) 73 / 68, bs 16 (380) 89 / 71; 524,288 rows, bs 1 FP64
-      // (250) 128 / 129, FP32 111 / 117, bs 2 FP64 129 / 121.
+      // (250) 128 / 129, FP32 111 / 117, bs 2 FP64 129 / 121. With the matrix not in L2, rows of 64 bytes or more
+      // gain earlier: 100,003 rows FP32 bs 16 (95) 64 / 61, 150,000 (143) 74 / 68, 60,000 FP64 bs 16 57 / 56.
       const int64_t per_warp = op->stored / op->C / (static_cast<int64_t>(grid) * kSpmmWarps); // slots
       const bool wide = bs * es >= 16;
-      bool tickets = wide && (op->interleave ? per_warp >= 150 : per_warp >= 400 && op->stored >= 48 * op->nslices * op->C);
+      bool tickets = wide && (op->interleave ? per_warp >= (bs * es >= 64 ? 90 : 150) : per_warp >= 400 && op->stored >= 48 * op->nslices * op->C);
       // replays of a captured product may run beside one another: they share no counter
       cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
       if (tickets && cudaStreamIsCapturing(h->stream, &capture) != cudaSuccess) cudaGetLastError();
