@@ -1645,8 +1645,8 @@ int launch_block_dot(trl_cuda_context* h, const T* V, int nblk, const T* W, int6
   }
   // Shapes measured on B200 for the 884,736 x 8 blocks of the 96^3 workload (GB/s of
   // algorithmic bytes; the STREAM copy reference is 6,552): FP64 with 2 KB tiles, JC=8, S=3
-  // gives 6,662 (24 blocks) and 6,970 (48 blocks); FP32 with 4 KB tiles gives 4,371 (8),
-  // 5,269 (24) and with JC=4 5,804 (48).
+  // gives 6,835 (24 blocks) and 6,921 (48 blocks); FP32 with 4 KB tiles gives 5,176 (8 blocks,
+  // JC=8) and with JC=4 5,849 (24) and 5,831 (48).
   // A single block (the driver's T_ii = V_i^T W, both operands usually still in L2 from the
   // SpMM): the register-fed kernel with 8 (FP64) / 4 (FP32) row groups per warp and 4 CTAs
   // per SM measured 6,851 / 5,682 GB/s against 4,759 / 4,562 for the bulk pipeline.
